@@ -2,8 +2,13 @@
 
 The library is built in-tree by deepgengraph_b200/build.py.  There is no fallback: if the
 shared object is missing and cannot be built, importing the ops raises.
+
+`host` is the torch host path of the public operators (csrc/torch_binding.cpp): `host.attn_fwd(...)` and so on, each of
+which returns None when the call is not the regular case and the Python operator has to take it from there.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 from . import build as _build
@@ -75,6 +80,27 @@ def load():
     fn.argtypes = args
   _LIB = lib
   return lib
+
+
+class _Host:
+  """The functions of b200torch.so; the module is loaded (built first if needed) on the first use of any of them."""
+
+  def __getattr__(self, name):
+    load()      # the CUDA library it links against
+    if _build.needs_torch_build():
+      try:
+        _build.build_torch()
+      except Exception as e:
+        if not os.path.exists(_build.TORCH_EXT):
+          raise RuntimeError(f"b200torch.so is missing and could not be built: {e}") from e
+    loader = importlib.machinery.ExtensionFileLoader("b200torch", _build.TORCH_EXT)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200torch", loader))
+    loader.exec_module(mod)
+    self.__dict__.update({n: f for n, f in vars(mod).items() if not n.startswith("_")})
+    return self.__dict__[name]
+
+
+host = _Host()
 
 
 class B200Error(RuntimeError):

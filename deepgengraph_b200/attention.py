@@ -22,6 +22,7 @@ import torch
 from .tracing import traced
 
 from . import _lib
+from ._lib import host
 from .native_ops import _dtype_code, _on_device, _require_cuda, _stream_ptr
 
 
@@ -338,9 +339,10 @@ def _(q, k, v, causal, scale):
 # ----------------------------------------------------------------------------------------------
 def _tracing_graph():
   """True while torch.compile / export traces the caller: only then do the public functions go through the
-  registered custom ops (which carry the fake kernels a tracer needs).  In eager mode they call the implementation
-  directly -- the dispatcher round trip of a Python custom op costs ~17 us of host time per call, more than the
-  kernel takes for a short sequence."""
+  registered custom ops (which carry the fake kernels a tracer needs).  In eager mode they enter the library directly
+  through csrc/torch_binding.cpp, and through the implementations above for everything that path does not take -- the
+  dispatcher round trip of a Python custom op costs ~17 us of host time per call, more than the kernel takes for a
+  short sequence."""
   return torch.compiler.is_compiling()
 
 
@@ -348,13 +350,18 @@ def _tracing_graph():
 def attn_fwd(q, k, v, causal=True, window=-1, softcap=0.0, scale=None):
   """softmax(mask(softcap(q k^T * scale))) v   (kernels/attn.py:18-34, kernels/gemma2.py:19-38)."""
   if not _tracing_graph():
-    return _attn_fwd_impl(q, k, v, causal, window, softcap, scale)
+    out = host.attn_fwd(q, k, v, causal, window, softcap, scale, False)
+    return out if out is not None else _attn_fwd_impl(q, k, v, causal, window, softcap, scale)
   return _op_attn_fwd(q, k, v, bool(causal), int(window), float(softcap), float(scale or 0.0))
 
 
 @traced
 def attn_fwd_with_lse(q, k, v, causal=True, window=-1, softcap=0.0, scale=None):
   """attn_fwd plus the base-2 log-sum-exp of every row of scaled logits, float32 [B, H, Sq]."""
+  if not _tracing_graph():
+    out = host.attn_fwd(q, k, v, causal, window, softcap, scale, True)
+    if out is not None:
+      return out
   return _attn_fwd_impl(q, k, v, causal, window, softcap, scale, want_lse=True)
 
 
@@ -363,7 +370,8 @@ def attn_score_fwd(q, k, v, want_sq=False, causal=True, window=-1, softcap=0.0, 
   """Attention output + per-key column sums of the fp32 probabilities (kernels/h2o.py:35-38);
   want_sq adds the column sums of the squared probabilities (kernels/roco.py:42-48)."""
   if not _tracing_graph():
-    return _attn_score_impl(q, k, v, bool(want_sq), causal, window, softcap, scale)
+    out = host.attn_score(q, k, v, want_sq, causal, window, softcap, scale)
+    return out if out is not None else _attn_score_impl(q, k, v, bool(want_sq), causal, window, softcap, scale)
   op = _op_attn_score_sq_fwd if want_sq else _op_attn_score_fwd
   return op(q, k, v, bool(causal), int(window), float(softcap), float(scale or 0.0))
 
@@ -375,6 +383,9 @@ def attn_kf_fwd(q, k, v, exp_rand=None, tau=1.5, causal=True, scale=None, seed=0
   generate the noise themselves from `seed` (the tensor kf_noise(seed, ...) describes), and nothing of size
   Sq x Skv is read or stored."""
   if not _tracing_graph():
+    out = host.attn_kf(q, k, v, exp_rand, seed, tau, causal, scale)
+    if out is not None:
+      return out
     if exp_rand is None:
       return _attn_kf_seeded_impl(q, k, v, int(seed), float(tau), causal, scale)
     return _attn_kf_impl(q, k, v, exp_rand, float(tau), causal, scale)
@@ -388,7 +399,8 @@ def attn_snapkv_fwd(q, k, v, kernel_size=5, causal=True, scale=None):
   """Attention output + column sums average-pooled over a window of `kernel_size` keys, zero padded
   (kernels/snapkv.py:36-38)."""
   if not _tracing_graph():
-    return _attn_snapkv_impl(q, k, v, int(kernel_size), causal, scale)
+    out = host.attn_snapkv(q, k, v, kernel_size, causal, scale)
+    return out if out is not None else _attn_snapkv_impl(q, k, v, int(kernel_size), causal, scale)
   return _op_attn_snapkv_fwd(q, k, v, int(kernel_size), bool(causal), float(scale or 0.0))
 
 
@@ -397,7 +409,8 @@ def attn_corm_fwd(q, k, v, causal=True, scale=None):
   """Attention output + bool [B, H, Skv]: does any query i attend to the key with probability >= 1 / (i + 1)
   (kernels/corm.py:35-37; the thresholds of Corm.prepare, kernels/corm.py:47-49, are evaluated in the kernel)."""
   if not _tracing_graph():
-    return _attn_corm_impl(q, k, v, causal, scale)
+    out = host.attn_corm(q, k, v, causal, scale)
+    return out if out is not None else _attn_corm_impl(q, k, v, causal, scale)
   return _op_attn_corm_fwd(q, k, v, bool(causal), float(scale or 0.0))
 
 
@@ -407,6 +420,10 @@ def kv_evict_topk(score, k, v, budget, return_indices=False):
   head) keep the `budget` keys with the largest score, in position order.
   score float32 [B, H, S]; k, v [B, S, H, D].  Returns kv_cache [B, 2, budget, H, D] (plane 0 keys, plane 1
   values) and, if asked, the selected positions int32 [B, H, budget]."""
+  if not _tracing_graph():
+    out = host.kv_evict(score, None, k, v, 1, budget, 0, return_indices)
+    if out is not None:
+      return out
   where = "kv_evict_topk"
   dev = _require_cuda(where, score, k, v)
   if score.dtype != torch.float32 or score.dim() != 3 or not score.is_contiguous():
@@ -433,6 +450,10 @@ def kv_evict_roco(score, score_sq, k, v, q_len, budget, recent, return_indices=F
   the largest mean probability; position order.
   score, score_sq float32 [B, H, S] (from attn_score_fwd(want_sq=True)); k, v [B, S, H, D].  Returns kv_cache
   [B, 2, budget + recent, H, D] and, if asked, the selected positions int32 [B, H, budget + recent]."""
+  if not _tracing_graph() and score_sq is not None:
+    out = host.kv_evict(score, score_sq, k, v, q_len, budget, recent, return_indices)
+    if out is not None:
+      return out
   where = "kv_evict_roco"
   dev = _require_cuda(where, score, score_sq, k, v)
   for name, t in (("score", score), ("score_sq", score_sq)):

@@ -1,20 +1,25 @@
-"""Builds the native library in-tree: deepgengraph_b200/csrc/libb200attn.so (sm_100a only).
+"""Builds the native code in-tree, under deepgengraph_b200/csrc/:
 
-The library is one translation unit (csrc/b200attn.cu) compiled with nvcc; it links only the
-CUDA runtime (the driver's tensor-map encoder is looked up at run time), so it can be loaded
-with ctypes from any host language.
+  libb200attn.so   the CUDA library (sm_100a only): one translation unit (b200attn.cu) compiled with nvcc; it links only the
+                   CUDA runtime (the driver's tensor-map encoder is looked up at run time), so it can be loaded with
+                   ctypes from any host language
+  b200torch.so     the torch host path of the public operators (torch_binding.cpp), linked against the library
 """
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libb200attn.so")
+TORCH_EXT = os.path.join(CSRC, "b200torch.so")
 SOURCES = ["b200attn.cu"]
+HEADER = os.path.join("..", "..", "include", "b200attn.h")
 DEPS = ["b200attn.cu", "common.cuh", "elementwise.cuh", "attn_fwd.cuh", "attn_fwd_persist.cuh", "attn_sweep.cuh", "kv_evict.cuh",
-        os.path.join("..", "..", "include", "b200attn.h")]
+        HEADER]
+TORCH_DEPS = ["torch_binding.cpp", HEADER]
 
 
 def _nvcc():
@@ -24,30 +29,60 @@ def _nvcc():
   raise RuntimeError("nvcc not found (set NVCC or install the CUDA toolkit)")
 
 
-def needs_build():
-  if not os.path.exists(LIB):
+def _older(target, deps):
+  if not os.path.exists(target):
     return True
-  t = os.path.getmtime(LIB)
-  return any(os.path.getmtime(os.path.join(CSRC, d)) > t for d in DEPS)
+  t = os.path.getmtime(target)
+  return any(os.path.getmtime(os.path.join(CSRC, d)) > t for d in deps)
 
 
-def build(force=False, verbose=False):
-  """Compile the library if it is missing or older than its sources. Returns its path."""
-  if not force and not needs_build():
-    return LIB
-  cmd = [
-      _nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
-      "-shared", "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v" if verbose else "-O3",
-      "-o", LIB + ".tmp",
-  ] + [os.path.join(CSRC, s) for s in SOURCES] + ["-lcudart"]
+def needs_build():
+  return _older(LIB, DEPS)
+
+
+def needs_torch_build():
+  return _older(TORCH_EXT, TORCH_DEPS)
+
+
+def _run(cmd, target, verbose):
   res = subprocess.run(cmd, capture_output=True, text=True)
   if res.returncode != 0:
     sys.stderr.write(res.stdout + res.stderr)
-    raise RuntimeError("nvcc failed building libb200attn.so")
+    raise RuntimeError(f"{os.path.basename(cmd[0])} failed building {os.path.basename(target)}")
   if verbose:
     sys.stderr.write(res.stdout + res.stderr)
-  os.replace(LIB + ".tmp", LIB)
+  os.replace(target + ".tmp", target)
+
+
+def build(force=False, verbose=False):
+  """Compile what is missing or older than its sources. Returns the path of the CUDA library."""
+  if force or needs_build():
+    cmd = [
+        _nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
+        "-shared", "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v" if verbose else "-O3",
+        "-o", LIB + ".tmp",
+    ] + [os.path.join(CSRC, s) for s in SOURCES] + ["-lcudart"]
+    _run(cmd, LIB, verbose)
+  build_torch(force, verbose)
   return LIB
+
+
+def build_torch(force=False, verbose=False):
+  """The torch host path; needs only a C++ compiler and torch's headers."""
+  if not (force or needs_torch_build()):
+    return TORCH_EXT
+  import torch
+  from torch.utils import cpp_extension
+  cuda_home = os.path.dirname(os.path.dirname(_nvcc()))
+  includes = cpp_extension.include_paths() + [os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+  torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+  cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+  cmd += ["-isystem" + p for p in includes]
+  cmd += ["-o", TORCH_EXT + ".tmp", os.path.join(CSRC, "torch_binding.cpp"), "-L" + torch_lib, "-L" + CSRC,
+          "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-l:libb200attn.so", "-Wl,-rpath,$ORIGIN"]
+  _run(cmd, TORCH_EXT, verbose)
+  return TORCH_EXT
 
 
 if __name__ == "__main__":

@@ -17,6 +17,7 @@ import torch
 from .tracing import traced
 
 from . import _lib
+from ._lib import host
 
 _DTYPES = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 
@@ -68,6 +69,8 @@ class _on_device:
 @traced
 def rms_norm(out, input, weight, epsilon):
   """out = T(input * rsqrt(mean(input^2, -1) + epsilon)) * weight   (csrc/norm.cu:34-56)."""
+  if not torch.compiler.is_compiling() and out is not None and host.norm(out, input, None, weight, epsilon):
+    return
   where = "rms_norm"
   dev = _require_cuda(where, out, input, weight)
   hidden = input.size(-1)
@@ -87,6 +90,8 @@ def rms_norm(out, input, weight, epsilon):
 @traced
 def fused_add_rms_norm(input, residual, weight, epsilon):
   """residual += input; input = rms_norm(residual) * weight, both in place (csrc/norm.cu:59-83)."""
+  if not torch.compiler.is_compiling() and residual is not None and host.norm(None, input, residual, weight, epsilon):
+    return
   where = "fused_add_rms_norm"
   dev = _require_cuda(where, input, residual, weight)
   hidden = input.size(-1)
@@ -123,13 +128,15 @@ def _act_and_mul(fn_name, out, input):
 @traced
 def silu_and_mul(out, input):
   """out[..., i] = T(silu(input[..., i])) * input[..., d + i]   (csrc/activation.cu:6-34)."""
-  _act_and_mul("silu_and_mul", out, input)
+  if torch.compiler.is_compiling() or not host.act_and_mul(out, input, False):
+    _act_and_mul("silu_and_mul", out, input)
 
 
 @traced
 def gelu_tanh_and_mul(out, input):
   """out[..., i] = T(gelu_tanh(input[..., i])) * input[..., d + i] (GeGLU gate)."""
-  _act_and_mul("gelu_tanh_and_mul", out, input)
+  if torch.compiler.is_compiling() or not host.act_and_mul(out, input, True):
+    _act_and_mul("gelu_tanh_and_mul", out, input)
 
 
 @traced
@@ -138,6 +145,8 @@ def rotary_embedding_online(positions, query, key, head_size, rope_theta):
 
   positions: int32 [T].  The reference asserts head_size == 128; 64 and 256 are accepted too.
   """
+  if not torch.compiler.is_compiling() and host.rotary(positions, query, key, head_size, rope_theta):
+    return
   where = "rotary_embedding_online"
   dev = _require_cuda(where, positions, query, key)
   if positions.dtype != torch.int32:
