@@ -17,7 +17,7 @@ LIB = os.path.join(CSRC, "libb200attn.so")
 TORCH_EXT = os.path.join(CSRC, "b200torch.so")
 SOURCES = ["b200attn.cu"]
 HEADER = os.path.join("..", "..", "include", "b200attn.h")
-DEPS = ["b200attn.cu", "common.cuh", "elementwise.cuh", "attn_fwd.cuh", "attn_fwd_persist.cuh", "attn_sweep.cuh", "kv_evict.cuh",
+DEPS = ["b200attn.cu", "common.cuh", "elementwise.cuh", "attn_fwd.cuh", "attn_fwd_persist.cuh", "attn_decode.cuh", "attn_sweep.cuh", "kv_evict.cuh",
         HEADER]
 TORCH_DEPS = ["torch_binding.cpp", HEADER]
 

@@ -744,6 +744,11 @@ struct AttnStrides {
   int64_t q_token, q_batch, k_token, k_batch, v_token, v_batch;
 };
 
+// few query rows against many keys (attn_decode.cuh)
+bool use_decode(int q_len, int group, int units);
+int attn_decode_impl(const void* q, const void* k, const void* v, const FwdParams& f, int head_dim, bool bf16,
+                     const AttnStrides& st, cudaStream_t stream);
+
 inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v, void* out, float* lse,
                                     int lse_stride, int batch, int q_len, int kv_len, int heads, int kv_heads,
                                     int head_dim, int dtype, int causal, int window, float softcap, float scale,
@@ -760,18 +765,8 @@ inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v,
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out)) return B200_ERR_MISALIGNED;
 
   const bool bf16 = dtype == B200_BF16;
-  const int bn = head_dim == 128 ? B200_BN128 : 64;
-  CUtensorMap tq, tk, tv;
-  int rc;
   const AttnStrides contiguous{0, 0, 0, 0, 0, 0};
   const AttnStrides& st = strides ? *strides : contiguous;
-  if ((rc = make_bshd_tensor_map(&tq, q, batch, q_len, heads, head_dim, 128, bf16, st.q_token, st.q_batch)) != B200_OK)
-    return rc;
-  if ((rc = make_bshd_tensor_map(&tk, k, batch, kv_len, kv_heads, head_dim, bn, bf16, st.k_token, st.k_batch)) != B200_OK)
-    return rc;
-  if ((rc = make_bshd_tensor_map(&tv, v, batch, kv_len, kv_heads, head_dim, bn, bf16, st.v_token, st.v_batch)) != B200_OK)
-    return rc;
-
   FwdParams p;
   p.out = out;
   p.lse = lse;
@@ -788,6 +783,18 @@ inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v,
   p.scale_log2 = scale * kLog2e;
   p.cap_in = softcap > 0.f ? scale / softcap : 0.f;
   p.cap_out = softcap * kLog2e;
+  if (use_decode(q_len, heads / kv_heads, batch * kv_heads)) return attn_decode_impl(q, k, v, p, head_dim, bf16, st, stream);
+
+  const int bn = head_dim == 128 ? B200_BN128 : 64;
+  CUtensorMap tq, tk, tv;
+  int rc;
+  if ((rc = make_bshd_tensor_map(&tq, q, batch, q_len, heads, head_dim, 128, bf16, st.q_token, st.q_batch)) != B200_OK)
+    return rc;
+  if ((rc = make_bshd_tensor_map(&tk, k, batch, kv_len, kv_heads, head_dim, bn, bf16, st.k_token, st.k_batch)) != B200_OK)
+    return rc;
+  if ((rc = make_bshd_tensor_map(&tv, v, batch, kv_len, kv_heads, head_dim, bn, bf16, st.v_token, st.v_batch)) != B200_OK)
+    return rc;
+
   const bool cap = softcap > 0.f;
 
 #define B200_FWD_DISPATCH(D_, BN_, NQ_, SB_)                                                                 \
