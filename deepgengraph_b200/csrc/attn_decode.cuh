@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(WARPS * 32, (DecodeCfg<D, WARPS>::CTAS_PER_SM)
   const uint16_t* v_head = p.v + b * p.v_batch + (int64_t)hk * D;
   const int t_lo = p.first_tile + rank * p.tiles_per_cta;
   const int t_hi = min(t_lo + p.tiles_per_cta, p.first_tile + p.n_tiles);
+  pdl_wait();
 
   // ---- this warp's ring: tile t of the warp goes to stage t % 3; rows of D * 2 bytes, 16-byte chunk c of row r at c ^ (r & 7)
   const uint32_t ring = smem_u32(smem) + warp * (kDecodeStages * Cfg::STAGE_BYTES);
@@ -375,19 +376,7 @@ int launch_attn_decode(DecodeParams p, int units, int c, cudaStream_t stream) {
     configured_dev = dev;
   }
   p.tiles_per_cta = (p.n_tiles + c - 1) / c;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(units, c);
-  cfg.blockDim = dim3(WARPS * 32);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = c;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, (const DecodeParams)p));
+  B200_CUDA_TRY(launch_kernel(kern, dim3(units, c), WARPS * 32, Cfg::SMEM_BYTES, stream, c, p));
   return B200_OK;
 }
 

@@ -675,6 +675,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
   if (threadIdx.x == 0) s_skip = status_now;
   tc_fence_before();
+  pdl_wait();
   __syncthreads();
   tc_fence_after();
   c.tmem_base = *tmem_slot;
@@ -729,8 +730,7 @@ int launch_attn_fwd_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   }
   const int groups = (p.q_len + Cfg::BM * NQ - 1) / (Cfg::BM * NQ);
   dim3 grid(groups, p.heads, p.batch);
-  kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_kernel(kern, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, 1, tq, tk, tv, p));
   return B200_OK;
 }
 

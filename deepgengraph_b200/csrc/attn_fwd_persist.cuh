@@ -137,6 +137,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   }
   if (threadIdx.x == 0) s_skip = status_now;
   tc_fence_before();
+  pdl_wait();
   __syncthreads();
   tc_fence_after();
   c.tmem_base = *tmem_slot;
@@ -542,8 +543,7 @@ int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const 
     sp.group_heads = gh;
   }
   const int grid = std::min(sp.total_items, Cfg::CTAS_PER_SM * sm_count());
-  kern<<<grid, Cfg::THREADS_P, Cfg::SMEM_BYTES_P, stream>>>(tq, tk, tv, p, sp);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_kernel(kern, grid, Cfg::THREADS_P, Cfg::SMEM_BYTES_P, stream, 1, tq, tk, tv, p, sp));
   return B200_OK;
 }
 

@@ -704,6 +704,7 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
   if (c.blk_hi == c.blk_lo) {
     // nothing visible in this chunk: its partial vector is all zeros
+    pdl_wait();
     if constexpr (MODE != SWEEP_KF_ROWLSE) {
       if (threadIdx.x < 128) {
         const int64_t off = ((int64_t)c.bh * p.n_chunks + chunk) * p.kv_pad + c.a0 + threadIdx.x;
@@ -737,6 +738,7 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
   if (threadIdx.x == 0) s_skip = status_now;
   tc_fence_before();
+  pdl_wait();
   __syncthreads();
   tc_fence_after();
   c.tmem_base = *tmem_slot;
@@ -797,6 +799,7 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 __global__ void __launch_bounds__(256)
 score_reduce_kernel(float* __restrict__ out, float* __restrict__ out_sq, const float* __restrict__ partial,
                     const float* __restrict__ partial_sq, int kv_len, int kv_pad, int n_chunks, float mul) {
+  pdl_wait();
   const int bh = blockIdx.y;
   const int j = blockIdx.x * 256 + threadIdx.x;
   if (j >= kv_len) return;
@@ -904,8 +907,7 @@ int launch_sweep(const CUtensorMap& ta, const CUtensorMap& tx, const CUtensorMap
     configured_dev = dev;
   }
   dim3 grid(p.batch * (GROUPED ? p.heads / p.kv_group : p.heads), n_tiles, n_chunks);
-  kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tx, tn, p);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_kernel(kern, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, 1, ta, tx, tn, p));
   return B200_OK;
 }
 
@@ -927,6 +929,7 @@ inline int score_common_checks(const void* q, const void* k, const void* v, void
 __global__ void __launch_bounds__(256)
 corm_reduce_kernel(uint8_t* __restrict__ out, const float* __restrict__ partial_flag, int kv_len, int kv_pad,
                    int n_chunks) {
+  pdl_wait();
   const int bh = blockIdx.y;
   const int j = blockIdx.x * 256 + threadIdx.x;
   if (j >= kv_len) return;
@@ -940,6 +943,7 @@ corm_reduce_kernel(uint8_t* __restrict__ out, const float* __restrict__ partial_
 // the column sums: F.avg_pool1d(kernel_size, padding = kernel_size // 2, stride = 1), kernels/snapkv.py:36-38)
 __global__ void __launch_bounds__(256)
 avg_pool1d_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t rows, int len, int kernel) {
+  pdl_wait();
   const int64_t r = blockIdx.y;
   const int j = blockIdx.x * 256 + threadIdx.x;
   if (j >= len) return;
@@ -1026,12 +1030,11 @@ inline int attn_score_impl(const void* q, const void* k, const void* v, void* ou
 #undef B200_SWEEPG
     if (rc != B200_OK) return rc;
     dim3 ggrid((kv_len + 255) / 256, batch * kv_heads);
-    score_reduce_kernel<<<ggrid, 256, 0, stream>>>(score, score_sq, p.partial, p.partial_sq, kv_len, w.kv_pad,
-                                                   p.n_chunks, 1.0f);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_kernel(score_reduce_kernel, ggrid, 256, 0, stream, 1, score, score_sq, p.partial, p.partial_sq,
+                                kv_len, w.kv_pad, p.n_chunks, 1.0f));
     if (corm_flags != nullptr) {
-      corm_reduce_kernel<<<ggrid, 256, 0, stream>>>(corm_flags, p.partial_sq, kv_len, w.kv_pad, p.n_chunks);
-      B200_CUDA_TRY(cudaGetLastError());
+      B200_CUDA_TRY(launch_kernel(corm_reduce_kernel, ggrid, 256, 0, stream, 1, corm_flags, p.partial_sq, kv_len,
+                                  w.kv_pad, p.n_chunks));
     }
     return B200_OK;
   }
@@ -1051,12 +1054,11 @@ inline int attn_score_impl(const void* q, const void* k, const void* v, void* ou
   if (rc != B200_OK) return rc;
 
   dim3 rgrid((kv_len + 255) / 256, batch * kv_heads);
-  score_reduce_kernel<<<rgrid, 256, 0, stream>>>(score, score_sq, p.partial, p.partial_sq, kv_len, w.kv_pad,
-                                                 p.n_chunks * group, 1.0f / (float)group);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_kernel(score_reduce_kernel, rgrid, 256, 0, stream, 1, score, score_sq, p.partial, p.partial_sq,
+                              kv_len, w.kv_pad, p.n_chunks * group, 1.0f / (float)group));
   if (corm_flags != nullptr) {
-    corm_reduce_kernel<<<rgrid, 256, 0, stream>>>(corm_flags, p.partial_sq, kv_len, w.kv_pad, p.n_chunks);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_kernel(corm_reduce_kernel, rgrid, 256, 0, stream, 1, corm_flags, p.partial_sq, kv_len,
+                                w.kv_pad, p.n_chunks));
   }
   return B200_OK;
 }
@@ -1155,9 +1157,8 @@ inline int attn_kf_impl(const void* q, const void* k, const void* v, const float
   if (rc != B200_OK) return rc;
 
   dim3 rgrid((kv_len + 255) / 256, batch * kv_heads);
-  score_reduce_kernel<<<rgrid, 256, 0, stream>>>(kf_score, nullptr, p.partial, nullptr, kv_len, w.kv_pad,
-                                                 p.n_chunks * group, 1.0f / (float)group);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_kernel(score_reduce_kernel, rgrid, 256, 0, stream, 1, kf_score, (float*)nullptr, p.partial,
+                              (float*)nullptr, kv_len, w.kv_pad, p.n_chunks * group, 1.0f / (float)group));
   return B200_OK;
 }
 

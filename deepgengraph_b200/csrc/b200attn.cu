@@ -322,8 +322,8 @@ int b200_avg_pool1d_f32(const float* input, float* output, int64_t rows, int len
   if (rows == 0) return B200_OK;
   if (rows > 65535) return B200_ERR_UNSUPPORTED;
   dim3 grid((length + 255) / 256, (unsigned)rows);
-  avg_pool1d_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(input, output, rows, length, kernel_size);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_kernel(avg_pool1d_kernel, grid, 256, 0, (cudaStream_t)stream, 1, input, output, rows, length,
+                              kernel_size));
   return B200_OK;
 }
 

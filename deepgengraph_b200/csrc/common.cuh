@@ -208,6 +208,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_slow(bar, parity, abort_flag, code);
 }
 
+// programmatic dependent launch (see launch_kernel below)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies, global -> shared, completion on an mbarrier)
 // ---------------------------------------------------------------------------
@@ -527,6 +530,35 @@ inline int sm_count() {
     cached_dev = dev;
   }
   return cached;
+}
+
+// Every kernel of the library is launched with programmatic stream serialization: the launch is handed to the SMs while the
+// previous kernel of the stream drains, and the kernel itself waits (pdl_wait) for that kernel's end and its memory
+// before it touches global memory.  Measured (148 blocks, back to back on one stream): a 1 us kernel every 4.1 us without
+// and every 2.0 us with, a 2.6 us kernel every 6.1 and 3.5 us -- without it the front end also starts kernels on a
+// 2 us raster.  No kernel triggers its successor early (griddepcontrol.launch_dependents): the next launch's CTAs would
+// take the slots of an SM one by one as this launch's CTAs end, so that SMs with light CTAs receive two of the heaviest
+// tiles -- causal attention, 32 heads, 1024 tokens: 21.9 us with a trigger after the set-up, 19.1 with one before the
+// epilogue, 18.2 with the implicit one at the kernel's end (20.5 without programmatic launch).
+// Every CTA that leaves early waits first: a kernel's end then implies the end of everything before it in the stream.
+template <class... Params, class... Args>
+inline cudaError_t launch_kernel(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                 unsigned cluster_y, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = cluster_y;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster_y > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

@@ -125,6 +125,7 @@ rms_norm_rows_kernel(T* __restrict__ out, T* __restrict__ input, T* __restrict__
   constexpr int VN = 16 / sizeof(T);
   const int nvec = hidden / VN;  // hidden % VN == 0 checked on the host
   const int lane = threadIdx.x & 31;
+  pdl_wait();
   const int64_t warp_global = (int64_t)blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
   const int64_t warp_count = (int64_t)gridDim.x * (THREADS / 32);
   for (int64_t row = warp_global; row < num_tokens; row += warp_count) {
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(256)
 rms_norm_generic_kernel(T* __restrict__ out, T* __restrict__ input, T* __restrict__ residual,
                         const T* __restrict__ weight, float epsilon, int64_t num_tokens, int hidden) {
   __shared__ float red[33];
+  pdl_wait();
   for (int64_t row = blockIdx.x; row < num_tokens; row += gridDim.x) {
     T* in_row = input + row * hidden;
     T* res_row = FUSED_ADD ? residual + row * hidden : nullptr;
@@ -239,6 +241,7 @@ int launch_rms_norm(void* out, void* input, void* residual, const void* weight, 
   T* in = (T*)input;
   T* res = (T*)residual;
   const T* w = (const T*)weight;
+  cudaError_t launched;
   if (vec_ok && nvec <= 32 * 32) {
     // One row per warp, small blocks (4 warps): the register footprint of a row (MAXV 16-byte vectors per lane) limits
     // an SM to a few hundred resident threads, and with small blocks those threads belong to several blocks that
@@ -247,8 +250,9 @@ int launch_rms_norm(void* out, void* input, void* residual, const void* weight, 
     static const int env_grid = std::getenv("B200_RMS_GRID_PER_SM") ? std::atoi(std::getenv("B200_RMS_GRID_PER_SM")) : 0;
     const int per_sm = env_grid > 0 ? env_grid : 16;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((num_tokens + TH / 32 - 1) / (TH / 32), (int64_t)sms * per_sm));
-#define B200_RMS_LAUNCH(MAXV_) \
-  rms_norm_rows_kernel<T, MAXV_, FUSED_ADD, TH><<<grid, TH, 0, stream>>>(o, in, res, w, eps, num_tokens, hidden)
+#define B200_RMS_LAUNCH(MAXV_)                                                                                        \
+  launched = launch_kernel(rms_norm_rows_kernel<T, MAXV_, FUSED_ADD, TH>, grid, TH, 0, stream, 1, o, in, res, w, eps, \
+                           num_tokens, hidden)
     if (nvec <= 64) B200_RMS_LAUNCH(2);
     else if (nvec <= 128) B200_RMS_LAUNCH(4);
     else if (nvec <= 256) B200_RMS_LAUNCH(8);
@@ -258,9 +262,10 @@ int launch_rms_norm(void* out, void* input, void* residual, const void* weight, 
 #undef B200_RMS_LAUNCH
   } else {
     const int grid = (int)std::min<int64_t>(num_tokens, (int64_t)sms * 8);
-    rms_norm_generic_kernel<T, FUSED_ADD><<<grid, 256, 0, stream>>>(o, in, res, w, eps, num_tokens, hidden);
+    launched = launch_kernel(rms_norm_generic_kernel<T, FUSED_ADD>, grid, 256, 0, stream, 1, o, in, res, w, eps, num_tokens,
+                             hidden);
   }
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launched);
   return B200_OK;
 }
 
@@ -322,6 +327,7 @@ act_and_mul_vec_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t nu
   const Index vec_per_row = (Index)(d / VN);
   const Index total = (Index)num_tokens * vec_per_row;
   const Index step = (Index)gridDim.x * 256;
+  pdl_wait();
   // two vectors per thread and step: four 16-byte loads in flight before the first store
   for (Index g = (Index)blockIdx.x * 256 + threadIdx.x; g < total; g += 2 * step) {
     const Index g1 = g + step;
@@ -346,6 +352,7 @@ __global__ void __launch_bounds__(256)
 act_and_mul_generic_kernel(T* __restrict__ out, const T* __restrict__ in, int64_t num_tokens, int d) {
   const int64_t total = num_tokens * d;
   Op op;
+  pdl_wait();
   for (int64_t g = (int64_t)blockIdx.x * 256 + threadIdx.x; g < total; g += (int64_t)gridDim.x * 256) {
     const int64_t t = g / d;
     const int i = (int)(g - t * d);
@@ -360,19 +367,23 @@ int launch_act_and_mul(void* out, const void* in, int64_t num_tokens, int d, cud
   constexpr int VN = 16 / sizeof(T);
   const int sms = sm_count();
   const bool vec_ok = (d % VN == 0) && aligned16(out) && aligned16(in);
+  cudaError_t launched;
   if (vec_ok) {
     const int64_t total = num_tokens * (d / VN);
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((total + 511) / 512, (int64_t)sms * 16));
     if (total + 2 * (int64_t)grid * 256 < (int64_t)1 << 31)
-      act_and_mul_vec_kernel<T, Op, int><<<grid, 256, 0, stream>>>((T*)out, (const T*)in, num_tokens, d);
+      launched = launch_kernel(act_and_mul_vec_kernel<T, Op, int>, grid, 256, 0, stream, 1, (T*)out, (const T*)in,
+                               num_tokens, d);
     else
-      act_and_mul_vec_kernel<T, Op, int64_t><<<grid, 256, 0, stream>>>((T*)out, (const T*)in, num_tokens, d);
+      launched = launch_kernel(act_and_mul_vec_kernel<T, Op, int64_t>, grid, 256, 0, stream, 1, (T*)out, (const T*)in,
+                               num_tokens, d);
   } else {
     const int64_t total = num_tokens * d;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, (int64_t)sms * 16));
-    act_and_mul_generic_kernel<T, Op><<<grid, 256, 0, stream>>>((T*)out, (const T*)in, num_tokens, d);
+    launched = launch_kernel(act_and_mul_generic_kernel<T, Op>, grid, 256, 0, stream, 1, (T*)out, (const T*)in,
+                             num_tokens, d);
   }
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launched);
   return B200_OK;
 }
 
@@ -413,6 +424,7 @@ rotary_online_kernel(const int32_t* __restrict__ positions, T* __restrict__ quer
 #pragma unroll
     for (int t = 0; t < PER_LANE; ++t) inv_freq[t] = exp2(-(double)(2 * (lane + 32 * t)) / (double)HEAD_DIM * l2t);
   }
+  pdl_wait();   // (the frequencies above need no memory)
   constexpr double kTwoPi = 6.283185307179586476925286766559, kInvTwoPi = 0.15915494309189533576888376337251;
   for (int64_t tok = warp_global; tok < num_tokens; tok += warp_count) {
     const double pos = (double)positions[tok];
@@ -491,23 +503,24 @@ int launch_rotary(const int32_t* positions, void* query, void* key, int64_t num_
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((num_tokens + 7) / 8, (int64_t)sm_count() * 8));
   T* q = (T*)query;
   T* k = (T*)key;
+  cudaError_t launched;
   switch (head_dim) {
     case 64:
-      rotary_online_kernel<T, 64><<<grid, 256, 0, stream>>>(positions, q, k, num_tokens, heads, kv_heads, q_stride,
-                                                            k_stride, theta, vec_ok);
+      launched = launch_kernel(rotary_online_kernel<T, 64>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
+                               kv_heads, q_stride, k_stride, theta, vec_ok);
       break;
     case 128:
-      rotary_online_kernel<T, 128><<<grid, 256, 0, stream>>>(positions, q, k, num_tokens, heads, kv_heads, q_stride,
-                                                             k_stride, theta, vec_ok);
+      launched = launch_kernel(rotary_online_kernel<T, 128>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
+                               kv_heads, q_stride, k_stride, theta, vec_ok);
       break;
     case 256:
-      rotary_online_kernel<T, 256><<<grid, 256, 0, stream>>>(positions, q, k, num_tokens, heads, kv_heads, q_stride,
-                                                             k_stride, theta, vec_ok);
+      launched = launch_kernel(rotary_online_kernel<T, 256>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
+                               kv_heads, q_stride, k_stride, theta, vec_ok);
       break;
     default:
       return B200_ERR_UNSUPPORTED;
   }
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launched);
   return B200_OK;
 }
 

@@ -189,6 +189,7 @@ kv_evict_topk_kernel(const float* __restrict__ score, const uint8_t* __restrict_
   extern __shared__ int32_t s_idx[];   // [budget] selected key indices, ascending
   uint32_t* s_keys = reinterpret_cast<uint32_t*>(s_idx + budget);   // [seq] order keys, when they fit (`staged`)
 
+  pdl_wait();
   const int bh = blockIdx.x, b = bh / heads, h = bh - b * heads;
   const float* sc = score + (int64_t)bh * seq;
 
@@ -259,6 +260,7 @@ kv_evict_roco_kernel(const float* __restrict__ score, const float* __restrict__ 
   uint32_t* s_mean = s_std + key_words;                          // order keys of score / q_len
   uint8_t* in_a = reinterpret_cast<uint8_t*>(s_mean + key_words);   // [seq] 1 = key belongs to A
 
+  pdl_wait();
   const int bh = blockIdx.x, b = bh / heads, h = bh - b * heads;
   const float* sc = score + (int64_t)bh * seq;
   const float* sq = score_sq + (int64_t)bh * seq;
@@ -325,10 +327,9 @@ int launch_kv_evict_roco(dim3 grid, size_t smem, cudaStream_t stream, const floa
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     configured_dev = dev;
   }
-  kern<<<grid, kEvictThreads, smem, stream>>>(score, score_sq, (const uint8_t*)k, (const uint8_t*)v,
-                                              (uint8_t*)kv_cache, indices, seq, heads, head_dim, (float)q_len, budget,
-                                              recent, staged);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_kernel(kern, grid, kEvictThreads, smem, stream, 1, score, score_sq, (const uint8_t*)k,
+                              (const uint8_t*)v, (uint8_t*)kv_cache, indices, seq, heads, head_dim, (float)q_len, budget,
+                              recent, staged));
   return B200_OK;
 }
 
@@ -344,9 +345,8 @@ int launch_kv_evict_topk(dim3 grid, size_t smem, cudaStream_t stream, const floa
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     configured_dev = dev;
   }
-  kern<<<grid, kEvictThreads, smem, stream>>>(score, (const uint8_t*)k, (const uint8_t*)v, (uint8_t*)kv_cache, indices,
-                                              seq, heads, head_dim, budget, staged);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_kernel(kern, grid, kEvictThreads, smem, stream, 1, score, (const uint8_t*)k, (const uint8_t*)v,
+                              (uint8_t*)kv_cache, indices, seq, heads, head_dim, budget, staged));
   return B200_OK;
 }
 
