@@ -6,12 +6,15 @@
 //     k_cache = gather(k, idx); v_cache = gather(v, idx); kv_cache = cat([k_cache, v_cache], dim=1)
 // i.e. the result only depends on the SET of the top-`budget` keys; it is emitted in ascending key order.
 //
-// One to eight CTAs per (batch, head), each of which repeats the (cheap) selection and gathers its share of the
-// rows: the order keys are staged in shared memory once, a 4-pass radix select (8 bits per pass, shared-memory
-// histogram) finds the value of the budget-th largest score, one ordered compaction (per-thread key segments, two
-// block scans in all) emits the selected key indices already sorted, and the rows are copied with 16-byte accesses.  Ties at the threshold value are
-// resolved towards the lower key index (torch.topk leaves that choice unspecified).  The selection is a chain of
-// block-wide steps on 16 KB of keys (latency-bound); the gather moves 2 * budget * D elements per head.
+// Several CTAs per (batch, head), each of which repeats the (cheap) selection and gathers its share of the rows.  A radix
+// select (4 passes of 8 bits, shared-memory histogram) finds the value of the budget-th largest score, one ordered
+// compaction emits the selected key indices already sorted, and the rows are copied with 16-byte accesses.  Ties at the
+// threshold value are resolved towards the lower key index (torch.topk leaves that choice unspecified).  The selection is
+// a chain of block-wide steps on a few KB of keys (latency-bound); the gather moves 2 * budget * D elements per head.
+//   seq <= 16384: kv_evict_regs_kernel -- a thread owns consecutive keys in registers from the one load of the scores to
+//                 the emission of the indices; seven block barriers in all (RoCo: twelve).
+//   longer:       kv_evict_topk_kernel / kv_evict_roco_kernel -- keys in shared memory (or re-read from L2 where they do
+//                 not fit), read again by each of the five (ten) walks over them.
 #pragma once
 
 #include "common.cuh"
@@ -135,6 +138,7 @@ __device__ __forceinline__ void ordered_compact(SureFn sure, TieFn tie, EmitFn e
 // Gather of the selected rows: kv_cache[b, 0, i, h, :] = k[b, idx_i, h, :], kv_cache[b, 1, i, h, :] = v[b, idx_i, h, :].
 // The CTAs of one (batch, head) -- gridDim.y of them, each of which has made the same selection -- take
 // interleaved slices of the rows; four 16-byte K and V loads are in flight per thread before the first store.
+template <int THREADS>
 __device__ __forceinline__ void gather_selected_rows(const int32_t* s_idx, const uint8_t* __restrict__ k,
                                                      const uint8_t* __restrict__ v, uint8_t* __restrict__ kv_cache,
                                                      int b, int h, int seq, int heads, int row_bytes, int keep) {
@@ -144,9 +148,9 @@ __device__ __forceinline__ void gather_selected_rows(const int32_t* s_idx, const
   const int64_t dst_plane = (int64_t)keep * heads * row_bytes;               // [B, 2, keep, H, D]
   const int64_t dst_batch = (int64_t)b * 2 * dst_plane + (int64_t)h * row_bytes;
   const int total = keep * vec_per_row;
-  const int stride = kEvictThreads * gridDim.y;
+  const int stride = THREADS * gridDim.y;
   constexpr int U = 4;
-  for (int g0 = blockIdx.y * kEvictThreads + threadIdx.x; g0 < total; g0 += U * stride) {
+  for (int g0 = blockIdx.y * THREADS + threadIdx.x; g0 < total; g0 += U * stride) {
     uint4 kk[U], vv[U];
     int64_t dst[U];
 #pragma unroll
@@ -218,7 +222,7 @@ kv_evict_topk_kernel(const float* __restrict__ score, const uint8_t* __restrict_
   if (indices_out != nullptr && blockIdx.y == 0)
     for (int i = threadIdx.x; i < budget; i += kEvictThreads) indices_out[(int64_t)bh * budget + i] = s_idx[i];
 
-  gather_selected_rows(s_idx, k, v, kv_cache, b, h, seq, heads, head_dim * ELEM_BYTES, budget);
+  gather_selected_rows<kEvictThreads>(s_idx, k, v, kv_cache, b, h, seq, heads, head_dim * ELEM_BYTES, budget);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -307,7 +311,195 @@ kv_evict_roco_kernel(const float* __restrict__ score, const float* __restrict__ 
   if (indices_out != nullptr && blockIdx.y == 0)
     for (int i = threadIdx.x; i < keep; i += kEvictThreads) indices_out[(int64_t)bh * keep + i] = s_idx[i];
 
-  gather_selected_rows(s_idx, k, v, kv_cache, b, h, seq, heads, head_dim * ELEM_BYTES, keep);
+  gather_selected_rows<kEvictThreads>(s_idx, k, v, kv_cache, b, h, seq, heads, head_dim * ELEM_BYTES, keep);
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// Both selections with the keys in registers: thread t owns keys [t * NK, (t + 1) * NK).
+// What bounds it is the chain of block-wide steps, so each of them is as short as it can be:
+//   * every pass has its own histogram (all cleared at the start) and every warp scans it for itself (eight bins per lane,
+//     five shuffles), so a pass has ONE barrier -- between the counting and the scan;
+//   * the candidates of a pass are a bit mask of the thread's keys, narrowed by the digit just found;
+//   * the (#sure, #tie) counts before a thread come from one packed scan with one barrier.
+// Measured (2 x 32 heads, 512 of 4096 keys, head_dim 128, back to back): 17.2 -> 11.8 us with the kernel above; the rows
+// alone are 33.5 MB, 5.1 us at the copy rate.
+// ---------------------------------------------------------------------------------------------------------
+constexpr int kEvictRegThreads = 512;
+constexpr int kEvictRegWarps = kEvictRegThreads / 32;
+constexpr int kEvictRegMaxSeq = 32 * kEvictRegThreads;   // a thread's candidates fit a 32-bit mask
+
+// Key value of the `want`-th largest among the keys whose `live` bit is set in the thread that owns them (at least `want`
+// of them in the block).  hist: four cleared histograms.  *need_equal = how many keys EQUAL to it are among the `want`.
+template <int NK>
+__device__ __forceinline__ uint32_t regs_radix_select(const uint32_t (&key)[NK], uint32_t live, int want, int* hist,
+                                                      int* need_equal) {
+  const int lane = threadIdx.x & 31;
+  uint32_t prefix = 0;
+  int remaining = want;
+#pragma unroll
+  for (int pass = 3; pass >= 0; --pass) {
+    int* h = hist + pass * 256;
+    const int shift = pass * 8;
+#pragma unroll
+    for (int u = 0; u < NK; ++u)
+      if (live >> u & 1u) atomicAdd(&h[(key[u] >> shift) & 0xff], 1);
+    __syncthreads();
+    // lane l scans bins 255 - 8 l, 254 - 8 l, ..., 248 - 8 l
+    const int4 hi = reinterpret_cast<const int4*>(h)[63 - 2 * lane], lo = reinterpret_cast<const int4*>(h)[62 - 2 * lane];
+    const int bin[8] = {hi.w, hi.z, hi.y, hi.x, lo.w, lo.z, lo.y, lo.x};
+    int own = 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) own += bin[e];
+    int incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const int above = incl - own;   // keys in the bins of the lanes before
+    int digit = 0, before = 0;      // before: keys in this lane's bins above the wanted one
+    const bool here = above < remaining && remaining <= incl;
+    bool found = false;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (!found && remaining <= above + before + bin[e]) {
+        digit = 255 - 8 * lane - e;
+        found = true;
+      }
+      if (!found) before += bin[e];
+    }
+    const int src = __ffs(__ballot_sync(0xffffffffu, here)) - 1;
+    digit = __shfl_sync(0xffffffffu, digit, src);
+    remaining -= __shfl_sync(0xffffffffu, above + before, src);
+    prefix |= (uint32_t)digit << shift;
+    if (pass > 0) {
+#pragma unroll
+      for (int u = 0; u < NK; ++u)
+        if (((key[u] >> shift) & 0xff) != (uint32_t)digit) live &= ~(1u << u);
+    }
+  }
+  *need_equal = remaining;
+  return prefix;
+}
+
+// Sure and tied keys of the threads before this one, packed (ties in the upper half: at most kEvictRegMaxSeq = 2^14 each).
+__device__ __forceinline__ uint32_t regs_scan_counts(uint32_t sure, uint32_t tie, uint32_t* warp_totals) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t own = __popc(sure) | __popc(tie) << 16;
+  uint32_t incl = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) warp_totals[wid] = incl;
+  __syncthreads();
+  return __reduce_add_sync(0xffffffffu, lane < wid ? warp_totals[lane] : 0u) + incl - own;
+}
+
+// ROCO = false: the `budget` largest scores.  ROCO = true: the two-stage selection described above.
+template <int NK, bool ROCO>
+__global__ void __launch_bounds__(kEvictRegThreads)
+kv_evict_regs_kernel(const float* __restrict__ score, const float* __restrict__ score_sq, const uint8_t* __restrict__ k,
+                     const uint8_t* __restrict__ v, uint8_t* __restrict__ kv_cache, int32_t* __restrict__ indices_out,
+                     int seq, int heads, int row_bytes, float q_len, int budget, int recent) {
+  constexpr int HISTS = ROCO ? 8 : 4;
+  __shared__ __align__(16) int hist[HISTS * 256];
+  __shared__ uint32_t warp_totals[2][kEvictRegWarps];
+  extern __shared__ int32_t s_idx[];   // [keep] selected key indices, ascending
+  const int keep = ROCO ? budget + recent : budget;
+  const int bh = blockIdx.x, b = bh / heads, h = bh - b * heads;
+#pragma unroll
+  for (int i = threadIdx.x; i < HISTS * 256; i += kEvictRegThreads) hist[i] = 0;
+  pdl_wait();
+
+  const int first = threadIdx.x * NK;
+  const int owned = max(0, min(NK, seq - first));
+  const uint32_t valid = owned == 32 ? 0xffffffffu : (1u << owned) - 1u;
+  const float* sc = score + (int64_t)bh * seq;
+  const float* sq = ROCO ? score_sq + (int64_t)bh * seq : nullptr;
+  auto load = [&](const float* src, float (&x)[NK]) {
+    if (NK % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && owned == NK) {
+#pragma unroll
+      for (int u = 0; u < NK; u += 4) {
+        const float4 f = *reinterpret_cast<const float4*>(src + first + u);
+        x[u] = f.x, x[u + 1] = f.y, x[u + 2] = f.z, x[u + 3] = f.w;
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < NK; ++u) x[u] = u < owned ? src[first + u] : 0.f;
+    }
+  };
+  uint32_t key[NK];      // order keys of the score (ROCO: of the mean)
+  uint32_t sure = 0;     // ROCO: the keys in A
+  {
+    float x[NK];
+    load(sc, x);
+    if constexpr (ROCO) {
+      float x2[NK];
+      load(sq, x2);
+      uint32_t std_key[NK];
+#pragma unroll
+      for (int u = 0; u < NK; ++u) {
+        std_key[u] = score_key_nan_high(roco_std(x[u], x2[u], q_len));
+        key[u] = score_key_nan_high(roco_mean(x[u], q_len));
+      }
+      __syncthreads();   // histograms are clear
+      if (recent > 0) {
+        int need_tie;
+        const uint32_t thr = regs_radix_select<NK>(std_key, valid, recent, hist + 4 * 256, &need_tie);
+        uint32_t tie = 0;
+#pragma unroll
+        for (int u = 0; u < NK; ++u) {
+          if (std_key[u] > thr) sure |= 1u << u;
+          if (std_key[u] == thr) tie |= 1u << u;
+        }
+        sure &= valid;
+        tie &= valid;
+        int ties_before = (int)(regs_scan_counts(sure, tie, warp_totals[0]) >> 16);
+#pragma unroll
+        for (int u = 0; u < NK; ++u)
+          if (tie >> u & 1u) {
+            if (ties_before < need_tie) sure |= 1u << u;
+            ++ties_before;
+          }
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < NK; ++u) key[u] = score_key(x[u]);
+      __syncthreads();   // histograms are clear
+    }
+  }
+
+  // the keys above the threshold of the `budget` largest (outside A), and the first `need_tie` of those that equal it
+  int need_tie = 0;
+  uint32_t tie = 0;
+  if (budget > 0) {
+    const uint32_t rest = valid & ~sure;
+    const uint32_t thr = regs_radix_select<NK>(key, rest, budget, hist, &need_tie);
+    uint32_t more = 0;
+#pragma unroll
+    for (int u = 0; u < NK; ++u) {
+      if (key[u] > thr) more |= 1u << u;
+      if (key[u] == thr) tie |= 1u << u;
+    }
+    sure |= more & rest;
+    tie &= rest;
+  }
+  const uint32_t before = regs_scan_counts(sure, tie, warp_totals[1]);
+  int sure_before = (int)(before & 0xffffu), ties_before = (int)(before >> 16);
+#pragma unroll
+  for (int u = 0; u < NK; ++u) {
+    const bool is_sure = sure >> u & 1u, is_tie = tie >> u & 1u;
+    if (is_sure || (is_tie && ties_before < need_tie)) s_idx[sure_before + min(ties_before, need_tie)] = first + u;
+    sure_before += is_sure ? 1 : 0;
+    ties_before += is_tie ? 1 : 0;
+  }
+  __syncthreads();
+
+  if (indices_out != nullptr && blockIdx.y == 0)
+    for (int i = threadIdx.x; i < keep; i += kEvictRegThreads) indices_out[(int64_t)bh * keep + i] = s_idx[i];
+  gather_selected_rows<kEvictRegThreads>(s_idx, k, v, kv_cache, b, h, seq, heads, row_bytes, keep);
 }
 
 // Dynamic shared memory beyond which a kernel must opt in (cudaFuncAttributeMaxDynamicSharedMemorySize).  The
@@ -350,6 +542,46 @@ int launch_kv_evict_topk(dim3 grid, size_t smem, cudaStream_t stream, const floa
   return B200_OK;
 }
 
+// CTAs per (batch, head): as many as are resident at once (two per SM), so that the launch has no second wave (each repeats
+// the selection, which reads a few KB of scores from L2), and at most 16.
+template <int NK, bool ROCO>
+int launch_evict_regs_nk(const float* score, const float* score_sq, const void* k, const void* v, void* kv_cache,
+                         int32_t* indices, int batch, int seq, int heads, int row_bytes, int q_len, int budget, int recent,
+                         cudaStream_t stream) {
+  auto kern = kv_evict_regs_kernel<NK, ROCO>;
+  const size_t smem = (size_t)(budget + recent) * sizeof(int32_t);
+  static thread_local int configured_dev = -1;
+  int dev = 0;
+  B200_CUDA_TRY(cudaGetDevice(&dev));
+  if (smem > kEvictSmemOptIn - 8 * 1024 && configured_dev != dev) {
+    B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
+    configured_dev = dev;
+  }
+  const int units = batch * heads;
+  const dim3 grid(units, std::max(1, std::min(16, 2 * sm_count() / units)));
+  B200_CUDA_TRY(launch_kernel(kern, grid, kEvictRegThreads, smem, stream, 1, score, score_sq, (const uint8_t*)k,
+                              (const uint8_t*)v, (uint8_t*)kv_cache, indices, seq, heads, row_bytes, (float)q_len, budget,
+                              recent));
+  return B200_OK;
+}
+
+// keys per thread: the smallest of 2, 4, 8, 16, 32 that covers the sequence
+template <bool ROCO>
+int launch_evict_regs(const float* score, const float* score_sq, const void* k, const void* v, void* kv_cache,
+                      int32_t* indices, int batch, int seq, int heads, int row_bytes, int q_len, int budget, int recent,
+                      cudaStream_t stream) {
+  const int per_thread = (seq + kEvictRegThreads - 1) / kEvictRegThreads;
+#define B200_EVICT_NK(NK_)                                                                                          \
+  launch_evict_regs_nk<NK_, ROCO>(score, score_sq, k, v, kv_cache, indices, batch, seq, heads, row_bytes, q_len, budget, \
+                                  recent, stream)
+  if (per_thread <= 2) return B200_EVICT_NK(2);
+  if (per_thread <= 4) return B200_EVICT_NK(4);
+  if (per_thread <= 8) return B200_EVICT_NK(8);
+  if (per_thread <= 16) return B200_EVICT_NK(16);
+  return B200_EVICT_NK(32);
+#undef B200_EVICT_NK
+}
+
 inline int kv_evict_roco_impl(const float* score, const float* score_sq, const void* k, const void* v,
                               void* kv_cache, int32_t* indices, int batch, int seq, int heads, int head_dim,
                               int q_len, int budget, int recent, int elem_bytes, cudaStream_t stream) {
@@ -361,6 +593,9 @@ inline int kv_evict_roco_impl(const float* score, const float* score_sq, const v
     return B200_ERR_MISALIGNED;
   const size_t smem_min = (size_t)(budget + recent) * sizeof(int32_t) + (size_t)((seq + 15) / 16) * 16;
   if (smem_min > 200 * 1024) return B200_ERR_UNSUPPORTED;
+  if (seq <= kEvictRegMaxSeq)
+    return launch_evict_regs<true>(score, score_sq, k, v, kv_cache, indices, batch, seq, heads, head_dim * elem_bytes, q_len,
+                                   budget, recent, stream);
   const size_t key_bytes = 2 * skewed_words(seq) * sizeof(uint32_t);   // std and mean keys, padded
   const int staged = smem_min + key_bytes <= 200 * 1024 ? 1 : 0;
   const size_t smem = smem_min + (staged ? key_bytes : 0);
@@ -382,6 +617,9 @@ inline int kv_evict_topk_impl(const float* score, const void* k, const void* v, 
   if ((head_dim * elem_bytes) % 16 != 0 || !aligned16(k) || !aligned16(v) || !aligned16(kv_cache))
     return B200_ERR_MISALIGNED;
   if (budget > 12288) return B200_ERR_UNSUPPORTED;   // index list lives in shared memory (48 KB)
+  if (seq <= kEvictRegMaxSeq)
+    return launch_evict_regs<false>(score, nullptr, k, v, kv_cache, indices, batch, seq, heads, head_dim * elem_bytes, 0,
+                                    budget, 0, stream);
   const size_t smem_idx = (size_t)budget * sizeof(int32_t);
   const size_t key_bytes = skewed_words(seq) * sizeof(uint32_t);   // padded key array
   const int staged = smem_idx + key_bytes <= 200 * 1024 ? 1 : 0;
