@@ -111,9 +111,9 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // ---------------------------------------------------------------------------
 // RMSNorm.  out = T(x * rsqrt(mean(x^2) + eps)) * w, the last product taken in T
 // exactly as the reference does (csrc/norm.cu:54).
-// One warp per row, the row kept in registers: MAXV 16-byte vectors per lane.  FUSED_ADD: x = input + residual, residual <- T(x), and the second
-// phase re-reads the ROUNDED residual like csrc/norm.cu:80 (variance from the
-// unrounded sum, csrc/norm.cu:68-70).
+// The row is kept in registers between the sum and the scaling.  FUSED_ADD: x = input + residual, residual <- T(x), and
+// the second phase sees the ROUNDED residual like csrc/norm.cu:80 (variance from the unrounded sum, csrc/norm.cu:68-70).
+// Short rows: a warp each, MAXV 16-byte vectors per lane.
 // ---------------------------------------------------------------------------
 template <typename T, int MAXV, bool FUSED_ADD, int THREADS>
 __global__ void __launch_bounds__(THREADS)
@@ -134,38 +134,31 @@ rms_norm_rows_kernel(T* __restrict__ out, T* __restrict__ input, T* __restrict__
     float ss = 0.f;
     if constexpr (FUSED_ADD) {
       T* res_row = residual + row * hidden;
-      // the input row is loaded whole, the residual row in two halves (each half's loads are issued together, before
-      // that half's stores): the second operand never needs more than half a row of registers, which lets more
-      // rows be resident per SM
-      constexpr int HV = MAXV >= 8 ? (MAXV + 1) / 2 : MAXV;
+      uint4 rres[MAXV];
 #pragma unroll
       for (int v = 0; v < MAXV; ++v) {
         const int idx = lane + v * 32;
         if (idx < nvec) raw[v] = ld_16(in_row + (int64_t)idx * VN);
       }
 #pragma unroll
-      for (int h0 = 0; h0 < MAXV; h0 += HV) {
-        uint4 rres[HV];
+      for (int v = 0; v < MAXV; ++v) {
+        const int idx = lane + v * 32;
+        if (idx < nvec) rres[v] = ld_16(res_row + (int64_t)idx * VN);
+      }
 #pragma unroll
-        for (int v = 0; v < HV; ++v) {
-          const int idx = lane + (h0 + v) * 32;
-          if (idx < nvec) rres[v] = ld_16(res_row + (int64_t)idx * VN);
-        }
+      for (int v = 0; v < MAXV; ++v) {
+        const int idx = lane + v * 32;
+        if (idx < nvec) {
+          float x[VN], r[VN];
+          unpack16<T>(raw[v], x);
+          unpack16<T>(rres[v], r);
 #pragma unroll
-        for (int v = 0; v < HV; ++v) {
-          const int idx = lane + (h0 + v) * 32;
-          if (idx < nvec) {
-            float x[VN], r[VN];
-            unpack16<T>(raw[h0 + v], x);
-            unpack16<T>(rres[v], r);
-#pragma unroll
-            for (int i = 0; i < VN; ++i) {
-              x[i] += r[i];
-              ss += x[i] * x[i];      // variance from the unrounded sum (csrc/norm.cu:68-70)
-            }
-            raw[h0 + v] = pack16<T>(x);    // phase two sees the rounded residual (csrc/norm.cu:80)
-            st_16(res_row + (int64_t)idx * VN, raw[h0 + v]);
+          for (int i = 0; i < VN; ++i) {
+            x[i] += r[i];
+            ss += x[i] * x[i];      // variance from the unrounded sum (csrc/norm.cu:68-70)
           }
+          raw[v] = pack16<T>(x);    // phase two sees the rounded residual (csrc/norm.cu:80)
+          st_16(res_row + (int64_t)idx * VN, raw[v]);
         }
       }
     } else {
@@ -195,6 +188,69 @@ rms_norm_rows_kernel(T* __restrict__ out, T* __restrict__ input, T* __restrict__
         unpack16<T>(raw[v], x);
         st_16(out_row + (int64_t)idx * VN, scale_round_mul<T>(x, inv, ld_16(weight + (int64_t)idx * VN)));
       }
+    }
+  }
+}
+
+// One BLOCK per row, MAXV vectors per thread, all of a row's loads in flight at once.
+template <typename T, int MAXV, bool FUSED_ADD, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+rms_norm_block_kernel(T* __restrict__ out, T* __restrict__ input, T* __restrict__ residual, const T* __restrict__ weight,
+                      float epsilon, int hidden) {
+  constexpr int VN = 16 / sizeof(T);
+  __shared__ float red[THREADS / 32];
+  const int nvec = hidden / VN;
+  const int64_t row = (int64_t)blockIdx.x * hidden;
+  T* in_row = input + row;
+  pdl_wait();
+  uint4 raw[MAXV], w[MAXV];
+#pragma unroll
+  for (int v = 0; v < MAXV; ++v) {
+    const int idx = threadIdx.x + v * THREADS;
+    if (idx < nvec) raw[v] = ld_16(in_row + idx * VN);
+  }
+  if constexpr (FUSED_ADD) {
+#pragma unroll
+    for (int v = 0; v < MAXV; ++v) {   // (the weights' registers hold the residual first)
+      const int idx = threadIdx.x + v * THREADS;
+      if (idx < nvec) w[v] = ld_16(residual + row + idx * VN);
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int v = 0; v < MAXV; ++v) {
+    const int idx = threadIdx.x + v * THREADS;
+    if (idx < nvec) {
+      float x[VN];
+      unpack16<T>(raw[v], x);
+      if constexpr (FUSED_ADD) {
+        float r[VN];
+        unpack16<T>(w[v], r);
+#pragma unroll
+        for (int i = 0; i < VN; ++i) x[i] += r[i];
+        raw[v] = pack16<T>(x);    // phase two sees the rounded residual, the variance the unrounded sum
+        st_16(residual + row + idx * VN, raw[v]);
+      }
+#pragma unroll
+      for (int i = 0; i < VN; ++i) ss += x[i] * x[i];
+      w[v] = ld_16(weight + idx * VN);
+    }
+  }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float total = 0.f;
+#pragma unroll
+  for (int i = 0; i < THREADS / 32; ++i) total += red[i];
+  const float inv = rsqrtf(total / (float)hidden + epsilon);
+  T* out_row = (FUSED_ADD ? input : out) + row;
+#pragma unroll
+  for (int v = 0; v < MAXV; ++v) {
+    const int idx = threadIdx.x + v * THREADS;
+    if (idx < nvec) {
+      float x[VN];
+      unpack16<T>(raw[v], x);
+      st_16(out_row + idx * VN, scale_round_mul<T>(x, inv, w[v]));
     }
   }
 }
@@ -242,23 +298,29 @@ int launch_rms_norm(void* out, void* input, void* residual, const void* weight, 
   T* res = (T*)residual;
   const T* w = (const T*)weight;
   cudaError_t launched;
-  if (vec_ok && nvec <= 32 * 32) {
-    // One row per warp, small blocks (4 warps): the register footprint of a row (MAXV 16-byte vectors per lane) limits
-    // an SM to a few hundred resident threads, and with small blocks those threads belong to several blocks that
-    // start and finish at different times, so the load phase of one block overlaps the store phase of another.
+  // A block per row, except for many rows of at most 128 vectors, which take a warp each: a warp that holds 8 to 32 vectors
+  // per lane has a long serial part (all that a launch of a few rows consists of) and leaves an SM a few hundred threads,
+  // while a block with one vector per thread is mostly its barrier.  Measured, warp -> block per row (fp16, us): hidden
+  // 4096, 8 rows 5.4 -> 1.4, 1024 rows 6.2 -> 2.9, 4096 rows 11.8 -> 7.8; with the residual added 6.9 -> 1.7, 8.0 -> 4.0,
+  // 18.2 -> 12.1; hidden 1024, 8 rows 2.3 -> 1.4, 1024 rows 2.5 -> 1.8, 4096 rows 3.1 -> 3.5; fp32, hidden 4096, 8192 rows
+  // 55 -> 40.
+  if (vec_ok && (nvec > 128 || num_tokens <= 1024) && nvec <= 4 * 256 && num_tokens <= INT32_MAX) {
+#define B200_RMS_BLOCK(MAXV_, THREADS_)                                                                                   \
+  launched = launch_kernel(rms_norm_block_kernel<T, MAXV_, FUSED_ADD, THREADS_>, (unsigned)num_tokens, THREADS_, 0, stream, 1, \
+                           o, in, res, w, eps, hidden)
+    if (nvec <= 256) B200_RMS_BLOCK(2, 128);
+    else if (nvec <= 512) B200_RMS_BLOCK(2, 256);
+    else B200_RMS_BLOCK(4, 256);
+#undef B200_RMS_BLOCK
+  } else if (vec_ok && nvec <= 128) {
+    // small blocks (4 warps) start and finish at different times, so the load phase of one overlaps the store phase of another
     constexpr int TH = 128;
-    static const int env_grid = std::getenv("B200_RMS_GRID_PER_SM") ? std::atoi(std::getenv("B200_RMS_GRID_PER_SM")) : 0;
-    const int per_sm = env_grid > 0 ? env_grid : 16;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((num_tokens + TH / 32 - 1) / (TH / 32), (int64_t)sms * per_sm));
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((num_tokens + TH / 32 - 1) / (TH / 32), (int64_t)sms * 16));
 #define B200_RMS_LAUNCH(MAXV_)                                                                                        \
   launched = launch_kernel(rms_norm_rows_kernel<T, MAXV_, FUSED_ADD, TH>, grid, TH, 0, stream, 1, o, in, res, w, eps, \
                            num_tokens, hidden)
     if (nvec <= 64) B200_RMS_LAUNCH(2);
-    else if (nvec <= 128) B200_RMS_LAUNCH(4);
-    else if (nvec <= 256) B200_RMS_LAUNCH(8);
-    else if (nvec <= 448) B200_RMS_LAUNCH(14);
-    else if (nvec <= 512) B200_RMS_LAUNCH(16);
-    else B200_RMS_LAUNCH(32);
+    else B200_RMS_LAUNCH(4);
 #undef B200_RMS_LAUNCH
   } else {
     const int grid = (int)std::min<int64_t>(num_tokens, (int64_t)sms * 8);
@@ -403,9 +465,10 @@ template <typename T, int HEAD_DIM>
 __global__ void __launch_bounds__(256)
 rotary_online_kernel(const int32_t* __restrict__ positions, T* __restrict__ query, T* __restrict__ key,
                      int64_t num_tokens, int heads, int kv_heads, int64_t q_stride, int64_t k_stride,
-                     float theta, int vec_ok) {
+                     double log2_theta, int vec_ok, int parts) {
   // One WARP per token: its D/2 angles go to a warp-private slice of shared memory (no block-wide barrier),
-  // then the warp rotates every query and key head of the token.
+  // then the warp rotates every query and key head of the token -- or, with `parts` > 1 (few tokens), one of `parts`
+  // interleaved shares of them.
   constexpr int HALF = HEAD_DIM / 2;
   constexpr int VN = 16 / sizeof(T);
   constexpr int WARPS = 256 / 32;
@@ -419,14 +482,14 @@ rotary_online_kernel(const int32_t* __restrict__ positions, T* __restrict__ quer
   // inverse frequencies theta^(-2i/D) of the elements this lane evaluates (i = lane, lane + 32, ...), in fp64
   constexpr int PER_LANE = HALF / 32;
   double inv_freq[PER_LANE];
-  {
-    const double l2t = log2((double)theta);
 #pragma unroll
-    for (int t = 0; t < PER_LANE; ++t) inv_freq[t] = exp2(-(double)(2 * (lane + 32 * t)) / (double)HEAD_DIM * l2t);
-  }
+  for (int t = 0; t < PER_LANE; ++t) inv_freq[t] = exp2(-(double)(2 * (lane + 32 * t)) / (double)HEAD_DIM * log2_theta);
   pdl_wait();   // (the frequencies above need no memory)
   constexpr double kTwoPi = 6.283185307179586476925286766559, kInvTwoPi = 0.15915494309189533576888376337251;
-  for (int64_t tok = warp_global; tok < num_tokens; tok += warp_count) {
+  const int64_t items = num_tokens * parts;
+  for (int64_t item = warp_global; item < items; item += warp_count) {
+    const int64_t tok = parts == 1 ? item : item / parts;
+    const int part = (int)(item - tok * parts);
     const double pos = (double)positions[tok];
     __syncwarp();
 #pragma unroll
@@ -444,7 +507,7 @@ rotary_online_kernel(const int32_t* __restrict__ positions, T* __restrict__ quer
       // warp keeps 4 KB in flight (with one pair per step the kernel was bound by load latency at ~70 % of the
       // copy rate)
       constexpr int U = 4;
-      for (int g0 = lane; g0 < total; g0 += 32 * U) {
+      for (int g0 = part * 32 * U + lane; g0 < total; g0 += parts * 32 * U) {
         T* base[U];
         int col[U];
         uint4 rx[U], ry[U];
@@ -480,7 +543,7 @@ rotary_online_kernel(const int32_t* __restrict__ positions, T* __restrict__ quer
       }
     } else {
       const int total = (heads + kv_heads) * HALF;
-      for (int g = lane; g < total; g += 32) {
+      for (int g = part * 32 + lane; g < total; g += parts * 32) {
         const int head = g / HALF;
         const int c = g - head * HALF;
         T* base = (head < heads) ? query + tok * q_stride + (int64_t)head * HEAD_DIM
@@ -500,22 +563,28 @@ int launch_rotary(const int32_t* positions, void* query, void* key, int64_t num_
   constexpr int VN = 16 / sizeof(T);
   const int vec_ok = aligned16(query) && aligned16(key) && (q_stride % VN == 0) && (k_stride % VN == 0) &&
                      ((head_dim / 2) % VN == 0);
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((num_tokens + 7) / 8, (int64_t)sm_count() * 8));
+  // Few tokens: a token's heads are shared out over `parts` warps -- at most as many as there are steps of 128 vector pairs, and
+  // no more than 16 warps per SM in all.  Measured, 1 warp -> parts per token (fp16, 64 heads of 128, us): 8 tokens 5.9 ->
+  // 2.7, 592 tokens 6.1 -> 3.8; from 1024 tokens on the two are equal.
+  const int64_t steps = ((int64_t)(heads + kv_heads) * (head_dim / 2 / VN) + 127) / 128;
+  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t)sm_count() * 16 / num_tokens));
+  const double log2_theta = std::log2((double)theta);
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((num_tokens * parts + 7) / 8, (int64_t)sm_count() * 8));
   T* q = (T*)query;
   T* k = (T*)key;
   cudaError_t launched;
   switch (head_dim) {
     case 64:
       launched = launch_kernel(rotary_online_kernel<T, 64>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
-                               kv_heads, q_stride, k_stride, theta, vec_ok);
+                               kv_heads, q_stride, k_stride, log2_theta, vec_ok, parts);
       break;
     case 128:
       launched = launch_kernel(rotary_online_kernel<T, 128>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
-                               kv_heads, q_stride, k_stride, theta, vec_ok);
+                               kv_heads, q_stride, k_stride, log2_theta, vec_ok, parts);
       break;
     case 256:
       launched = launch_kernel(rotary_online_kernel<T, 256>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
-                               kv_heads, q_stride, k_stride, theta, vec_ok);
+                               kv_heads, q_stride, k_stride, log2_theta, vec_ok, parts);
       break;
     default:
       return B200_ERR_UNSUPPORTED;
