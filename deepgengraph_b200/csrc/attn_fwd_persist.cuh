@@ -32,9 +32,9 @@ struct TileInfo {
 
 // Work order: the (batch, head) units are taken in groups of `group_heads`; inside a group the items run
 // tile-major, heaviest query tile first (all heads' last tile, then all heads' second-to-last tile, ...).
-// The K/V of one group (group_heads x 2 x kv_len x D x 2 bytes; 32 MB for 16 heads at 4096 keys) stay
-// L2-resident while ~2 x #SM CTAs walk it, and the launch ends on the LIGHTEST tiles, so that the CTAs drain
-// within a few key blocks of each other (longest-processing-time-first order).
+// The K/V of one group (32 MB for 16 heads at 4096 keys; see the launch below) stay L2-resident while ~2 x #SM CTAs walk it,
+// and the launch ends on the LIGHTEST tiles, so that the CTAs drain within a few key blocks of each other
+// (longest-processing-time-first order).
 __device__ __forceinline__ TileInfo decode_item(int item, const FwdParams& p, const SchedParams& sp, int bn) {
   TileInfo t;
   const int per_group = sp.group_heads * sp.n_q_tiles;
@@ -534,10 +534,17 @@ int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const 
   if (rc != B200_OK) return rc;
   sp.n_q_tiles = (p.q_len + 127) / 128;
   sp.total_items = p.batch * p.heads * sp.n_q_tiles;
-  // group size: K/V of a group within a quarter of L2 (~32 MB), at least 1 and at most 32 units
+  // Group size.  Where all of K and V stay in L2 (126 MB) beside q and out, one group: the whole launch then runs heaviest
+  // tile first and ends on the lightest.  Else as many units as have a quarter of L2 of K/V, at least 1 and at most 32.  K/V
+  // of a head count once for the query heads that share it.  Measured, groups -> one group (bf16, causal, us): 2 x 12 heads,
+  // 3000 tokens, head_dim 256 (74 MB) 114.5 -> 101.8; 4 x 32/8 heads, 1024 tokens (17 MB) 47.5 -> 45.9; 2 x 32/8, 777
+  // queries, 3001 keys (25 MB) 85.9 -> 84.1; 8 x 32, 512 tokens (67 MB) 37.3 -> 36.4; but 32 heads, 8192 tokens (134 MB)
+  // 454.9 -> 469.7 and 4 x 32, 4096 tokens (268 MB) 494.5 -> 559.6.
   {
-    const int64_t kv_bytes_per_unit = (int64_t)2 * p.kv_len * D_ * 2;
-    int gh = (int)std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)32 << 20) / kv_bytes_per_unit));
+    const int64_t kv_bytes_per_head = (int64_t)2 * p.kv_len * D_ * 2;
+    const int units = p.batch * p.heads, group = p.heads / p.kv_heads;
+    const bool in_l2 = kv_bytes_per_head * p.batch * p.kv_heads <= ((int64_t)80 << 20);
+    int gh = in_l2 ? units : (int)std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)32 << 20) * group / kv_bytes_per_head));
     static const char* env = std::getenv("B200_ATTN_GROUP_HEADS");
     if (env != nullptr && std::atoi(env) > 0) gh = std::atoi(env);
     sp.group_heads = gh;
