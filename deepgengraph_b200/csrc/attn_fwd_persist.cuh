@@ -544,7 +544,14 @@ int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const 
     const int64_t kv_bytes_per_head = (int64_t)2 * p.kv_len * D_ * 2;
     const int units = p.batch * p.heads, group = p.heads / p.kv_heads;
     const bool in_l2 = kv_bytes_per_head * p.batch * p.kv_heads <= ((int64_t)80 << 20);
-    int gh = in_l2 ? units : (int)std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)32 << 20) * group / kv_bytes_per_head));
+    int gh = units;
+    if (!in_l2) {
+      // groups of one size (a small last one drains badly: 4 x 16/8 heads, 6000 tokens, 64 units: groups of 21 -- 546 us, of
+      // 16 -- 509), not cut between query heads that share K/V
+      const int64_t fit = std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)32 << 20) * group / kv_bytes_per_head));
+      const int n_groups = (int)((units + fit - 1) / fit);
+      gh = ((units + n_groups - 1) / n_groups + group - 1) / group * group;
+    }
     static const char* env = std::getenv("B200_ATTN_GROUP_HEADS");
     if (env != nullptr && std::atoi(env) > 0) gh = std::atoi(env);
     sp.group_heads = gh;
