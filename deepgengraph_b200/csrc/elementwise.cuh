@@ -461,14 +461,18 @@ int launch_act_and_mul(void* out, const void* in, int64_t num_tokens, int d, cud
 // fp64 too, and only the reduced angle goes through the fp32 sine / cosine
 // intrinsics, which are accurate to ~5e-7 on that range.
 // ---------------------------------------------------------------------------
-template <typename T, int HEAD_DIM>
-__global__ void __launch_bounds__(256)
+template <typename T, int HEAD_DIM, bool SHARED_OUT>
+__global__ void __launch_bounds__(256, SHARED_OUT ? 1 : 2)
 rotary_online_kernel(const int32_t* __restrict__ positions, T* __restrict__ query, T* __restrict__ key,
                      int64_t num_tokens, int heads, int kv_heads, int64_t q_stride, int64_t k_stride,
-                     double log2_theta, int vec_ok, int parts) {
+                     double log2_theta, int vec_ok, int n_parts) {
   // One WARP per token: its D/2 angles go to a warp-private slice of shared memory (no block-wide barrier),
-  // then the warp rotates every query and key head of the token -- or, with `parts` > 1 (few tokens), one of `parts`
-  // interleaved shares of them.
+  // then the warp rotates every query and key head of the token -- or, SHARED_OUT (few tokens), one of `n_parts`
+  // interleaved shares of them.  Two instantiations because the step of the loop over the vectors has to be a constant: with
+  // a run-time step the compiler no longer has the next step's loads in flight under this one's stores.  Measured, run-time
+  // -> constant step (bf16, 8192 tokens, graph replay, us): 16 + 8 heads of 256 44.9 -> 33.5 (6.0 TB/s), 32 + 32 of 128
+  // 52.0 -> 46.6 (5.8 TB/s); fp16 41.7 -> 33.6 and 46.0 -> 46.6 (there the run-time form leaves room for a third block).
+  const int parts = SHARED_OUT ? n_parts : 1;
   constexpr int HALF = HEAD_DIM / 2;
   constexpr int VN = 16 / sizeof(T);
   constexpr int WARPS = 256 / 32;
@@ -488,7 +492,7 @@ rotary_online_kernel(const int32_t* __restrict__ positions, T* __restrict__ quer
   constexpr double kTwoPi = 6.283185307179586476925286766559, kInvTwoPi = 0.15915494309189533576888376337251;
   const int64_t items = num_tokens * parts;
   for (int64_t item = warp_global; item < items; item += warp_count) {
-    const int64_t tok = parts == 1 ? item : item / parts;
+    const int64_t tok = SHARED_OUT ? item / parts : item;
     const int part = (int)(item - tok * parts);
     const double pos = (double)positions[tok];
     __syncwarp();
@@ -564,31 +568,36 @@ int launch_rotary(const int32_t* positions, void* query, void* key, int64_t num_
   const int vec_ok = aligned16(query) && aligned16(key) && (q_stride % VN == 0) && (k_stride % VN == 0) &&
                      ((head_dim / 2) % VN == 0);
   // Few tokens: a token's heads are shared out over `parts` warps -- at most as many as there are steps of 128 vector pairs, and
-  // no more than 16 warps per SM in all.  Measured, 1 warp -> parts per token (fp16, 64 heads of 128, us): 8 tokens 5.9 ->
-  // 2.7, 592 tokens 6.1 -> 3.8; from 1024 tokens on the two are equal.
+  // no more than 16 warps per SM in all.  Measured, 1 warp -> parts per token (graph replay, us): fp16, 64 heads of 128: 8
+  // tokens 6.1 -> 2.3, 592 tokens 6.4 -> 3.5, 1024 tokens (2 parts) 5.8 -> 5.4.  Every warp evaluates a token's angles in
+  // fp64, which at head_dim 256 is half of what two warps per token would do: two are taken there only up to 8 warps per SM
+  // (8 + 4 heads, bf16: 592 tokens 3.2 -> 3.0, but 700 tokens 3.2 -> 4.0;  16 + 8 heads, 1024 tokens 4.9 -> 6.2).
   const int64_t steps = ((int64_t)(heads + kv_heads) * (head_dim / 2 / VN) + 127) / 128;
-  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t)sm_count() * 16 / num_tokens));
+  const int sms = sm_count();
+  int parts = (int)std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t)sms * 16 / num_tokens));
+  if (head_dim == 256 && parts == 2 && num_tokens * 2 > (int64_t)sms * 8) parts = 1;
   const double log2_theta = std::log2((double)theta);
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((num_tokens * parts + 7) / 8, (int64_t)sm_count() * 8));
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((num_tokens * parts + 7) / 8, (int64_t)sms * 8));
   T* q = (T*)query;
   T* k = (T*)key;
   cudaError_t launched;
-  switch (head_dim) {
-    case 64:
-      launched = launch_kernel(rotary_online_kernel<T, 64>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
-                               kv_heads, q_stride, k_stride, log2_theta, vec_ok, parts);
-      break;
-    case 128:
-      launched = launch_kernel(rotary_online_kernel<T, 128>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
-                               kv_heads, q_stride, k_stride, log2_theta, vec_ok, parts);
-      break;
-    case 256:
-      launched = launch_kernel(rotary_online_kernel<T, 256>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads,
-                               kv_heads, q_stride, k_stride, log2_theta, vec_ok, parts);
-      break;
-    default:
-      return B200_ERR_UNSUPPORTED;
+#define B200_ROTARY(D_, SHARED_OUT_)                                                                                      \
+  launched = launch_kernel(rotary_online_kernel<T, D_, SHARED_OUT_>, grid, 256, 0, stream, 1, positions, q, k, num_tokens, heads, \
+                           kv_heads, q_stride, k_stride, log2_theta, vec_ok, parts)
+#define B200_ROTARY_D(D_) \
+  if (parts > 1) B200_ROTARY(D_, true); \
+  else B200_ROTARY(D_, false)
+  if (head_dim == 64) {
+    B200_ROTARY_D(64);
+  } else if (head_dim == 128) {
+    B200_ROTARY_D(128);
+  } else if (head_dim == 256) {
+    B200_ROTARY_D(256);
+  } else {
+    return B200_ERR_UNSUPPORTED;
   }
+#undef B200_ROTARY_D
+#undef B200_ROTARY
   B200_CUDA_TRY(launched);
   return B200_OK;
 }
