@@ -88,23 +88,30 @@ def run_sharded(fn, q, k, v, world: int, rank: int, extra=None, dense: bool = Tr
 # up to its last row only, and no reduction follows.  (The score variants sum over queries; cutting their rows would
 # need one -- they shard by units only.)
 # --------------------------------------------------------------------------------------------
+FEW_ROWS = 16   # up to so many query rows per K/V head go to csrc/attn_decode.cuh (kDecodeRows)
+
+
 def row_ranges(q_len: int, kv_len: int, parts: int, causal: bool = True, window: int = 0,
                align: int = 128) -> List[Tuple[int, int]]:
   """Cuts the query rows [0, q_len) into `parts` contiguous ranges of about equal WORK -- visible (query, key) pairs
   under the causal / sliding-window mask -- with boundaries on multiples of `align` rows: query tiles stay whole, so
-  a range computes exactly what the full problem computes for those rows.  Fewer than `parts` ranges come back when
-  there are fewer tiles; no range is empty."""
+  a range computes exactly what the full problem computes for those rows.  A last tile of no more than
+  `FEW_ROWS` rows stays with the tile before it: alone it would be a problem of few query rows, which another kernel takes.
+  Fewer than `parts` ranges come back when there are fewer tiles; no range is empty."""
   if parts <= 0 or q_len <= 0 or kv_len < q_len:
     raise ValueError(f"bad row split: q_len {q_len}, kv_len {kv_len}, parts {parts}")
   delta = kv_len - q_len
   n_tiles = -(-q_len // align)
+  if n_tiles > 1 and q_len - (n_tiles - 1) * align <= FEW_ROWS:
+    n_tiles -= 1
+  first = [t * align for t in range(n_tiles)] + [q_len]
 
   def visible(i):
     hi = min(i + delta, kv_len - 1) if causal else kv_len - 1
     lo = max(0, i + delta - window + 1) if (causal and window > 0) else 0
     return hi - lo + 1
-  tile_work = [sum(visible(i) for i in (t * align, min(q_len, (t + 1) * align) - 1)) * 0.5 *
-               (min(q_len, (t + 1) * align) - t * align) for t in range(n_tiles)]   # trapezoid: work is linear per tile
+  tile_work = [sum(visible(i) for i in (first[t], first[t + 1] - 1)) * 0.5 * (first[t + 1] - first[t])
+               for t in range(n_tiles)]   # trapezoid: work is linear per tile
   total = sum(tile_work)
   parts = min(parts, n_tiles)
   cuts, acc, nxt = [0], 0.0, 1
@@ -115,7 +122,7 @@ def row_ranges(q_len: int, kv_len: int, parts: int, causal: bool = True, window:
       cuts.append(t + 1)
       nxt += 1
   cuts.append(n_tiles)
-  return [(cuts[i] * align, min(q_len, cuts[i + 1] * align)) for i in range(len(cuts) - 1) if cuts[i + 1] > cuts[i]]
+  return [(first[cuts[i]], first[cuts[i + 1]]) for i in range(len(cuts) - 1) if cuts[i + 1] > cuts[i]]
 
 
 def slice_rows(q, k, v, r0: int, r1: int, causal: bool = True):

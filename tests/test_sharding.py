@@ -187,3 +187,13 @@ def test_slice_rows_keeps_the_mask_alignment():
       qs, ks, vs = sh.slice_rows(q, k, v, r0, r1, causal=True)
       part = rm.attention_ref(qs, ks, vs, causal=True, window=window)["out"]
       torch.testing.assert_close(part, full[:, r0:r1], rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("q_len,kv_len,parts", [(1040, 4096, 9), (260, 8192, 2), (1032, 1032, 8), (140, 140, 2), (17, 64, 3), (16, 4096, 4),
+                                                (1041, 4096, 9)])
+def test_no_row_range_is_a_lone_tile_of_few_rows(q_len, kv_len, parts):
+  # up to 16 query rows per K/V head are another kernel's work: such a range would not have the full problem's bits
+  ranges = sh.row_ranges(q_len, kv_len, parts)
+  assert ranges[0][0] == 0 and ranges[-1][1] == q_len and all(a[1] == b[0] for a, b in zip(ranges, ranges[1:]))
+  assert all(r0 % 128 == 0 for r0, _ in ranges)
+  assert len(ranges) == 1 or min(r1 - r0 for r0, r1 in ranges) > 16
