@@ -44,14 +44,24 @@ def needs_torch_build():
   return _older(TORCH_EXT, TORCH_DEPS)
 
 
+def _temporary(target):
+  return f"{target}.{os.getpid()}.tmp"   # of this process: several ranks may build at the same time
+
+
 def _run(cmd, target, verbose):
-  res = subprocess.run(cmd, capture_output=True, text=True)
-  if res.returncode != 0:
-    sys.stderr.write(res.stdout + res.stderr)
-    raise RuntimeError(f"{os.path.basename(cmd[0])} failed building {os.path.basename(target)}")
-  if verbose:
-    sys.stderr.write(res.stdout + res.stderr)
-  os.replace(target + ".tmp", target)
+  """Runs `cmd`, which writes _temporary(target), and puts the result in place in one step."""
+  tmp = _temporary(target)
+  try:
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+      sys.stderr.write(res.stdout + res.stderr)
+      raise RuntimeError(f"{os.path.basename(cmd[0])} failed building {os.path.basename(target)}")
+    if verbose:
+      sys.stderr.write(res.stdout + res.stderr)
+    os.replace(tmp, target)
+  finally:
+    if os.path.exists(tmp):
+      os.remove(tmp)
 
 
 def build(force=False, verbose=False):
@@ -60,7 +70,7 @@ def build(force=False, verbose=False):
     cmd = [
         _nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
         "-shared", "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v" if verbose else "-O3",
-        "-o", LIB + ".tmp",
+        "-o", _temporary(LIB),
     ] + [os.path.join(CSRC, s) for s in SOURCES] + ["-lcudart"]
     _run(cmd, LIB, verbose)
   build_torch(force, verbose)
@@ -79,7 +89,7 @@ def build_torch(force=False, verbose=False):
   cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
   cmd += ["-isystem" + p for p in includes]
-  cmd += ["-o", TORCH_EXT + ".tmp", os.path.join(CSRC, "torch_binding.cpp"), "-L" + torch_lib, "-L" + CSRC,
+  cmd += ["-o", _temporary(TORCH_EXT), os.path.join(CSRC, "torch_binding.cpp"), "-L" + torch_lib, "-L" + CSRC,
           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-l:libb200attn.so", "-Wl,-rpath,$ORIGIN"]
   _run(cmd, TORCH_EXT, verbose)
   return TORCH_EXT
