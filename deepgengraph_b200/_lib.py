@@ -83,17 +83,18 @@ def load():
 
 
 class _Host:
-  """The functions of b200torch.so; the module is loaded (built first if needed) on the first use of any of them."""
+  """The functions of b200torch.*.so; the module is loaded (built first if needed) on the first use of any of them."""
 
   def __getattr__(self, name):
     load()      # the CUDA library it links against
+    path = _build.torch_ext()
     if _build.needs_torch_build():
       try:
         _build.build_torch()
       except Exception as e:
-        if not os.path.exists(_build.TORCH_EXT):
-          raise RuntimeError(f"b200torch.so is missing and could not be built: {e}") from e
-    loader = importlib.machinery.ExtensionFileLoader("b200torch", _build.TORCH_EXT)
+        if not os.path.exists(path):
+          raise RuntimeError(f"{path} is missing and could not be built: {e}") from e
+    loader = importlib.machinery.ExtensionFileLoader("b200torch", path)
     mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200torch", loader))
     loader.exec_module(mod)
     self.__dict__.update({n: f for n, f in vars(mod).items() if not n.startswith("_")})

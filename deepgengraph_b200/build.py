@@ -3,7 +3,8 @@
   libb200attn.so   the CUDA library (sm_100a only): one translation unit (b200attn.cu) compiled with nvcc; it links only the
                    CUDA runtime (the driver's tensor-map encoder is looked up at run time), so it can be loaded with
                    ctypes from any host language
-  b200torch.so     the torch host path of the public operators (torch_binding.cpp), linked against the library
+  b200torch.<torch version>.<ABI tags>.so
+                   the torch host path of the public operators (torch_binding.cpp), linked against the library
 """
 import os
 import shutil
@@ -14,7 +15,6 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libb200attn.so")
-TORCH_EXT = os.path.join(CSRC, "b200torch.so")
 SOURCES = ["b200attn.cu"]
 HEADER = os.path.join("..", "..", "include", "b200attn.h")
 DEPS = ["b200attn.cu", "common.cuh", "elementwise.cuh", "attn_fwd.cuh", "attn_fwd_persist.cuh", "attn_decode.cuh", "attn_sweep.cuh", "kv_evict.cuh",
@@ -40,8 +40,16 @@ def needs_build():
   return _older(LIB, DEPS)
 
 
+def torch_ext():
+  """Path of the torch host path for this interpreter: the name carries what its binary interface depends on, so that another
+  torch or Python finds no file and builds its own."""
+  import torch
+  abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
+  return os.path.join(CSRC, f"b200torch.{torch.__version__}.cxx11abi{abi}.{sysconfig.get_config_var('SOABI')}.so")
+
+
 def needs_torch_build():
-  return _older(TORCH_EXT, TORCH_DEPS)
+  return _older(torch_ext(), TORCH_DEPS)
 
 
 def _temporary(target):
@@ -79,8 +87,9 @@ def build(force=False, verbose=False):
 
 def build_torch(force=False, verbose=False):
   """The torch host path; needs only a C++ compiler and torch's headers."""
+  target = torch_ext()
   if not (force or needs_torch_build()):
-    return TORCH_EXT
+    return target
   import torch
   from torch.utils import cpp_extension
   cuda_home = os.path.dirname(os.path.dirname(_nvcc()))
@@ -89,10 +98,10 @@ def build_torch(force=False, verbose=False):
   cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
   cmd += ["-isystem" + p for p in includes]
-  cmd += ["-o", _temporary(TORCH_EXT), os.path.join(CSRC, "torch_binding.cpp"), "-L" + torch_lib, "-L" + CSRC,
+  cmd += ["-o", _temporary(target), os.path.join(CSRC, "torch_binding.cpp"), "-L" + torch_lib, "-L" + CSRC,
           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-l:libb200attn.so", "-Wl,-rpath,$ORIGIN"]
-  _run(cmd, TORCH_EXT, verbose)
-  return TORCH_EXT
+  _run(cmd, target, verbose)
+  return target
 
 
 if __name__ == "__main__":
