@@ -10,6 +10,8 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import os
+import threading
+import warnings
 
 from . import build as _build
 
@@ -83,22 +85,44 @@ def load():
 
 
 class _Host:
-  """The functions of b200torch.*.so; the module is loaded (built first if needed) on the first use of any of them."""
+  """The functions of the torch host path (b200torch.*.so), loaded -- built first if needed -- on the first use of any of
+  them.  Where it can be neither built nor loaded there is one warning, and every function returns None: the operators then
+  take their Python path, which needs the CUDA library only."""
+  FUNCTIONS = ("attn_fwd", "attn_score", "attn_snapkv", "attn_corm", "attn_kf", "kv_evict", "norm", "act_and_mul", "rotary")
 
-  def __getattr__(self, name):
+  def __init__(self):
+    self._lock = threading.Lock()
+
+  def __getattr__(self, name):   # only reached while `name` is not set
+    if name not in self.FUNCTIONS:
+      raise AttributeError(name)
     load()      # the CUDA library it links against
+    with self._lock:
+      if name not in self.__dict__:
+        try:
+          self.__dict__.update(self._load())
+        except Exception as e:   # noqa: BLE001 -- no compiler, no headers, no loadable file: whatever it is, the path is optional
+          warnings.warn(f"the native host path of deepgengraph_b200 is not available ({type(e).__name__}: {e}); its operators "
+                        "take several microseconds more of host time per call", RuntimeWarning, stacklevel=3)
+          self.__dict__.update({n: _declined for n in self.FUNCTIONS})
+    return self.__dict__[name]
+
+  def _load(self):
     path = _build.torch_ext()
     if _build.needs_torch_build():
       try:
         _build.build_torch()
-      except Exception as e:
+      except Exception:   # a present file is still usable where no compiler is installed
         if not os.path.exists(path):
-          raise RuntimeError(f"{path} is missing and could not be built: {e}") from e
+          raise
     loader = importlib.machinery.ExtensionFileLoader("b200torch", path)
     mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200torch", loader))
     loader.exec_module(mod)
-    self.__dict__.update({n: f for n, f in vars(mod).items() if not n.startswith("_")})
-    return self.__dict__[name]
+    return {n: getattr(mod, n) for n in self.FUNCTIONS}
+
+
+def _declined(*args):
+  return None
 
 
 host = _Host()

@@ -4,7 +4,8 @@
                    CUDA runtime (the driver's tensor-map encoder is looked up at run time), so it can be loaded with
                    ctypes from any host language
   b200torch.<torch version>.<ABI tags>.so
-                   the torch host path of the public operators (torch_binding.cpp), linked against the library
+                   the torch host path of the public operators (torch_binding.cpp), linked against the library; optional: the
+                   operators run without it, with a slower host path
 """
 import os
 import shutil
@@ -17,8 +18,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libb200attn.so")
 SOURCES = ["b200attn.cu"]
 HEADER = os.path.join("..", "..", "include", "b200attn.h")
-DEPS = ["b200attn.cu", "common.cuh", "elementwise.cuh", "attn_fwd.cuh", "attn_fwd_persist.cuh", "attn_decode.cuh", "attn_sweep.cuh", "kv_evict.cuh",
-        HEADER]
+DEPS = ["b200attn.cu", "common.cuh", "elementwise.cuh", "attn_fwd.cuh", "attn_fwd_persist.cuh", "attn_decode.cuh",
+        "attn_sweep.cuh", "kv_evict.cuh", HEADER]
 TORCH_DEPS = ["torch_binding.cpp", HEADER]
 
 
@@ -73,20 +74,20 @@ def _run(cmd, target, verbose):
 
 
 def build(force=False, verbose=False):
-  """Compile what is missing or older than its sources. Returns the path of the CUDA library."""
-  if force or needs_build():
-    cmd = [
-        _nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
-        "-shared", "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v" if verbose else "-O3",
-        "-o", _temporary(LIB),
-    ] + [os.path.join(CSRC, s) for s in SOURCES] + ["-lcudart"]
-    _run(cmd, LIB, verbose)
-  build_torch(force, verbose)
+  """Compile the CUDA library if it is missing or older than its sources. Returns its path."""
+  if not force and not needs_build():
+    return LIB
+  cmd = [
+      _nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
+      "-shared", "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v" if verbose else "-O3",
+      "-o", _temporary(LIB),
+  ] + [os.path.join(CSRC, s) for s in SOURCES] + ["-lcudart"]
+  _run(cmd, LIB, verbose)
   return LIB
 
 
 def build_torch(force=False, verbose=False):
-  """The torch host path; needs only a C++ compiler and torch's headers."""
+  """The torch host path, after the library it is linked against; needs only a C++ compiler and torch's headers."""
   target = torch_ext()
   if not (force or needs_torch_build()):
     return target
@@ -105,4 +106,5 @@ def build_torch(force=False, verbose=False):
 
 
 if __name__ == "__main__":
-  print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+  for step in (build, build_torch):
+    print(step(force="--force" in sys.argv, verbose="-v" in sys.argv))
