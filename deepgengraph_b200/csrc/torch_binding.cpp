@@ -60,10 +60,10 @@ bool bool_arg(PyObject* o, bool* v) {
   return true;
 }
 
-// softmax scale: None or a non-positive number selects 1 / sqrt(head_dim)
+// softmax scale: None or a non-positive number selects 1 / sqrt(head_dim); the library refuses a NaN
 bool scale_arg(PyObject* o, int64_t head_dim, float* v) {
   double s = 0.0;
-  if (o != Py_None && !float_arg(o, &s)) return false;
+  if (o != Py_None && (!float_arg(o, &s) || std::isnan(s))) return false;
   *v = (float)(s > 0.0 ? s : 1.0 / std::sqrt((double)head_dim));
   return true;
 }
