@@ -397,9 +397,13 @@ __device__ __forceinline__ uint32_t regs_scan_counts(uint32_t sure, uint32_t tie
   return __reduce_add_sync(0xffffffffu, lane < wid ? warp_totals[lane] : 0u) + incl - own;
 }
 
+// CTAs per SM: 64 registers a thread for two.  RoCo with 32 keys per thread needs 95, and bounded to 64 would spill 216 bytes.
+template <int NK, bool ROCO>
+constexpr int kEvictRegCtas = NK == 32 && ROCO ? 1 : 2;
+
 // ROCO = false: the `budget` largest scores.  ROCO = true: the two-stage selection described above.
 template <int NK, bool ROCO>
-__global__ void __launch_bounds__(kEvictRegThreads)
+__global__ void __launch_bounds__(kEvictRegThreads, kEvictRegCtas<NK, ROCO>)
 kv_evict_regs_kernel(const float* __restrict__ score, const float* __restrict__ score_sq, const uint8_t* __restrict__ k,
                      const uint8_t* __restrict__ v, uint8_t* __restrict__ kv_cache, int32_t* __restrict__ indices_out,
                      int seq, int heads, int row_bytes, float q_len, int budget, int recent) {
@@ -542,8 +546,10 @@ int launch_kv_evict_topk(dim3 grid, size_t smem, cudaStream_t stream, const floa
   return B200_OK;
 }
 
-// CTAs per (batch, head): as many as are resident at once (two per SM), so that the launch has no second wave (each repeats
-// the selection, which reads a few KB of scores from L2), and at most 16.
+// CTAs per (batch, head): as many as are resident at once, so that the launch has no second wave (each repeats the selection,
+// which reads a few KB of scores from L2), and at most 16.  Measured, two CTAs per SM assumed for every
+// instantiation -> asked for and counted (32 heads, graph replay, us): RoCo 5000 keys 46.5 -> 32.3, 8192 37.2 -> 28.2, 12000 83.5 ->
+// 43.7, 16384 65.5 -> 36.3; largest scores 12000 keys 29.5 -> 23.8, 16384 31.5 -> 26.0.
 template <int NK, bool ROCO>
 int launch_evict_regs_nk(const float* score, const float* score_sq, const void* k, const void* v, void* kv_cache,
                          int32_t* indices, int batch, int seq, int heads, int row_bytes, int q_len, int budget, int recent,
@@ -558,7 +564,7 @@ int launch_evict_regs_nk(const float* score, const float* score_sq, const void* 
     configured_dev = dev;
   }
   const int units = batch * heads;
-  const dim3 grid(units, std::max(1, std::min(16, 2 * sm_count() / units)));
+  const dim3 grid(units, std::max(1, std::min(16, kEvictRegCtas<NK, ROCO> * sm_count() / units)));
   B200_CUDA_TRY(launch_kernel(kern, grid, kEvictRegThreads, smem, stream, 1, score, score_sq, (const uint8_t*)k,
                               (const uint8_t*)v, (uint8_t*)kv_cache, indices, seq, heads, row_bytes, (float)q_len, budget,
                               recent));
