@@ -192,13 +192,39 @@ rms_norm_rows_kernel(T* __restrict__ out, T* __restrict__ input, T* __restrict__
   }
 }
 
+// Sum of the W (4 or 8) warps' sums, pairwise: one after the other rounds a sum near the total at every step.  Both forms are the
+// same tree.  IN_FOURS needs fewer registers at a time, which two vectors per thread want (32 of them fill an SM: 8192 rows of
+// 3584, bf16, 17.8 us against 19.9); with four vectors it is the slower one (1024 rows of 4096, fp32, 4.6 us against 4.1).  By
+// shuffles the short rows lose 5 to 9 %.
+template <int W, bool IN_FOURS>
+__device__ __forceinline__ float add_pairwise(const float* red) {
+  if constexpr (IN_FOURS) {
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < W / 4; ++i) {
+      const float4 four = reinterpret_cast<const float4*>(red)[i];
+      sum += (four.x + four.y) + (four.z + four.w);
+    }
+    return sum;
+  } else {
+    float part[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) part[i] = red[i];
+#pragma unroll
+    for (int step = 1; step < W; step *= 2)
+#pragma unroll
+      for (int i = 0; i < W; i += 2 * step) part[i] += part[i + step];
+    return part[0];
+  }
+}
+
 // One BLOCK per row, MAXV vectors per thread, all of a row's loads in flight at once.
 template <typename T, int MAXV, bool FUSED_ADD, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 rms_norm_block_kernel(T* __restrict__ out, T* __restrict__ input, T* __restrict__ residual, const T* __restrict__ weight,
                       float epsilon, int hidden) {
   constexpr int VN = 16 / sizeof(T);
-  __shared__ float red[THREADS / 32];
+  __shared__ __align__(16) float red[THREADS / 32];
   const int nvec = hidden / VN;
   const int64_t row = (int64_t)blockIdx.x * hidden;
   T* in_row = input + row;
@@ -239,9 +265,7 @@ rms_norm_block_kernel(T* __restrict__ out, T* __restrict__ input, T* __restrict_
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
-  float total = 0.f;
-#pragma unroll
-  for (int i = 0; i < THREADS / 32; ++i) total += red[i];
+  const float total = add_pairwise<THREADS / 32, MAXV == 2>(red);
   const float inv = rsqrtf(total / (float)hidden + epsilon);
   T* out_row = (FUSED_ADD ? input : out) + row;
 #pragma unroll
