@@ -5,7 +5,7 @@
 // the tensor pipe:
 //   * the group * q_len query rows that share a K/V head (at most 16) are ONE tile, so every K/V element is read once
 //     -- the 128-row kernel reads it once per query head and walks the keys of a head in one serial chain of 64-key blocks;
-//   * a unit (batch, K/V head) is split over a cluster of CTAs (decode_split below) that merge through distributed shared
+//   * a unit (batch, K/V head) is split over a cluster of CTAs (attn_decode_plan.h) that merge through distributed shared
 //     memory: no scratch, no second launch, no atomics;
 //   * inside a CTA the warps take 16-key tiles in turn, each with its own ring of three stages filled by 16-byte cp.async:
 //     no CTA-wide barrier until the merge, 128 KB in flight per SM;
@@ -16,13 +16,13 @@
 // The 16-bit rounding of P, the fp32 accumulation and the base-2 log-sum-exp are those of the tile kernel.
 #pragma once
 
+#include "attn_decode_plan.h"
 #include "attn_fwd.cuh"
 
 namespace b200 {
 
 constexpr int kDecodeRows = 16;     // query rows of a unit that one CTA takes (the M of the MMA)
 constexpr int kDecodeStages = 3;
-constexpr int kDecodeMaxCluster = 16;
 
 struct DecodeParams {
   const uint16_t *q, *k, *v;
@@ -342,39 +342,42 @@ __global__ void __launch_bounds__(WARPS * 32, (DecodeCfg<D, WARPS>::CTAS_PER_SM)
   cluster_wait();
 }
 
-// CTAs per unit and warps per CTA.  One eight-warp CTA (192 KB of ring: one per SM) streams 86 GB/s, so 76 of them saturate
-// the HBM; a unit is therefore split by the largest power of two that keeps the launch within one CTA per SM -- every CTA
-// resident, no second wave, no merge that is not needed -- with at least two 16-key tiles for every warp.  Measured
-// (head_dim 128, us; the choice in brackets):  128 units x 512 keys: [1 CTA, 8 warps: 7.0], 2 x 4 warps 8.0;  64 x 8192:
-// [2 x 8: 41.9], 4 x 4: 42.4, 1 x 8: 51.8;  40 x 12195: [2 x 8: 40.9], 4 x 4: 42.3;  10 x 2729: [8 x 8: 7.1], 16 x 4: 7.7.
-// Clusters above the portable size of 8 need a whole GPC each, and more than four of them queue (8 x 16384: [8 x 8: 18.3],
-// 16 x 8: 24.7;  2 x 16384: 8 x 8: 17.5, [16 x 8: 11.7]).
-// More units than SMs: one four-warp CTA per unit, two per SM.
-struct DecodeSplit {
-  int ctas;
-  bool wide;   // eight warps per CTA (head_dim 128; four at 256), else half of that
-};
-inline DecodeSplit decode_split(int units, int n_tiles) {
-  const int sms = sm_count();
-  if (units > sms) return {1, false};
-  const int most = units <= 4 ? kDecodeMaxCluster : 8;
-  int c = 1;
-  while (2 * c <= most && 2 * c * units <= sms && n_tiles >= 32 * c) c *= 2;
-  return {c, n_tiles > 8 * c};
+// How many clusters of `c` CTAs of a kernel the device holds at once; 0 if it cannot hold any.
+template <class Kernel>
+inline int placeable_clusters(Kernel kern, int c, int threads, size_t smem) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = (unsigned)c;
+  attr.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(1, c);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return n;
 }
 
 template <int D, int WARPS, bool BF16, bool SOFTCAP>
 int launch_attn_decode(DecodeParams p, int units, int c, cudaStream_t stream) {
   using Cfg = DecodeCfg<D, WARPS>;
   auto kern = attn_decode_kernel<D, WARPS, BF16, SOFTCAP>;
-  static thread_local int configured_dev = -1;
+  static thread_local int configured_dev = -1, placeable = 0;   // of the largest clusters
   int dev = 0;
   B200_CUDA_TRY(cudaGetDevice(&dev));
   if (configured_dev != dev) {
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    placeable = placeable_clusters(kern, kDecodeMaxCluster, WARPS * 32, Cfg::SMEM_BYTES);
     configured_dev = dev;
   }
+  c = decode_cluster_that_fits(c, units, placeable);
   p.tiles_per_cta = (p.n_tiles + c - 1) / c;
   B200_CUDA_TRY(launch_kernel(kern, dim3(units, c), WARPS * 32, Cfg::SMEM_BYTES, stream, c, p));
   return B200_OK;
@@ -418,7 +421,7 @@ inline int attn_decode_impl(const void* q, const void* k, const void* v, const F
   p.tiles_per_cta = p.n_tiles;
   const bool cap = f.cap_out > 0.f;
   const int units = f.batch * f.kv_heads;
-  const DecodeSplit split = decode_split(units, p.n_tiles);
+  const DecodeSplit split = decode_split(units, p.n_tiles, sm_count());
   const int c = split.ctas;
 #define B200_DECODE_W(D_, W_)                                                                \
   (bf16 ? (cap ? launch_attn_decode<D_, W_, true, true>(p, units, c, stream)                  \
