@@ -89,9 +89,7 @@ class _Host:
   them.  Where it can be neither built nor loaded there is one warning, and every function returns None: the operators then
   take their Python path, which needs the CUDA library only."""
   FUNCTIONS = ("attn_fwd", "attn_score", "attn_snapkv", "attn_corm", "attn_kf", "kv_evict", "norm", "act_and_mul", "rotary")
-
-  def __init__(self):
-    self._lock = threading.Lock()
+  _lock = threading.Lock()   # of the class: an attribute set in __init__ makes every later look-up of a function 20 ns slower
 
   def __getattr__(self, name):   # only reached while `name` is not set
     if name not in self.FUNCTIONS:
