@@ -619,10 +619,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   // A launch that follows an expired wait on this device drains immediately (the status word stays
   // set until the host reads it), so that one stuck kernel cannot stall a whole queue of launches.
-  // (the word is loaded here and looked at after the set-up, whose barrier it shares)
   __shared__ int s_skip;
-  int status_now = 0;
-  if (threadIdx.x == 0) status_now = *reinterpret_cast<volatile int*>(&g_device_status);
+  if (threadIdx.x == 32) prefetch_l2(&g_device_status);   // read after the wait below
   [[maybe_unused]] const uint64_t cta_start_ns = global_timer_ns();
   [[maybe_unused]] const long long cta_start_clk = clock64();
   B200_TL_INIT();
@@ -669,13 +667,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
   }
+  // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
+  // to allocate columns of its own, and what it wrote is visible only now.
+  pdl_wait();
+  if (threadIdx.x == 32) s_skip = *reinterpret_cast<volatile int*>(&g_device_status);
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
-  if (threadIdx.x == 0) s_skip = status_now;
   tc_fence_before();
-  pdl_wait();
   __syncthreads();
   tc_fence_after();
   c.tmem_base = *tmem_slot;

@@ -94,11 +94,9 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
   // A launch that follows an expired wait on this device drains immediately (the status word stays set until the
-  // host reads it).  The word is loaded here and looked at after the set-up below, whose barrier it shares: a
-  // global load of its own before anything else costs every launch most of a microsecond.
+  // host reads it).
   __shared__ int s_skip;
-  int status_now = 0;
-  if (threadIdx.x == 0) status_now = *reinterpret_cast<volatile int*>(&g_device_status);
+  if (threadIdx.x == 32) prefetch_l2(&g_device_status);   // read after the wait below
 
   [[maybe_unused]] const uint64_t cta_start_ns = global_timer_ns();
   [[maybe_unused]] const long long cta_start_clk = clock64();
@@ -131,13 +129,15 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
   }
+  // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
+  // to allocate columns of its own, and what it wrote is visible only now.
+  pdl_wait();
+  if (threadIdx.x == 32) s_skip = *reinterpret_cast<volatile int*>(&g_device_status);
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
-  if (threadIdx.x == 0) s_skip = status_now;
   tc_fence_before();
-  pdl_wait();
   __syncthreads();
   tc_fence_after();
   c.tmem_base = *tmem_slot;

@@ -662,9 +662,12 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   // A launch that follows an expired wait on this device drains immediately (the status word stays
-  // set until the host reads it), so that one stuck kernel cannot stall a whole queue of launches.  The word is
-  // loaded here and looked at after the set-up below, whose barrier it shares.
+  // set until the host reads it), so that one stuck kernel cannot stall a whole queue of launches.
   __shared__ int s_skip;
+  // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
+  // to allocate columns of its own, and what it wrote is visible only now.  It comes first of all, because a launch has several
+  // waves of CTAs: those of the later ones load the word while they set up.
+  pdl_wait();
   int status_now = 0;
   if (threadIdx.x == 0) status_now = *reinterpret_cast<volatile int*>(&g_device_status);
 
@@ -704,7 +707,6 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
   if (c.blk_hi == c.blk_lo) {
     // nothing visible in this chunk: its partial vector is all zeros
-    pdl_wait();
     if constexpr (MODE != SWEEP_KF_ROWLSE) {
       if (threadIdx.x < 128) {
         const int64_t off = ((int64_t)c.bh * p.n_chunks + chunk) * p.kv_pad + c.a0 + threadIdx.x;
@@ -738,7 +740,6 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
   if (threadIdx.x == 0) s_skip = status_now;
   tc_fence_before();
-  pdl_wait();
   __syncthreads();
   tc_fence_after();
   c.tmem_base = *tmem_slot;

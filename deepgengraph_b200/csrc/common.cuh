@@ -209,6 +209,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_slow(bar, parity, abort_flag, code);
 }
 
+// Brings the line of `p` into L2, without reading it: a load that follows costs a round trip to L2 instead of one to HBM.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // programmatic dependent launch (see launch_kernel below)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -533,15 +536,17 @@ inline int sm_count() {
   return cached;
 }
 
-// Every kernel of the library is launched with programmatic stream serialization: the launch is handed to the SMs while the
-// previous kernel of the stream drains, and the kernel itself waits (pdl_wait) for that kernel's end and its memory
-// before it touches global memory.  Measured (148 blocks, back to back on one stream): a 1 us kernel every 4.1 us without
-// and every 2.0 us with, a 2.6 us kernel every 6.1 and 3.5 us -- without it the front end also starts kernels on a
-// 2 us raster.  No kernel triggers its successor early (griddepcontrol.launch_dependents): the next launch's CTAs would
-// take the slots of an SM one by one as this launch's CTAs end, so that SMs with light CTAs receive two of the heaviest
-// tiles -- causal attention, 32 heads, 1024 tokens: 21.9 us with a trigger after the set-up, 19.1 with one before the
-// epilogue, 18.2 with the implicit one at the kernel's end (20.5 without programmatic launch).
-// Every CTA that leaves early waits first: a kernel's end then implies the end of everything before it in the stream.
+// Every kernel of the library but the noise fill and the self-test of the bounded wait is launched with programmatic stream
+// serialization: the launch is handed to the SMs while the previous kernel of the stream drains, and the kernel itself
+// waits (pdl_wait) for that kernel's end and its memory before it touches global memory or takes tensor memory -- a
+// predecessor that is not the library's own may let its successor start before it has allocated its own tensor memory.
+// Measured (148 blocks, back to back on one stream): a 1 us kernel every 4.1 us without and every 2.0 us with, a 2.6 us
+// kernel every 6.1 and 3.5 us -- without it the front end also starts kernels on a 2 us raster.  No kernel triggers its
+// successor early (griddepcontrol.launch_dependents): the next launch's CTAs would take the slots of an SM one by one as
+// this launch's CTAs end, so that SMs with light CTAs receive two of the heaviest tiles -- causal attention, 32 heads, 1024
+// tokens: 21.9 us with a trigger after the set-up, 19.1 with one before the epilogue, 18.2 with the implicit one at the
+// kernel's end (20.5 without programmatic launch). Every CTA that leaves early waits first: a kernel's end then implies the
+// end of everything before it in the stream.
 template <class... Params, class... Args>
 inline cudaError_t launch_kernel(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                  unsigned cluster_y, Args&&... args) {

@@ -1,0 +1,58 @@
+"""Every launch of the library may start while its predecessor in the stream still runs (csrc/common.cuh, launch_kernel).  What a
+kernel may do before it has waited for that predecessor is checked on the source text, since going wrong could hang a GPU."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "deepgengraph_b200", "csrc")
+PLAIN_LAUNCHES = {"kf_noise_fill_kernel", "bounded_wait_selftest_kernel"}   # <<< >>>: these start after their predecessor's end
+
+
+def _kernels():
+  for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    for m in re.finditer(r"__global__ void\b(?:\s*__launch_bounds__\((?:[^()]|\([^()]*\))*\))?\s*(\w+)\s*\(", text):
+      start = text.index("{", text.index(")", m.end()))
+      depth, end = 0, start
+      while True:
+        depth += {"{": 1, "}": -1}.get(text[end], 0)
+        end += 1
+        if depth == 0:
+          break
+      yield m.group(1), text[start:end]
+
+
+KERNELS = dict(_kernels())
+
+
+def test_the_kernels_are_found():
+  assert {"attn_fwd_kernel", "attn_fwd_persist_kernel", "attn_decode_kernel", "attn_sweep_kernel", "kv_evict_regs_kernel",
+          "rms_norm_block_kernel", "rotary_online_kernel"} | PLAIN_LAUNCHES <= set(KERNELS)
+
+
+@pytest.mark.parametrize("name", sorted(KERNELS))
+def test_nothing_is_taken_before_the_wait(name):
+  body = KERNELS[name]
+  if name in PLAIN_LAUNCHES:
+    return
+  assert "pdl_wait()" in body
+  # Tensor memory: a predecessor that let this launch start early may still have to allocate its own.  The status word: what the
+  # predecessor wrote is visible only after the wait.
+  waits, depth = [], 0    # where the whole block waits: not inside a branch
+  for m in re.finditer(r"[{}]|pdl_wait\(\)", body):
+    if m.group() == "pdl_wait()":
+      waits += [m.start()] if depth == 1 else []
+    else:
+      depth += 1 if m.group() == "{" else -1
+  assert waits
+  for taken in re.finditer(r"tmem_alloc\(|(?<!prefetch_l2\(&)g_device_status", body):
+    assert waits[0] < taken.start(), f"{taken.group()} before pdl_wait()"
+
+
+def test_only_the_plain_launches_are_plain():
+  launched = set()
+  for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+    launched |= set(re.findall(r"(\w+)(?:<[^<>;]*>)?<<<", open(path).read()))
+  assert launched == PLAIN_LAUNCHES
