@@ -15,67 +15,83 @@
 
 namespace b200 {
 
+template <class Fn>
+static Fn driver_entry_point(const char* name) {
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult qres;
+  if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  return reinterpret_cast<Fn>(p);
+}
+
 EncodeTiledFn get_encode_tiled() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess) {
-      (void)cudaGetLastError();
-      return nullptr;
-    }
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
+  static EncodeTiledFn fn = driver_entry_point<EncodeTiledFn>("cuTensorMapEncodeTiled");
   return fn;
 }
 
-// One tensor map.  A call on a short problem is bound by the host, and an attention call needs three to nine maps.  A map is
-// a pure function of the address, sizes and strides below, so each thread keeps the ones it encoded last (a direct-mapped
-// table of 128, 28 KB; a layer loop meets the same buffers over and over).  Measured per call from Python on a tiny
-// problem: attention 7.5 -> 6.9 us, attention with scores 18.8 -> 17.7 us.
-struct TensorMapKey {
-  const void* base;
+typedef CUresult (*ReplaceAddressFn)(CUtensorMap*, void*);
+static ReplaceAddressFn get_replace_address() {
+  static ReplaceAddressFn fn = driver_entry_point<ReplaceAddressFn>("cuTensorMapReplaceAddress");
+  return fn;
+}
+
+// One tensor map.  A call on a short problem is bound by the host, and an attention call needs three to nine maps.  Each thread
+// keeps the layouts that it encoded last -- sizes, strides and box, a direct-mapped table of 64, 16 KB -- and every call puts
+// its own address into a copy: a call on new buffers costs what a repeated one does.  Measured from Python on a
+// tiny problem: attention with scores 12.2 us a call on one set of buffers and 12.3 on 400 in turn.
+struct TensorMapLayout {
   cuuint64_t dims[4], strides[3];
   cuuint32_t box[4];
   uint32_t rank;
   CUtensorMapDataType type;
   CUtensorMapSwizzle swizzle;
-  uint32_t unused = 0;   // no padding: keys are compared as bytes
+  uint32_t unused = 0;   // no padding: layouts are compared as bytes
 };
-static_assert(sizeof(TensorMapKey) == 8 + 7 * 8 + 4 * 4 + 4 * 4, "TensorMapKey must have no padding");
+static_assert(sizeof(TensorMapLayout) == 7 * 8 + 4 * 4 + 4 * 4, "TensorMapLayout must have no padding");
 
-static int encode_tensor_map(CUtensorMap* map, const TensorMapKey& key) {
+static int make_tensor_map(CUtensorMap* map, const void* base, const TensorMapLayout& layout) {
   struct Entry {
     alignas(64) CUtensorMap map;
-    TensorMapKey key;
+    TensorMapLayout layout;
     int device;
     bool valid;
   };
-  constexpr int kEntries = 128;
+  constexpr int kEntries = 64;
+  static_assert(sizeof(Entry) * kEntries == 16 * 1024, "size of the table");
   static thread_local Entry table[kEntries];
-  uint64_t words[sizeof(TensorMapKey) / 8], hash = 0;
-  std::memcpy(words, &key, sizeof(key));
+  uint64_t words[sizeof(TensorMapLayout) / 8], hash = 0;
+  std::memcpy(words, &layout, sizeof(layout));
   for (uint64_t w : words) hash = (hash ^ w) * 0x9E3779B97F4A7C15ull, hash ^= hash >> 29;
   int dev = 0;
   B200_CUDA_TRY(cudaGetDevice(&dev));
   Entry& e = table[hash % kEntries];
-  if (!e.valid || e.device != dev || std::memcmp(&e.key, &key, sizeof(key)) != 0) {
-    EncodeTiledFn enc = get_encode_tiled();
+  const ReplaceAddressFn replace_address = get_replace_address();
+  if (!replace_address) return B200_ERR_CUDA;
+  CUresult r = CUDA_SUCCESS;
+  if (!e.valid || e.device != dev || std::memcmp(&e.layout, &layout, sizeof(layout)) != 0) {
+    const EncodeTiledFn enc = get_encode_tiled();
     if (!enc) return B200_ERR_CUDA;
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     e.valid = false;
-    const CUresult r = enc(&e.map, key.type, key.rank, const_cast<void*>(key.base), key.dims, key.strides, key.box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, key.swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-      g_last_cuda_error = (int)r;
-      return B200_ERR_CUDA;
+    r = enc(&e.map, layout.type, layout.rank, const_cast<void*>(base), layout.dims, layout.strides, layout.box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, layout.swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r == CUDA_SUCCESS) {
+      e.layout = layout;
+      e.device = dev;
+      e.valid = true;
     }
-    e.key = key;
-    e.device = dev;
-    e.valid = true;
   }
-  *map = e.map;
+  if (r == CUDA_SUCCESS) {
+    *map = e.map;
+    r = replace_address(map, const_cast<void*>(base));
+  }
+  if (r != CUDA_SUCCESS) {
+    g_last_cuda_error = (int)r;
+    return B200_ERR_CUDA;
+  }
   return B200_OK;
 }
 
@@ -84,26 +100,24 @@ int make_bshd_tensor_map(CUtensorMap* map, const void* base, int batch, int seq,
                          bool bf16, int64_t token_stride, int64_t batch_stride) {
   if (token_stride == 0) token_stride = (int64_t)heads * dim;
   if (batch_stride == 0) batch_stride = (int64_t)seq * token_stride;
-  const TensorMapKey key{base,
-                         {(cuuint64_t)dim, (cuuint64_t)heads, (cuuint64_t)seq, (cuuint64_t)batch},
-                         {(cuuint64_t)dim * 2, (cuuint64_t)token_stride * 2, (cuuint64_t)batch_stride * 2},
-                         {64, 1, (cuuint32_t)box_rows, 1},
-                         4,
-                         bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                         CU_TENSOR_MAP_SWIZZLE_128B};
-  return encode_tensor_map(map, key);
+  const TensorMapLayout layout{{(cuuint64_t)dim, (cuuint64_t)heads, (cuuint64_t)seq, (cuuint64_t)batch},
+                               {(cuuint64_t)dim * 2, (cuuint64_t)token_stride * 2, (cuuint64_t)batch_stride * 2},
+                               {64, 1, (cuuint32_t)box_rows, 1},
+                               4,
+                               bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                               CU_TENSOR_MAP_SWIZZLE_128B};
+  return make_tensor_map(map, base, layout);
 }
 
 int make_f32_matrix_tensor_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int box_rows,
                                int box_cols, bool swizzle128) {
-  const TensorMapKey key{base,
-                         {(cuuint64_t)cols, (cuuint64_t)rows, 0, 0},
-                         {(cuuint64_t)cols * 4, 0, 0},
-                         {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 0, 0},
-                         2,
-                         CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                         swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE};
-  return encode_tensor_map(map, key);
+  const TensorMapLayout layout{{(cuuint64_t)cols, (cuuint64_t)rows, 0, 0},
+                               {(cuuint64_t)cols * 4, 0, 0},
+                               {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 0, 0},
+                               2,
+                               CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                               swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE};
+  return make_tensor_map(map, base, layout);
 }
 
 // Self-test of the bounded-wait machinery: one warp waits on an mbarrier that nobody ever arrives on.  The wait
