@@ -11,8 +11,8 @@
 //     no CTA-wide barrier until the merge, 128 KB in flight per SM;
 //   * the products are mma.sync m16n8k16: a tcgen05 tile would be 128 rows high for 1 to 16 rows of use, and the
 //     contraction needs 5 % of what even mma.sync delivers.
-// Measured (bf16, head_dim 128, GPU time): batch 8, 32 query / 8 K/V heads, 8192 keys 115.6 -> 42 us (6.4 TB/s, 99 % of the
-// copy rate); batch 4, 32 heads, 512 keys 11.0 -> 7.0 us.
+// Measured (bf16, head_dim 128, GPU time): batch 8, 32 query / 8 K/V heads, 8192 keys 115.6 -> 42 us (6.4 TB/s; 96 % of the
+// copy rate with the launch gap); batch 4, 32 heads, 512 keys 11.0 -> 7.0 us.
 // The 16-bit rounding of P, the fp32 accumulation and the base-2 log-sum-exp are those of the tile kernel.
 #pragma once
 
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(WARPS * 32, (DecodeCfg<D, WARPS>::CTAS_PER_SM)
     stage = stage == kDecodeStages - 1 ? 0 : stage + 1;
   }
 
-  // ---- merge of the four warps (partial outputs in the ring's memory), then of the cluster's CTAs ----
+  // ---- merge of the CTA's warps (partial outputs in the ring's memory), then of the cluster's CTAs ----
   cp_async_wait<0>();
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -384,10 +384,8 @@ int launch_attn_decode(DecodeParams p, int units, int c, cudaStream_t stream) {
 }
 
 // Taken when the query rows of a unit fit one MMA tile: beyond that the 128-row tile kernel has enough rows to share a K/V
-// block among.
-inline bool use_decode(int q_len, int group, int units) {
-  return (int64_t)q_len * group <= kDecodeRows && units <= 65535;
-}
+// block among.  A function of the unit alone: a shard of the heads or batch elements goes to the same kernel as the whole problem.
+inline bool use_decode(int q_len, int group) { return (int64_t)q_len * group <= kDecodeRows; }
 
 inline int attn_decode_impl(const void* q, const void* k, const void* v, const FwdParams& f, int head_dim, bool bf16,
                             const AttnStrides& st, cudaStream_t stream) {

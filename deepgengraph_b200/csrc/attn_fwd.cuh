@@ -745,7 +745,7 @@ struct AttnStrides {
 };
 
 // few query rows against many keys (attn_decode.cuh)
-bool use_decode(int q_len, int group, int units);
+bool use_decode(int q_len, int group);
 int attn_decode_impl(const void* q, const void* k, const void* v, const FwdParams& f, int head_dim, bool bf16,
                      const AttnStrides& st, cudaStream_t stream);
 
@@ -783,7 +783,7 @@ inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v,
   p.scale_log2 = scale * kLog2e;
   p.cap_in = softcap > 0.f ? scale / softcap : 0.f;
   p.cap_out = softcap * kLog2e;
-  if (use_decode(q_len, heads / kv_heads, batch * kv_heads)) return attn_decode_impl(q, k, v, p, head_dim, bf16, st, stream);
+  if (use_decode(q_len, heads / kv_heads)) return attn_decode_impl(q, k, v, p, head_dim, bf16, st, stream);
 
   const int bn = head_dim == 128 ? B200_BN128 : 64;
   CUtensorMap tq, tk, tv;
