@@ -1,8 +1,8 @@
 // Bandwidth kernels: RMSNorm, fused-add RMSNorm, SiLU/GELU-gate, online rotary embedding.
-// All of them are HBM-bound; they move 16 bytes per thread per access, keep a row in
+// All of them are HBM-bound; they move 16 bytes per thread per access and keep a row in
 // registers between the reduction and the scaling (one read of the input instead of
-// the two passes of the reference kernels), and run as persistent grids sized to the
-// SM count.
+// the two passes of the reference kernels).  Their grids are a few blocks per SM that
+// walk the work, but for RMSNorm's block per row.
 #pragma once
 
 #include <type_traits>

@@ -547,9 +547,9 @@ int launch_kv_evict_topk(dim3 grid, size_t smem, cudaStream_t stream, const floa
 }
 
 // CTAs per (batch, head): as many as are resident at once, so that the launch has no second wave (each repeats the selection,
-// which reads a few KB of scores from L2), and at most 16.  Measured, two CTAs per SM assumed for every
-// instantiation -> asked for and counted (32 heads, graph replay, us): RoCo 5000 keys 46.5 -> 32.3, 8192 37.2 -> 28.2, 12000 83.5 ->
-// 43.7, 16384 65.5 -> 36.3; largest scores 12000 keys 29.5 -> 23.8, 16384 31.5 -> 26.0.
+// which reads a few KB of scores from L2), and at most 16.  Measured, two CTAs per SM assumed for every instantiation -> asked
+// for and counted (32 heads, graph replay, us): RoCo 5000 keys 46.5 -> 32.3, 8192 37.2 -> 28.2, 12000 83.5 -> 43.7, 16384 65.5
+// -> 36.3; largest scores 12000 keys 29.5 -> 23.8, 16384 31.5 -> 26.0.
 template <int NK, bool ROCO>
 int launch_evict_regs_nk(const float* score, const float* score_sq, const void* k, const void* v, void* kv_cache,
                          int32_t* indices, int batch, int seq, int heads, int row_bytes, int q_len, int budget, int recent,

@@ -2,7 +2,8 @@
 
 Every (batch, kv-head) pair -- with the `group` query heads that share it -- is an independent unit of
 work: attention rows never mix heads, and the per-key score vectors of a head only sum over that head's
-own queries.  So the path shards with NO data-path collective: rank r owns the contiguous unit range
+own queries.  A shard's results are the whole problem's, bit for bit -- except for calls with up to 16 query rows per K/V head
+(generation steps; csrc/attn_decode_plan.h), whose last bits follow the number of units in the launch.  So the path shards with NO data-path collective: rank r owns the contiguous unit range
 [r*U/N, (r+1)*U/N) of the flattened (batch, kv_head) index space and runs the single-GPU kernels on it.
 The only communication is optional and off the critical path: gathering the small fp32 score vectors
 ([units, kv_len], ~1 MiB in total) so that every rank sees the scores of all heads (a KV-eviction policy
