@@ -739,6 +739,12 @@ template <int D_, bool BF16, bool SOFTCAP>
 int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                             cudaStream_t stream);
 
+// head_dim 256 (attn_fwd_split.cuh)
+struct AttnStrides;
+template <bool BF16, bool SOFTCAP>
+int launch_attn_fwd_split(const void* q, const void* k, const void* v, const FwdParams& p, const AttnStrides& st,
+                          bool one_tile_per_cta, cudaStream_t stream);
+
 // element strides of q / k / v when they are views into a larger buffer (0 = contiguous)
 struct AttnStrides {
   int64_t q_token, q_batch, k_token, k_batch, v_token, v_batch;
@@ -785,7 +791,17 @@ inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v,
   p.cap_out = softcap * kLog2e;
   if (use_decode(q_len, heads / kv_heads)) return attn_decode_impl(q, k, v, p, head_dim, bf16, st, stream);
 
-  const int bn = head_dim == 128 ? B200_BN128 : 64;
+  const bool cap = softcap > 0.f;
+  // The grids are persistent; a launch of one CTA per tile stays selectable for A/B timing (read once per process).
+  static const bool one_tile_per_cta = std::getenv("B200_ATTN_ONE_TILE_PER_CTA") != nullptr;
+  if (head_dim == 256) {
+    return bf16 ? (cap ? launch_attn_fwd_split<true, true>(q, k, v, p, st, one_tile_per_cta, stream)
+                       : launch_attn_fwd_split<true, false>(q, k, v, p, st, one_tile_per_cta, stream))
+                : (cap ? launch_attn_fwd_split<false, true>(q, k, v, p, st, one_tile_per_cta, stream)
+                       : launch_attn_fwd_split<false, false>(q, k, v, p, st, one_tile_per_cta, stream));
+  }
+
+  const int bn = B200_BN128;
   CUtensorMap tq, tk, tv;
   int rc;
   if ((rc = make_bshd_tensor_map(&tq, q, batch, q_len, heads, head_dim, 128, bf16, st.q_token, st.q_batch)) != B200_OK)
@@ -795,33 +811,25 @@ inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v,
   if ((rc = make_bshd_tensor_map(&tv, v, batch, kv_len, kv_heads, head_dim, bn, bf16, st.v_token, st.v_batch)) != B200_OK)
     return rc;
 
-  const bool cap = softcap > 0.f;
-
 #define B200_FWD_DISPATCH(D_, BN_, NQ_, SB_)                                                                 \
   (bf16 ? (cap ? launch_attn_fwd_cfg<D_, BN_, NQ_, SB_, true, true>(tq, tk, tv, p, stream)                   \
                : launch_attn_fwd_cfg<D_, BN_, NQ_, SB_, true, false>(tq, tk, tv, p, stream))                 \
         : (cap ? launch_attn_fwd_cfg<D_, BN_, NQ_, SB_, false, true>(tq, tk, tv, p, stream)                  \
                : launch_attn_fwd_cfg<D_, BN_, NQ_, SB_, false, false>(tq, tk, tv, p, stream)))
-  // Default: the persistent kernel, whose CTAs walk query tiles handed out by an atomic counter (two CTAs per SM
-  // at head_dim 128, one at 256).  The one-tile-per-CTA launch stays selectable for A/B timing (environment
-  // variable read once per process).  (That kernel also supports NQ = 2 -- two tiles sharing one K/V stream in a
-  // single CTA; at head_dim 128 two independent CTAs per SM measured 13 % faster at seq 4096.)
-  static const bool one_tile_per_cta = std::getenv("B200_ATTN_ONE_TILE_PER_CTA") != nullptr;
+  // Default: the persistent kernel, whose CTAs walk query tiles handed out by an atomic counter, two CTAs per SM.  (The other
+  // kernel also supports NQ = 2 -- two tiles sharing one K/V stream in a single CTA; two independent CTAs per SM measured 13 %
+  // faster at seq 4096.)
 #define B200_PERSIST_DISPATCH(D_)                                                                    \
   (bf16 ? (cap ? launch_attn_fwd_persist<D_, true, true>(tq, tk, tv, p, stream)                       \
                : launch_attn_fwd_persist<D_, true, false>(tq, tk, tv, p, stream))                     \
         : (cap ? launch_attn_fwd_persist<D_, false, true>(tq, tk, tv, p, stream)                      \
                : launch_attn_fwd_persist<D_, false, false>(tq, tk, tv, p, stream)))
-  if (head_dim == 128) {
-    if (!one_tile_per_cta && B200_BN128 == 64 && B200_SB128 == 2) return B200_PERSIST_DISPATCH(128);
+  if (!one_tile_per_cta && B200_BN128 == 64 && B200_SB128 == 2) return B200_PERSIST_DISPATCH(128);
 #ifdef B200_NQ128
-    return B200_FWD_DISPATCH(128, B200_BN128, B200_NQ128, B200_SB128);
+  return B200_FWD_DISPATCH(128, B200_BN128, B200_NQ128, B200_SB128);
 #else
-    return B200_FWD_DISPATCH(128, B200_BN128, 1, B200_SB128);
+  return B200_FWD_DISPATCH(128, B200_BN128, 1, B200_SB128);
 #endif
-  }
-  if (!one_tile_per_cta) return B200_PERSIST_DISPATCH(256);
-  return B200_FWD_DISPATCH(256, 64, 1, 2);
 #undef B200_PERSIST_DISPATCH
 #undef B200_FWD_DISPATCH
 }

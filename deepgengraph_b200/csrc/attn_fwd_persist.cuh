@@ -517,6 +517,40 @@ inline int sched_counter_for_launch(unsigned int** out) {
   return B200_OK;
 }
 
+// Counter (only a persistent grid has one), number and order of the tiles of a launch.
+inline int sched_params(SchedParams* sp, const FwdParams& p, int head_dim, bool persistent) {
+  sp->counter = nullptr;
+  if (persistent) {
+    const int rc = sched_counter_for_launch(&sp->counter);
+    if (rc != B200_OK) return rc;
+  }
+  sp->n_q_tiles = (p.q_len + 127) / 128;
+  sp->total_items = p.batch * p.heads * sp->n_q_tiles;
+  // Group size.  Where all of K and V stay in L2 (126 MB) beside q and out, one group: the whole launch then runs heaviest
+  // tile first and ends on the lightest.  Else as many units as have a quarter of L2 of K/V, at least 1 and at most 32.  K/V
+  // of a head count once for the query heads that share it.  Measured, groups -> one group (bf16, causal, us): 2 x 12 heads,
+  // 3000 tokens, head_dim 256 (74 MB) 114.5 -> 101.8; 4 x 32/8 heads, 1024 tokens (17 MB) 47.5 -> 45.9; 2 x 32/8, 777
+  // queries, 3001 keys (25 MB) 85.9 -> 84.1; 8 x 32, 512 tokens (67 MB) 37.3 -> 36.4; but 32 heads, 8192 tokens (134 MB)
+  // 454.9 -> 469.7 and 4 x 32, 4096 tokens (268 MB) 494.5 -> 559.6.
+  {
+    const int64_t kv_bytes_per_head = (int64_t)2 * p.kv_len * head_dim * 2;
+    const int units = p.batch * p.heads, group = p.heads / p.kv_heads;
+    const bool in_l2 = kv_bytes_per_head * p.batch * p.kv_heads <= ((int64_t)80 << 20);
+    int gh = units;
+    if (!in_l2) {
+      // groups of one size (a small last one drains badly: 4 x 16/8 heads, 6000 tokens, 64 units: groups of 21 -- 546 us, of
+      // 16 -- 509), not cut between query heads that share K/V
+      const int64_t fit = std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)32 << 20) * group / kv_bytes_per_head));
+      const int n_groups = (int)((units + fit - 1) / fit);
+      gh = ((units + n_groups - 1) / n_groups + group - 1) / group * group;
+    }
+    static const char* env = std::getenv("B200_ATTN_GROUP_HEADS");
+    if (env != nullptr && std::atoi(env) > 0) gh = std::atoi(env);
+    sp->group_heads = gh;
+  }
+  return B200_OK;
+}
+
 template <int D_, bool BF16, bool SOFTCAP>
 int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                             cudaStream_t stream) {
@@ -530,32 +564,8 @@ int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const 
     configured_dev = dev;
   }
   SchedParams sp;
-  int rc = sched_counter_for_launch(&sp.counter);
+  const int rc = sched_params(&sp, p, D_, true);
   if (rc != B200_OK) return rc;
-  sp.n_q_tiles = (p.q_len + 127) / 128;
-  sp.total_items = p.batch * p.heads * sp.n_q_tiles;
-  // Group size.  Where all of K and V stay in L2 (126 MB) beside q and out, one group: the whole launch then runs heaviest
-  // tile first and ends on the lightest.  Else as many units as have a quarter of L2 of K/V, at least 1 and at most 32.  K/V
-  // of a head count once for the query heads that share it.  Measured, groups -> one group (bf16, causal, us): 2 x 12 heads,
-  // 3000 tokens, head_dim 256 (74 MB) 114.5 -> 101.8; 4 x 32/8 heads, 1024 tokens (17 MB) 47.5 -> 45.9; 2 x 32/8, 777
-  // queries, 3001 keys (25 MB) 85.9 -> 84.1; 8 x 32, 512 tokens (67 MB) 37.3 -> 36.4; but 32 heads, 8192 tokens (134 MB)
-  // 454.9 -> 469.7 and 4 x 32, 4096 tokens (268 MB) 494.5 -> 559.6.
-  {
-    const int64_t kv_bytes_per_head = (int64_t)2 * p.kv_len * D_ * 2;
-    const int units = p.batch * p.heads, group = p.heads / p.kv_heads;
-    const bool in_l2 = kv_bytes_per_head * p.batch * p.kv_heads <= ((int64_t)80 << 20);
-    int gh = units;
-    if (!in_l2) {
-      // groups of one size (a small last one drains badly: 4 x 16/8 heads, 6000 tokens, 64 units: groups of 21 -- 546 us, of
-      // 16 -- 509), not cut between query heads that share K/V
-      const int64_t fit = std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)32 << 20) * group / kv_bytes_per_head));
-      const int n_groups = (int)((units + fit - 1) / fit);
-      gh = ((units + n_groups - 1) / n_groups + group - 1) / group * group;
-    }
-    static const char* env = std::getenv("B200_ATTN_GROUP_HEADS");
-    if (env != nullptr && std::atoi(env) > 0) gh = std::atoi(env);
-    sp.group_heads = gh;
-  }
   const int grid = std::min(sp.total_items, Cfg::CTAS_PER_SM * sm_count());
   B200_CUDA_TRY(launch_kernel(kern, grid, Cfg::THREADS_P, Cfg::SMEM_BYTES_P, stream, 1, tq, tk, tv, p, sp));
   return B200_OK;

@@ -1,0 +1,640 @@
+// Attention forward at head_dim 256: one persistent CTA per SM, one query tile of 128 rows at a time, blocks of 128 keys.
+//   warps 0-3, 4-7   softmax: warpgroup h takes keys [64 h, 64 h + 64) of every block; thread = row = TMEM lane
+//   warp  8          TMA producer of Q, K and V, tile scheduler
+//   warp  9          MMA issuer: S = Q K^T (operands in shared memory), O += P V (P read from TMEM)
+// TMEM (512 columns): two S buffers of 128 (the 16-bit P of a thread's 64 keys overwrites the first half of its own 64 columns), O 256.
+//
+// What bounds it and why this shape.  Per block of 128 keys the tensor pipe needs 16 x 64 clk for S and 8 x 128 for P V, 2048 in all,
+// the special-function unit 1024, and with the soft-cap the softmax is issue-bound on top.  With 64-key blocks and one softmax
+// warpgroup a block cost every hand-over (S -> softmax -> P -> P V) twice as often, and one warp per SM sub-partition could not keep
+// up with the soft-cap: 1771 clk per 64 keys, where this one takes 3058 per 128 (2832 without the soft-cap: the issuer's barrier
+// polls, 630 clk a block, leave the pipe idle).  S with N = 128 runs at the full rate with Q in shared memory (N = 64: 48 instead
+// of 32 clk), so Q needs no TMEM and both S buffers hold 128 keys.
+// Measured, before -> now (one box, bf16): 16/8 heads, 8192 tokens, window 4096, soft-cap 50: 375 -> 353 us (422 -> 394 in a loop under
+// the power cap); 500 queries on 4000 keys, soft-cap: 65.5 -> 60.5; causal without soft-cap, 8192 tokens: 410 -> 410.
+#pragma once
+
+#include "attn_fwd_persist.cuh"
+
+namespace b200 {
+
+struct SplitCfg {
+  static constexpr int D = 256, BM = 128, BN = 128, SB = 2;
+  static constexpr int COLS = BN / 2;                // keys of a softmax thread
+  static constexpr int KSUB = D / 64;                // 64-element (128-byte) column blocks of a row
+  static constexpr int Q_TILE_BYTES = BM * D * 2;
+  // One ring of 32 KB stages.  A K block is two stages of 128 keys x 128 dims, a V block two of 64 keys x 256 dims: each stage is a
+  // complete operand of a run of eight (four) MMAs.
+  static constexpr int STAGE_BYTES = 32768, PARTS = 2, V_KEYS = BN / PARTS, SLOTS = 5;
+  static constexpr int O_COL = SB * BN, TMEM_COLS = 512;
+  static_assert(O_COL + D == TMEM_COLS, "TMEM plan");
+  static constexpr int SOFTMAX_WARPS = 8, PRODUCER_WARP = 8, THREADS = 320;
+  // barriers
+  static constexpr int BAR_Q_FULL = 0;
+  static constexpr int BAR_Q_FREE = 1;                       // last S of a tile retired
+  static constexpr int BAR_S_FULL = 2;                       // [SB]
+  static constexpr int BAR_P_FULL = BAR_S_FULL + SB;         // [SB] eight softmax warps
+  static constexpr int BAR_O_FULL = BAR_P_FULL + SB;         // [2] P V of block g completes barrier g % 2
+  static constexpr int BAR_FULL = BAR_O_FULL + 2;            // [SLOTS]
+  static constexpr int BAR_EMPTY = BAR_FULL + SLOTS;         // [SLOTS]
+  static constexpr int BAR_SCHED = BAR_EMPTY + SLOTS;        // [2] item of slot k % 2 published
+  static constexpr int BAR_SCHED_FREE = BAR_SCHED + 2;       // [2] read by the softmax warps and the issuer
+  static constexpr int BAR_DRAIN = BAR_SCHED_FREE + 2;
+  static constexpr int NUM_BARS = BAR_DRAIN + 1;
+  // behind the tiles: barriers, [half][row] floats (maxima and sums handed between a row's two threads), a failure flag per pair of
+  // softmax warps, TMEM address, abort flag, two scheduler slots, skip flag
+  static constexpr int OFF_BARS = Q_TILE_BYTES + SLOTS * STAGE_BYTES;
+  static constexpr int OFF_XCH = OFF_BARS + (NUM_BARS * 8 + 15) / 16 * 16;
+  static constexpr int OFF_FAIL = OFF_XCH + 2 * BM * 4;
+  static constexpr int OFF_MISC = OFF_FAIL + 16;
+  static constexpr int SMEM_BYTES = OFF_MISC + 32 + 1024;    // +1024: manual alignment
+  static_assert(SMEM_BYTES <= 232448, "shared memory budget exceeded");
+};
+
+struct SplitCtx {
+  uint8_t* smem;
+  uint64_t* bars;
+  float* xch;
+  volatile int* fail;
+  volatile int* abort_flag;
+  volatile int* sched;   // [2] item index or -1
+  volatile int* skip;    // status word of the device at the start
+  uint32_t tmem_base;
+
+  __device__ __forceinline__ bool wait(int bar, int parity, int code) const {
+    return mbar_wait(&bars[bar], parity & 1, abort_flag, code);
+  }
+  __device__ __forceinline__ bool wait_warp(int bar, int parity, int code) const {   // one outcome for the whole warp
+    return __all_sync(0xffffffffu, wait(bar, parity, code));
+  }
+};
+
+// The two warps that share a query tile's rows meet in a named barrier (64 threads) that also ORs a predicate.
+__device__ __forceinline__ bool pair_vote(int id, bool pred) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %2, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, 64, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(id), "r"((uint32_t)pred)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
+
+// ------------------------------ softmax warps ------------------------------
+// Both threads of a row need the same reference maximum m (their P feed one accumulator), but m moves only in a tile's first block
+// and where a block's maximum exceeds it by more than 2^8 (lazy rescale).  So the common block costs one vote between the two warps
+// of a 32-row group; only after a vote for it are the maxima exchanged through shared memory.
+//
+// Steps and failure.  Every pair_vote is a step; a step whose vote comes out true is followed by one pair_sync, after which the
+// pair's failure flag is looked at.  A warp whose bounded wait ran out sets the flag, takes part in one more step with a true
+// vote and leaves; its partner leaves in that same step.  A warp that is done takes part in one last step.  No named barrier is ever
+// waited for alone.
+template <bool BF16, bool SOFTCAP>
+struct SplitSoftmax {
+  using Cfg = SplitCfg;
+  static constexpr int D = Cfg::D, COLS = Cfg::COLS, SB = Cfg::SB;
+  const SplitCtx& c;
+  const FwdParams& p;
+  const int half, warp_q, lane, bar_id;
+  const uint32_t lane_addr, o_addr;   // o_addr: this thread's half of the row's O
+  float m, l;                         // l: sum of this thread's keys
+
+  __device__ __forceinline__ SplitSoftmax(const SplitCtx& c_, const FwdParams& p_, int warp, int lane_)
+      : c(c_), p(p_), half(warp >> 2), warp_q(warp & 3), lane(lane_), bar_id(1 + (warp & 3)),
+        lane_addr(c_.tmem_base + ((uint32_t)((warp & 3) * 32) << 16)),
+        o_addr(c_.tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::O_COL + (warp >> 2) * (D / 2)) {}
+
+  __device__ __forceinline__ volatile float* xch(int h) const { return c.xch + h * Cfg::BM + warp_q * 32 + lane; }
+  __device__ __forceinline__ void leave_failed() const {
+    c.fail[warp_q] = 1;
+    pair_vote(bar_id, true);
+    pair_sync(bar_id);
+  }
+
+  // One block of one row.  `g` counts the CTA's blocks, n those of the tile.  False: leave (no further step).
+  template <bool MASK>
+  __device__ __forceinline__ bool block(int n, int g, int lo_c, int hi_c, float cmul) {
+    const int buf = g % SB;
+    const uint32_t s_addr = lane_addr + buf * Cfg::BN + half * COLS;
+    const bool ok = c.wait(Cfg::BAR_S_FULL + buf, g / SB, WAIT_S_FULL);
+    tc_fence_after();
+    uint32_t sr[COLS / 32][32];
+#pragma unroll
+    for (int ch = 0; ch < COLS / 32; ++ch) tmem_ld32(s_addr + ch * 32, sr[ch]);
+    tmem_ld_wait();
+
+    // Maximum of the thread's 64 logits.  With a soft-cap the capped logit is a monotone function of the raw one, so the maximum
+    // is taken over the RAW values (no special-function work in this pass) and capped once; the pass also finds the largest
+    // |raw| so that the warp can vote for the polynomial-only exponential pass below.
+    float mx0 = -INFINITY, mx1 = -INFINITY;
+    [[maybe_unused]] float ab0 = 0.f, ab1 = 0.f;
+#pragma unroll
+    for (int ch = 0; ch < COLS / 32; ++ch) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) {
+        float v[4];
+        [[maybe_unused]] float va[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float s = __uint_as_float(sr[ch][i + u]);
+          [[maybe_unused]] float sa = fabsf(s);
+          if constexpr (MASK) {
+            const int col = ch * 32 + i + u;
+            if (col > hi_c || col < lo_c) {
+              s = -INFINITY;
+              sa = 0.f;
+            }
+            // (with a soft-cap the registers keep the raw value: the exponential pass masks by column again)
+            if constexpr (!SOFTCAP) sr[ch][i + u] = __float_as_uint(s);
+          }
+          v[u] = s;
+          if constexpr (SOFTCAP) va[u] = sa;
+        }
+        mx0 = fmax3(mx0, v[0], v[1]);
+        mx1 = fmax3(mx1, v[2], v[3]);
+        if constexpr (SOFTCAP) {
+          ab0 = fmax3(ab0, va[0], va[1]);
+          ab1 = fmax3(ab1, va[2], va[3]);
+        }
+      }
+    }
+    float m_blk = fmaxf(mx0, mx1);   // -inf when all 64 are masked
+    [[maybe_unused]] bool cap_poly_only = false;
+    if constexpr (SOFTCAP) {
+      m_blk = m_blk == -INFINITY ? -INFINITY : softcap_tanh(m_blk * p.cap_in) * cmul;   // cap_out is folded into cmul
+      cap_poly_only = !__any_sync(0xffffffffu, fmaxf(ab0, ab1) * p.cap_in > kCapPolyMax);
+    } else {
+      m_blk *= cmul;
+    }
+    if (pair_vote(bar_id, !ok || n == 0 || m_blk - m > 8.0f)) {   // exp2(x - m) stays <= 256
+      if (!ok) c.fail[warp_q] = 1;
+      *xch(half) = m_blk;
+      pair_sync(bar_id);
+      if (c.fail[warp_q] != 0) return false;
+      m_blk = fmaxf(m_blk, *xch(half ^ 1));
+      if (n == 0) {
+        m = fmaxf(m, m_blk);
+      } else {
+        float alpha = 1.0f;
+        bool rescale = false;
+        if (m_blk - m > 8.0f) {
+          alpha = ex2_approx(m - m_blk);
+          m = m_blk;
+          l *= alpha;
+          rescale = true;
+        }
+        if (__any_sync(0xffffffffu, rescale)) {   // the same in both warps: they hold the same rows
+          // P V(g-1): its barrier is exactly in or just past the awaited phase -- S(g) complete implies P V(g-2), and P V(g+1) waits
+          // for this thread's P(g).
+          if (!c.wait_warp(Cfg::BAR_O_FULL + ((g - 1) & 1), (g - 1) >> 1, WAIT_O_FULL)) {
+            leave_failed();
+            return false;
+          }
+          tc_fence_after();
+          const float2 a2 = make_float2(alpha, alpha);
+#pragma unroll
+          for (int ch = 0; ch < D / 2 / 16; ++ch) {
+            uint32_t o[16];
+            tmem_ld16(o_addr + ch * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              const float2 r = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), a2);
+              o[i] = __float_as_uint(r.x);
+              o[i + 1] = __float_as_uint(r.y);
+            }
+            tmem_st16(o_addr + ch * 16, o);
+          }
+        }
+      }
+    }
+    // P = exp2(x - m), packed to the 16-bit input type, written over the first half of the thread's own S columns
+    const float2 c2 = make_float2(cmul, cmul), nm2 = make_float2(-m, -m);
+    float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+    // x = logit - m in base-2 units for four columns; POLY_ONLY: every |raw / cap| of the warp's columns is <= 1
+    auto exponents = [&](auto poly_only_tag, int ch, int i, float2& x0, float2& x1) {
+      const float2 s0 = make_float2(__uint_as_float(sr[ch][i + 0]), __uint_as_float(sr[ch][i + 1]));
+      const float2 s1 = make_float2(__uint_as_float(sr[ch][i + 2]), __uint_as_float(sr[ch][i + 3]));
+      if constexpr (SOFTCAP) {
+        const float2 a2 = make_float2(p.cap_in, p.cap_in);
+        const float2 y0 = fmul2(s0, a2), y1 = fmul2(s1, a2);
+        if constexpr (decltype(poly_only_tag)::value) {
+          x0 = ffma2(y0, softcap_r2(y0, cmul), nm2);
+          x1 = ffma2(y1, softcap_r2(y1, cmul), nm2);
+        } else {
+          x0 = ffma2(make_float2(softcap_tanh(y0.x), softcap_tanh(y0.y)), c2, nm2);
+          x1 = ffma2(make_float2(softcap_tanh(y1.x), softcap_tanh(y1.y)), c2, nm2);
+        }
+        if constexpr (MASK) {
+          const int col = ch * 32 + i;
+          if (col + 0 > hi_c || col + 0 < lo_c) x0.x = -INFINITY;
+          if (col + 1 > hi_c || col + 1 < lo_c) x0.y = -INFINITY;
+          if (col + 2 > hi_c || col + 2 < lo_c) x1.x = -INFINITY;
+          if (col + 3 > hi_c || col + 3 < lo_c) x1.y = -INFINITY;
+        }
+      } else {
+        x0 = ffma2(s0, c2, nm2);
+        x1 = ffma2(s1, c2, nm2);
+      }
+    };
+    auto exp_pass = [&](auto poly_only_tag) {
+#pragma unroll
+      for (int ch = 0; ch < COLS / 32; ++ch) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          float2 x0, x1;
+          exponents(poly_only_tag, ch, i, x0, x1);
+          x0.x = ex2_approx(x0.x);
+          x0.y = ex2_approx(x0.y);
+          x1.x = ex2_approx(x1.x);
+          x1.y = ex2_approx(x1.y);
+          acc0 = fadd2(acc0, x0);
+          acc1 = fadd2(acc1, x1);
+          pk[i / 2] = pack2<BF16>(x0.x, x0.y);
+          pk[i / 2 + 1] = pack2<BF16>(x1.x, x1.y);
+        }
+        tmem_st16(s_addr + ch * 16, pk);
+      }
+    };
+    if constexpr (SOFTCAP) {
+      if (cap_poly_only)
+        exp_pass(std::true_type{});
+      else
+        exp_pass(std::false_type{});
+    } else {
+      exp_pass(std::false_type{});
+    }
+    l += (acc0.x + acc0.y) + (acc1.x + acc1.y);
+    tmem_st_wait();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_P_FULL + buf]);
+    return true;
+  }
+
+  __device__ __forceinline__ void run(const SchedParams& sp) {
+    const float cmul = SOFTCAP ? p.cap_out : p.scale_log2;
+    int g = 0;
+    for (int k = 0;; ++k) {
+      if (!c.wait_warp(Cfg::BAR_SCHED + (k & 1), k >> 1, WAIT_SCHED)) {
+        leave_failed();
+        return;
+      }
+      const int item = c.sched[k & 1];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_SCHED_FREE + (k & 1)]);   // slot may be rewritten for item k + 2
+      if (item < 0) break;
+      const TileInfo t = decode_item(item, p, sp, Cfg::BN);
+      const int row = t.q0 + warp_q * 32 + lane;
+      m = -1.0e30f;   // finite, so that fully masked blocks stay NaN-free
+      l = 0.f;
+      // visible keys of this row: [lo_key, hi_key]; a block needs element masks only if some row of the tile sees it partially
+      const int hi_key = (p.causal ? min(row + p.delta, p.kv_len - 1) : p.kv_len - 1) - half * COLS;
+      const int lo_key = ((p.causal && p.window > 0) ? (row + p.delta - p.window + 1) : -(1 << 28)) - half * COLS;
+      const int hi_first = p.causal ? min(t.q0 + p.delta, p.kv_len - 1) : p.kv_len - 1;
+      const int lo_last = (p.causal && p.window > 0) ? (t.q0 + 127 + p.delta - p.window + 1) : -(1 << 28);
+      for (int j = t.lo; j < t.hi; ++j, ++g) {
+        const int n = j - t.lo, k0 = j * Cfg::BN;
+        const bool need_mask = (hi_first - k0 < Cfg::BN - 1) || (lo_last - k0 > 0);
+        const bool go = need_mask ? block<true>(n, g, lo_key - k0, hi_key - k0, cmul) : block<false>(n, g, 0, 0, cmul);
+        if (!go) return;
+      }
+      // Epilogue; the issuer is already computing the next tile's S meanwhile.  The next tile's first P V (which overwrites O) is
+      // issued only after this warp has delivered that tile's first P, i.e. after the loads below have completed.
+      *xch(half) = l;
+      const bool ok = c.wait(Cfg::BAR_O_FULL + ((g - 1) & 1), (g - 1) >> 1, WAIT_O_FULL);
+      if (!ok) c.fail[warp_q] = 1;
+      if (pair_vote(bar_id, !ok)) {
+        pair_sync(bar_id);
+        return;
+      }
+      const float l_other = *xch(half ^ 1);
+      const float l_row = l + l_other;
+      tc_fence_after();
+      const float inv_l = 1.0f / l_row;
+      const bool in_range = row < p.q_len;
+      const bool wide_stores = (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
+      uint4* out_row = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
+                                                (((int64_t)t.b * p.q_len + row) * p.heads + t.h) * (int64_t)D + half * (D / 2));
+#pragma unroll
+      for (int ch = 0; ch < D / 2 / 32; ++ch) {
+        uint32_t o[32];
+        tmem_ld32(o_addr + ch * 32, o);
+        tmem_ld_wait();
+        if (in_range) {
+          // every lane writes its own row (rows are heads * D elements apart), so a store instruction costs one
+          // memory transaction per lane whatever its width: 32-byte stores halve the count
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            uint32_t x[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              x[e] = pack2<BF16>(__uint_as_float(o[v * 16 + 2 * e]) * inv_l, __uint_as_float(o[v * 16 + 2 * e + 1]) * inv_l);
+            if (wide_stores) {
+              st_global_v8(out_row + ch * 4 + v * 2, x);
+            } else {
+              out_row[ch * 4 + v * 2] = make_uint4(x[0], x[1], x[2], x[3]);
+              out_row[ch * 4 + v * 2 + 1] = make_uint4(x[4], x[5], x[6], x[7]);
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      if (half == 0 && p.lse != nullptr && in_range)
+        p.lse[((int64_t)t.b * p.heads + t.h) * p.lse_stride + row] = m + log2f(l_row);
+    }
+    if (pair_vote(bar_id, false)) pair_sync(bar_id);   // the partner failed where this warp did not
+  }
+};
+
+// ------------------------------- TMA producer -------------------------------
+// One thread.  Ring stages in the order the issuer consumes them: K(0 .. SB-1), then V(n), K(n+SB) for n = 0, 1, ...
+template <bool PERSISTENT>
+__device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
+                                               const CUtensorMap* tm_v, const FwdParams& p, const SchedParams& sp) {
+  using Cfg = SplitCfg;
+  constexpr int SL = Cfg::SLOTS;
+  uint8_t* ring = c.smem + Cfg::Q_TILE_BYTES;
+  int ring_i = 0, tiles = 0;   // stages and Q tiles issued so far
+  bool ok = true;
+  for (int k = 0; ok; ++k) {
+    // the first tile of a CTA is its own index (no round trip to the counter before the first load is issued)
+    int item = k == 0 ? (int)blockIdx.x : sp.total_items;
+    if (PERSISTENT && k > 0) item = (int)(gridDim.x + atomicAdd(&sp.counter[0], 1u));
+    const bool valid = item < sp.total_items;
+    // slot k % 2 still holds item k-2 until every reader has read it
+    if (k >= 2 && !c.wait(Cfg::BAR_SCHED_FREE + (k & 1), (k >> 1) - 1, WAIT_SCHED)) {
+      ok = false;
+      break;
+    }
+    c.sched[k & 1] = valid ? item : -1;
+    mbar_arrive(&c.bars[Cfg::BAR_SCHED + (k & 1)]);
+    if (!valid) {
+      if constexpr (PERSISTENT) {
+        // last CTA out resets the counters for the next launch that uses this pair
+        __threadfence();
+        const unsigned done = atomicAdd(&sp.counter[1], 1u);
+        if (done == gridDim.x - 1) {
+          sp.counter[0] = 0;
+          sp.counter[1] = 0;
+          __threadfence();
+        }
+      }
+      break;
+    }
+    const TileInfo t = decode_item(item, p, sp, Cfg::BN);
+    const int nb = t.hi - t.lo;
+    if (k > 0) ok = c.wait(Cfg::BAR_Q_FREE, k - 1, WAIT_Q_FREE);
+    if (!ok) break;
+    mbar_expect_tx(&c.bars[Cfg::BAR_Q_FULL], Cfg::Q_TILE_BYTES);
+#pragma unroll
+    for (int ks = 0; ks < Cfg::KSUB; ++ks)
+      tma_load_4d(c.smem + ks * (Cfg::BM * 128), tm_q, &c.bars[Cfg::BAR_Q_FULL], ks * 64, t.h, t.q0, t.b);
+    ++tiles;
+    auto load = [&](bool is_v, int n) {
+#pragma unroll
+      for (int part = 0; part < Cfg::PARTS; ++part) {
+        const int slot = ring_i % SL, use = ring_i / SL;
+        if (!ok || (use > 0 && !c.wait(Cfg::BAR_EMPTY + slot, use - 1, WAIT_K_EMPTY))) {
+          ok = false;
+          return;
+        }
+        uint64_t* full = &c.bars[Cfg::BAR_FULL + slot];
+        uint8_t* dst = ring + slot * Cfg::STAGE_BYTES;
+        mbar_expect_tx(full, Cfg::STAGE_BYTES);
+        const int key0 = (t.lo + n) * Cfg::BN;
+        if (is_v) {
+#pragma unroll
+          for (int ks = 0; ks < Cfg::KSUB; ++ks)
+            tma_load_4d(dst + ks * (Cfg::V_KEYS * 128), tm_v, full, ks * 64, t.hk, key0 + part * Cfg::V_KEYS, t.b);
+        } else {
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks)
+            tma_load_4d(dst + ks * (Cfg::BN * 128), tm_k, full, part * 128 + ks * 64, t.hk, key0, t.b);
+        }
+        ++ring_i;
+      }
+    };
+    for (int n = 0; n < Cfg::SB && n < nb && ok; ++n) load(false, n);
+    for (int n = 0; n < nb && ok; ++n) {
+      load(true, n);
+      if (ok && n + Cfg::SB < nb) load(false, n + Cfg::SB);
+    }
+  }
+  if (!ok || *c.abort_flag != 0) {
+    // Abort path: do not leave the CTA while our own bulk copies may still be landing in shared memory.  Wait (bounded, 20 ms) for
+    // the most recent load of every slot and of Q.
+    const uint64_t t0 = global_timer_ns();
+    for (int slot = 0; slot < SL; ++slot) {
+      if (ring_i <= slot) continue;
+      const int last = slot + ((ring_i - 1 - slot) / SL) * SL;   // last stage that used `slot`
+      while (!mbar_try_wait(&c.bars[Cfg::BAR_FULL + slot], (last / SL) & 1) && global_timer_ns() - t0 < 20000000ull) {
+      }
+    }
+    while (tiles > 0 && !mbar_try_wait(&c.bars[Cfg::BAR_Q_FULL], (tiles - 1) & 1) && global_timer_ns() - t0 < 20000000ull) {
+    }
+  }
+}
+
+// -------------------------------- MMA issuer --------------------------------
+// One warp, warp-uniform control flow, an elected lane issues:
+//   softmax(n) -> P -> [O += P V(n)] -> [S(n+SB) = Q K(n+SB)^T] -> softmax(n+SB)
+template <bool BF16>
+__device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams& p, const SchedParams& sp, int lane) {
+  using Cfg = SplitCfg;
+  constexpr int SL = Cfg::SLOTS, D = Cfg::D, BN = Cfg::BN, BM = Cfg::BM, SB = Cfg::SB, PARTS = Cfg::PARTS;
+  constexpr uint32_t IDESC_S = make_idesc(BF16, BM, BN, false, false);
+  constexpr uint32_t IDESC_PV = make_idesc(BF16, BM, D, false, true);
+  // descriptor halves: the upper word is constant, the lower word is (address >> 4) plus a compile-time step
+  const uint32_t desc_hi = smem_desc_hi(1024);
+  const uint32_t ring = smem_u32(c.smem) + Cfg::Q_TILE_BYTES;
+  const uint32_t q_lo = smem_desc_lo(smem_u32(c.smem), 16);
+  const uint32_t k_lo = smem_desc_lo(ring, 16);
+  const uint32_t v_lo = smem_desc_lo(ring, Cfg::V_KEYS * 128);   // MN-major: LBO = bytes between 64-wide column blocks
+  const uint32_t o_tmem = c.tmem_base + Cfg::O_COL;
+  int ring_i = 0, g0 = 0;
+  bool ok = true;
+  auto wait_full = [&](int i) { return c.wait(Cfg::BAR_FULL + i % SL, i / SL, WAIT_K_FULL); };
+  auto issue_s = [&](int gb, bool last_of_tile) {
+    const uint32_t s_tmem = c.tmem_base + (gb % SB) * BN;
+#pragma unroll
+    for (int part = 0; part < PARTS; ++part) {
+      const int slot = ring_i % SL;
+      if (ok) ok = wait_full(ring_i);
+      ++ring_i;
+      if (!ok) return;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t b0 = k_lo + (uint32_t)(slot * (Cfg::STAGE_BYTES >> 4));
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+          const int ka = part * 8 + kk;
+          const uint32_t a_off = (uint32_t)(((ka / 4) * (BM * 128) + (ka % 4) * 32) >> 4);
+          const uint32_t b_off = (uint32_t)(((kk / 4) * (BN * 128) + (kk % 4) * 32) >> 4);
+          if (ka == 0)
+            umma_ss_c<IDESC_S, 0>(s_tmem, q_lo + a_off, b0 + b_off, desc_hi);
+          else
+            umma_ss_c<IDESC_S, 1>(s_tmem, q_lo + a_off, b0 + b_off, desc_hi);
+        }
+        if (part == PARTS - 1) umma_commit(&c.bars[Cfg::BAR_S_FULL + gb % SB]);
+        umma_commit(&c.bars[Cfg::BAR_EMPTY + slot]);
+        if (part == PARTS - 1 && last_of_tile) umma_commit(&c.bars[Cfg::BAR_Q_FREE]);   // no later MMA reads this tile's Q
+      }
+      __syncwarp();
+    }
+  };
+  auto issue_pv = [&](int gb, bool first_of_tile) {
+    const uint32_t p_tmem = c.tmem_base + (gb % SB) * BN;
+#pragma unroll
+    for (int part = 0; part < PARTS; ++part) {   // part = half: keys [64 part, 64 part + 64), P in columns [64 part, 64 part + 32)
+      const int slot = (ring_i + part) % SL;
+      const uint32_t b0 = v_lo + (uint32_t)(slot * (Cfg::STAGE_BYTES >> 4));
+#pragma unroll
+      for (int kk = 0; kk < Cfg::V_KEYS / 16; ++kk) {
+        const uint32_t a = p_tmem + part * Cfg::COLS + kk * 8, b = b0 + (uint32_t)(kk * (2048 >> 4));
+        if (part == 0 && kk == 0 && first_of_tile)
+          umma_ts_c<IDESC_PV, 0>(o_tmem, a, b, desc_hi);
+        else
+          umma_ts_c<IDESC_PV, 1>(o_tmem, a, b, desc_hi);
+      }
+      umma_commit(&c.bars[Cfg::BAR_EMPTY + slot]);
+    }
+    // two O barriers in turn: the softmax can run two blocks ahead of the P V products, and a parity wait is exact only while at most
+    // one phase of a barrier is outstanding
+    umma_commit(&c.bars[Cfg::BAR_O_FULL + (gb & 1)]);
+  };
+  for (int k = 0; ok; ++k) {
+    if (!c.wait_warp(Cfg::BAR_SCHED + (k & 1), k >> 1, WAIT_SCHED)) break;
+    const int item = c.sched[k & 1];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_SCHED_FREE + (k & 1)]);
+    if (item < 0) break;
+    const TileInfo t = decode_item(item, p, sp, BN);
+    const int nb = t.hi - t.lo;
+    ok = c.wait(Cfg::BAR_Q_FULL, k, WAIT_Q_FULL);
+    for (int n = 0; n < SB && n < nb && ok; ++n) issue_s(g0 + n, n == nb - 1);
+    for (int n = 0; n < nb && ok; ++n) {
+      const int gb = g0 + n;
+      // V first: it landed long ago, and nothing but the wait for P should stand before the P V products
+#pragma unroll
+      for (int part = 0; part < PARTS; ++part)
+        if (ok) ok = wait_full(ring_i + part);
+      if (ok) ok = c.wait(Cfg::BAR_P_FULL + gb % SB, gb / SB, WAIT_P_FULL);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) issue_pv(gb, n == 0);
+      __syncwarp();
+      ring_i += PARTS;
+      if (n + SB < nb) issue_s(gb + SB, n + SB == nb - 1);
+    }
+    g0 += nb;
+  }
+  // every MMA issued above has retired before the CTA tears TMEM down
+  if (elect_one()) umma_commit(&c.bars[Cfg::BAR_DRAIN]);
+  __syncwarp();
+  c.wait(Cfg::BAR_DRAIN, 0, WAIT_DRAIN);
+}
+
+// PERSISTENT: tiles from the counter; otherwise one tile per CTA (A/B timing).
+template <bool BF16, bool SOFTCAP, bool PERSISTENT>
+__global__ void __launch_bounds__(SplitCfg::THREADS, 1)
+attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                      const __grid_constant__ CUtensorMap tm_v, const FwdParams p, const SchedParams sp) {
+  using Cfg = SplitCfg;
+  extern __shared__ uint8_t smem_raw[];
+  if (threadIdx.x == 32) prefetch_l2(&g_device_status);   // read after the wait below
+  SplitCtx c;
+  c.smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  c.bars = reinterpret_cast<uint64_t*>(c.smem + Cfg::OFF_BARS);
+  c.xch = reinterpret_cast<float*>(c.smem + Cfg::OFF_XCH);
+  c.fail = reinterpret_cast<volatile int*>(c.smem + Cfg::OFF_FAIL);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c.smem + Cfg::OFF_MISC);
+  c.abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  c.sched = reinterpret_cast<volatile int*>(tmem_slot + 2);
+  c.skip = reinterpret_cast<volatile int*>(tmem_slot + 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 0; i < Cfg::NUM_BARS; ++i) {
+      const bool p_full = i >= Cfg::BAR_P_FULL && i < Cfg::BAR_P_FULL + Cfg::SB;
+      const bool sched_free = i >= Cfg::BAR_SCHED_FREE && i < Cfg::BAR_SCHED_FREE + 2;
+      mbar_init(&c.bars[i], p_full ? (uint32_t)Cfg::SOFTMAX_WARPS : sched_free ? (uint32_t)Cfg::SOFTMAX_WARPS + 1u : 1u);
+    }
+    for (int i = 0; i < 4; ++i) c.fail[i] = 0;
+    *c.abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == Cfg::PRODUCER_WARP && lane == 0) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
+  // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
+  // to allocate columns of its own, and what it wrote is visible only now.
+  pdl_wait();
+  if (threadIdx.x == 32) *c.skip = *reinterpret_cast<volatile int*>(&g_device_status);
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  c.tmem_base = *tmem_slot;
+  // A launch that follows an expired wait on this device drains immediately (the status word stays set until the host reads it; the
+  // tile counter is untouched: the host zeroes it when it clears the word).
+  if (*c.skip == 0) {
+    if (warp < Cfg::SOFTMAX_WARPS) {
+      SplitSoftmax<BF16, SOFTCAP> s(c, p, warp, lane);
+      s.run(sp);
+    } else if (warp == Cfg::PRODUCER_WARP) {
+      if (lane == 0) split_producer<PERSISTENT>(c, &tm_q, &tm_k, &tm_v, p, sp);
+    } else {
+      split_issuer<BF16>(c, p, sp, lane);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(c.tmem_base, Cfg::TMEM_COLS);
+}
+
+template <bool BF16, bool SOFTCAP, bool PERSISTENT>
+int launch_attn_fwd_split_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
+                             cudaStream_t stream) {
+  auto kern = attn_fwd_split_kernel<BF16, SOFTCAP, PERSISTENT>;
+  static thread_local int configured_dev = -1;
+  int dev = 0;
+  B200_CUDA_TRY(cudaGetDevice(&dev));
+  if (configured_dev != dev) {
+    B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg::SMEM_BYTES));
+    configured_dev = dev;
+  }
+  SchedParams sp;
+  const int rc = sched_params(&sp, p, SplitCfg::D, PERSISTENT);
+  if (rc != B200_OK) return rc;
+  const int grid = PERSISTENT ? std::min(sp.total_items, sm_count()) : sp.total_items;
+  B200_CUDA_TRY(launch_kernel(kern, grid, SplitCfg::THREADS, SplitCfg::SMEM_BYTES, stream, 1, tq, tk, tv, p, sp));
+  return B200_OK;
+}
+
+template <bool BF16, bool SOFTCAP>
+int launch_attn_fwd_split(const void* q, const void* k, const void* v, const FwdParams& p, const AttnStrides& st,
+                          bool one_tile_per_cta, cudaStream_t stream) {
+  using Cfg = SplitCfg;
+  CUtensorMap tq, tk, tv;
+  int rc;
+  if ((rc = make_bshd_tensor_map(&tq, q, p.batch, p.q_len, p.heads, Cfg::D, Cfg::BM, BF16, st.q_token, st.q_batch)) != B200_OK ||
+      (rc = make_bshd_tensor_map(&tk, k, p.batch, p.kv_len, p.kv_heads, Cfg::D, Cfg::BN, BF16, st.k_token, st.k_batch)) != B200_OK ||
+      (rc = make_bshd_tensor_map(&tv, v, p.batch, p.kv_len, p.kv_heads, Cfg::D, Cfg::V_KEYS, BF16, st.v_token, st.v_batch)) !=
+          B200_OK)
+    return rc;
+  return one_tile_per_cta ? launch_attn_fwd_split_as<BF16, SOFTCAP, false>(tq, tk, tv, p, stream)
+                          : launch_attn_fwd_split_as<BF16, SOFTCAP, true>(tq, tk, tv, p, stream);
+}
+
+}  // namespace b200

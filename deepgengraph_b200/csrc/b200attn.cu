@@ -9,6 +9,7 @@
 #include "elementwise.cuh"
 #include "attn_fwd.cuh"
 #include "attn_fwd_persist.cuh"
+#include "attn_fwd_split.cuh"
 #include "attn_decode.cuh"
 #include "attn_sweep.cuh"
 #include "kv_evict.cuh"
