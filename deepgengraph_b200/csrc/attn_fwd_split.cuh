@@ -7,11 +7,12 @@
 // What bounds it and why this shape.  Per block of 128 keys the tensor pipe needs 16 x 64 clk for S and 8 x 128 for P V, 2048 in all,
 // the special-function unit 1024, and with the soft-cap the softmax is issue-bound on top.  With 64-key blocks and one softmax
 // warpgroup a block cost every hand-over (S -> softmax -> P -> P V) twice as often, and one warp per SM sub-partition could not keep
-// up with the soft-cap: 1771 clk per 64 keys, where this one takes 3058 per 128 (2832 without the soft-cap: the issuer's barrier
-// polls, 630 clk a block, leave the pipe idle).  S with N = 128 runs at the full rate with Q in shared memory (N = 64: 48 instead
-// of 32 clk), so Q needs no TMEM and both S buffers hold 128 keys.
-// Measured, before -> now (one box, bf16): 16/8 heads, 8192 tokens, window 4096, soft-cap 50: 375 -> 353 us (422 -> 394 in a loop under
-// the power cap); 500 queries on 4000 keys, soft-cap: 65.5 -> 60.5; causal without soft-cap, 8192 tokens: 410 -> 410.
+// up with the soft-cap: 1771 clk per 64 keys, where the first form of this kernel took 3058 per 128 (2832 without the soft-cap, 630 of
+// them the issuer's barrier polls).  S with N = 128 runs at the full rate with Q in shared memory (N = 64: 48 instead of 32 clk), so
+// Q needs no TMEM and both S buffers hold 128 keys.
+// Measured, before -> now (one box, bf16, idle GPU / in a loop under the power cap): 16/8 heads, 8192 tokens, window 4096, soft-cap 50:
+// 379 -> 347 / 422 -> 385 us; 500 queries on 4000 keys, soft-cap: 66.6 -> 57 / 65 -> 55; causal without soft-cap, 8192 tokens:
+// 412 -> 409 / 456 -> 454.
 #pragma once
 
 #include "attn_fwd_persist.cuh"
@@ -442,7 +443,7 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
 }
 
 // -------------------------------- MMA issuer --------------------------------
-// One warp, warp-uniform control flow, an elected lane issues:
+// One warp, convergent control flow, an elected lane issues (umma_ss_if):
 //   softmax(n) -> P -> [O += P V(n)] -> [S(n+SB) = Q K(n+SB)^T] -> softmax(n+SB)
 template <bool BF16>
 __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams& p, const SchedParams& sp, int lane) {
@@ -457,6 +458,7 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
   const uint32_t k_lo = smem_desc_lo(ring, 16);
   const uint32_t v_lo = smem_desc_lo(ring, Cfg::V_KEYS * 128);   // MN-major: LBO = bytes between 64-wide column blocks
   const uint32_t o_tmem = c.tmem_base + Cfg::O_COL;
+  const uint32_t elected = elect_one(), bars = smem_u32(c.bars);
   int ring_i = 0, g0 = 0;
   bool ok = true;
   auto wait_full = [&](int i) { return c.wait(Cfg::BAR_FULL + i % SL, i / SL, WAIT_K_FULL); };
@@ -469,23 +471,17 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
       ++ring_i;
       if (!ok) return;
       tc_fence_after();
-      if (elect_one()) {
-        const uint32_t b0 = k_lo + (uint32_t)(slot * (Cfg::STAGE_BYTES >> 4));
+      const uint32_t b0 = k_lo + (uint32_t)(slot * (Cfg::STAGE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const int ka = part * 8 + kk;
-          const uint32_t a_off = (uint32_t)(((ka / 4) * (BM * 128) + (ka % 4) * 32) >> 4);
-          const uint32_t b_off = (uint32_t)(((kk / 4) * (BN * 128) + (kk % 4) * 32) >> 4);
-          if (ka == 0)
-            umma_ss_c<IDESC_S, 0>(s_tmem, q_lo + a_off, b0 + b_off, desc_hi);
-          else
-            umma_ss_c<IDESC_S, 1>(s_tmem, q_lo + a_off, b0 + b_off, desc_hi);
-        }
-        if (part == PARTS - 1) umma_commit(&c.bars[Cfg::BAR_S_FULL + gb % SB]);
-        umma_commit(&c.bars[Cfg::BAR_EMPTY + slot]);
-        if (part == PARTS - 1 && last_of_tile) umma_commit(&c.bars[Cfg::BAR_Q_FREE]);   // no later MMA reads this tile's Q
+      for (int kk = 0; kk < 8; ++kk) {
+        const int ka = part * 8 + kk;
+        const uint32_t a_off = (uint32_t)(((ka / 4) * (BM * 128) + (ka % 4) * 32) >> 4);
+        const uint32_t b_off = (uint32_t)(((kk / 4) * (BN * 128) + (kk % 4) * 32) >> 4);
+        umma_ss_if<IDESC_S>(elected, s_tmem, q_lo + a_off, b0 + b_off, desc_hi, ka == 0 ? 0u : 1u);
       }
-      __syncwarp();
+      if (part == PARTS - 1) umma_commit_if(elected, bars + 8 * (Cfg::BAR_S_FULL + gb % SB));
+      umma_commit_if(elected, bars + 8 * (Cfg::BAR_EMPTY + slot));
+      if (part == PARTS - 1 && last_of_tile) umma_commit_if(elected, bars + 8 * Cfg::BAR_Q_FREE);   // no later MMA reads this Q
     }
   };
   auto issue_pv = [&](int gb, bool first_of_tile) {
@@ -497,16 +493,13 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
 #pragma unroll
       for (int kk = 0; kk < Cfg::V_KEYS / 16; ++kk) {
         const uint32_t a = p_tmem + part * Cfg::COLS + kk * 8, b = b0 + (uint32_t)(kk * (2048 >> 4));
-        if (part == 0 && kk == 0 && first_of_tile)
-          umma_ts_c<IDESC_PV, 0>(o_tmem, a, b, desc_hi);
-        else
-          umma_ts_c<IDESC_PV, 1>(o_tmem, a, b, desc_hi);
+        umma_ts_if<IDESC_PV>(elected, o_tmem, a, b, desc_hi, (part == 0 && kk == 0 && first_of_tile) ? 0u : 1u);
       }
-      umma_commit(&c.bars[Cfg::BAR_EMPTY + slot]);
+      umma_commit_if(elected, bars + 8 * (Cfg::BAR_EMPTY + slot));
     }
     // two O barriers in turn: the softmax can run two blocks ahead of the P V products, and a parity wait is exact only while at most
     // one phase of a barrier is outstanding
-    umma_commit(&c.bars[Cfg::BAR_O_FULL + (gb & 1)]);
+    umma_commit_if(elected, bars + 8 * (Cfg::BAR_O_FULL + (gb & 1)));
   };
   for (int k = 0; ok; ++k) {
     if (!c.wait_warp(Cfg::BAR_SCHED + (k & 1), k >> 1, WAIT_SCHED)) break;
@@ -527,16 +520,14 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
       if (ok) ok = c.wait(Cfg::BAR_P_FULL + gb % SB, gb / SB, WAIT_P_FULL);
       if (!ok) break;
       tc_fence_after();
-      if (elect_one()) issue_pv(gb, n == 0);
-      __syncwarp();
+      issue_pv(gb, n == 0);
       ring_i += PARTS;
       if (n + SB < nb) issue_s(gb + SB, n + SB == nb - 1);
     }
     g0 += nb;
   }
   // every MMA issued above has retired before the CTA tears TMEM down
-  if (elect_one()) umma_commit(&c.bars[Cfg::BAR_DRAIN]);
-  __syncwarp();
+  umma_commit_if(elected, bars + 8 * Cfg::BAR_DRAIN);
   c.wait(Cfg::BAR_DRAIN, 0, WAIT_DRAIN);
 }
 
