@@ -359,7 +359,7 @@ __device__ __forceinline__ bool fwd_softmax_block(const FwdCtx<Cfg, BF16>& c, co
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         float s = __uint_as_float(sr[ch][i + u]);
-        [[maybe_unused]] float sa = fabsf(s);
+        [[maybe_unused]] float sa = s;
         if constexpr (MASK) {
           const int col = ch * 32 + i + u;
           if (col > hi_c || col < lo_c) {
@@ -375,8 +375,8 @@ __device__ __forceinline__ bool fwd_softmax_block(const FwdCtx<Cfg, BF16>& c, co
       mx0 = fmax3(mx0, v[0], v[1]);
       mx1 = fmax3(mx1, v[2], v[3]);
       if constexpr (SOFTCAP) {
-        ab0 = fmax3(ab0, va[0], va[1]);
-        ab1 = fmax3(ab1, va[2], va[3]);
+        ab0 = fmax3_abs(ab0, va[0], va[1]);
+        ab1 = fmax3_abs(ab1, va[2], va[3]);
       }
     }
   }

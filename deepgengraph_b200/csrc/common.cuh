@@ -462,6 +462,13 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// of the magnitudes (an fabsf before an asm operand is an instruction of its own: soft-capped attention, 8192 tokens at head_dim 256
+// 380 -> 374 us, 2 x 4096 tokens at head_dim 128 377 -> 372)
+__device__ __forceinline__ float fmax3_abs(float a, float b, float c) {
+  float d;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
   float2 d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;"
@@ -518,8 +525,8 @@ __device__ __forceinline__ bool softcap_chunk_poly_only(const uint32_t (&sr)[32]
   float a0 = 0.f, a1 = 0.f;
 #pragma unroll
   for (int i = 0; i < 32; i += 4) {
-    a0 = fmax3(a0, fabsf(__uint_as_float(sr[i])), fabsf(__uint_as_float(sr[i + 1])));
-    a1 = fmax3(a1, fabsf(__uint_as_float(sr[i + 2])), fabsf(__uint_as_float(sr[i + 3])));
+    a0 = fmax3_abs(a0, __uint_as_float(sr[i]), __uint_as_float(sr[i + 1]));
+    a1 = fmax3_abs(a1, __uint_as_float(sr[i + 2]), __uint_as_float(sr[i + 3]));
   }
   return !__any_sync(0xffffffffu, fmaxf(a0, a1) * cap_in > kCapPolyMax);
 }
