@@ -18,8 +18,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libb200attn.so")
 SOURCES = ["b200attn.cu"]
 HEADER = os.path.join("..", "..", "include", "b200attn.h")
-DEPS = ["b200attn.cu", "common.cuh", "elementwise.cuh", "attn_fwd.cuh", "attn_fwd_persist.cuh", "attn_fwd_split.cuh", "attn_decode.cuh",
-        "attn_decode_plan.h", "attn_sweep.cuh", "kv_evict.cuh", HEADER]
+DEPS = ["b200attn.cu", "common.cuh", "elementwise.cuh", "attn_fwd.cuh", "attn_fwd_persist.cuh", "attn_fwd_split.cuh", "attn_pair.h",
+        "attn_decode.cuh", "attn_decode_plan.h", "attn_sweep.cuh", "kv_evict.cuh", HEADER]
 TORCH_DEPS = ["torch_binding.cpp", HEADER]
 
 

@@ -16,6 +16,7 @@
 #pragma once
 
 #include "attn_fwd_persist.cuh"
+#include "attn_pair.h"
 
 namespace b200 {
 
@@ -90,8 +91,7 @@ __device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sy
 // and where a block's maximum exceeds it by more than 2^8 (lazy rescale).  So the common block costs one vote between the two warps
 // of a 32-row group; only after a vote for it are the maxima exchanged through shared memory.
 //
-// Steps and failure.  Every pair_vote is a step; a step whose vote comes out true is followed by one pair_sync, after which the
-// pair's failure flag is looked at.  A warp whose bounded wait ran out sets the flag, takes part in one more step with a true
+// Steps and failure: attn_pair.h.  A warp whose bounded wait ran out sets the pair's flag, takes part in one more step with a true
 // vote and leaves; its partner leaves in that same step.  A warp that is done takes part in one last step.  No named barrier is ever
 // waited for alone.
 template <bool BF16, bool SOFTCAP>
@@ -109,12 +109,14 @@ struct SplitSoftmax {
         lane_addr(c_.tmem_base + ((uint32_t)((warp & 3) * 32) << 16)),
         o_addr(c_.tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::O_COL + (warp >> 2) * (D / 2)) {}
 
-  __device__ __forceinline__ volatile float* xch(int h) const { return c.xch + h * Cfg::BM + warp_q * 32 + lane; }
-  __device__ __forceinline__ void leave_failed() const {
-    c.fail[warp_q] = 1;
-    pair_vote(bar_id, true);
-    pair_sync(bar_id);
-  }
+  // the operations of attn_pair.h
+  __device__ __forceinline__ bool vote(bool x) const { return pair_vote(bar_id, x); }
+  __device__ __forceinline__ void sync() const { pair_sync(bar_id); }
+  __device__ __forceinline__ void put(float x) const { word(half) = x; }
+  __device__ __forceinline__ float get() const { return word(half ^ 1); }
+  __device__ __forceinline__ void fail() const { c.fail[warp_q] = 1; }
+  __device__ __forceinline__ bool failed() const { return c.fail[warp_q] != 0; }
+  __device__ __forceinline__ volatile float& word(int h) const { return c.xch[h * Cfg::BM + warp_q * 32 + lane]; }
 
   // One block of one row.  `g` counts the CTA's blocks, n those of the tile.  False: leave (no further step).
   template <bool MASK>
@@ -171,12 +173,9 @@ struct SplitSoftmax {
     } else {
       m_blk *= cmul;
     }
-    if (pair_vote(bar_id, !ok || n == 0 || m_blk - m > 8.0f)) {   // exp2(x - m) stays <= 256
-      if (!ok) c.fail[warp_q] = 1;
-      *xch(half) = m_blk;
-      pair_sync(bar_id);
-      if (c.fail[warp_q] != 0) return false;
-      m_blk = fmaxf(m_blk, *xch(half ^ 1));
+    const PairStep step = pair_block(*this, ok, n == 0 || m_blk - m > 8.0f, m_blk);   // exp2(x - m) stays <= 256
+    if (step == PairStep::kLeave) return false;
+    if (step == PairStep::kMoved) {
       if (n == 0) {
         m = fmaxf(m, m_blk);
       } else {
@@ -192,7 +191,7 @@ struct SplitSoftmax {
           // P V(g-1): its barrier is exactly in or just past the awaited phase -- S(g) complete implies P V(g-2), and P V(g+1) waits
           // for this thread's P(g).
           if (!c.wait_warp(Cfg::BAR_O_FULL + ((g - 1) & 1), (g - 1) >> 1, WAIT_O_FULL)) {
-            leave_failed();
+            pair_leave(*this);
             return false;
           }
           tc_fence_after();
@@ -283,7 +282,7 @@ struct SplitSoftmax {
     int g = 0;
     for (int k = 0;; ++k) {
       if (!c.wait_warp(Cfg::BAR_SCHED + (k & 1), k >> 1, WAIT_SCHED)) {
-        leave_failed();
+        pair_leave(*this);
         return;
       }
       const int item = c.sched[k & 1];
@@ -307,15 +306,8 @@ struct SplitSoftmax {
       }
       // Epilogue; the issuer is already computing the next tile's S meanwhile.  The next tile's first P V (which overwrites O) is
       // issued only after this warp has delivered that tile's first P, i.e. after the loads below have completed.
-      *xch(half) = l;
-      const bool ok = c.wait(Cfg::BAR_O_FULL + ((g - 1) & 1), (g - 1) >> 1, WAIT_O_FULL);
-      if (!ok) c.fail[warp_q] = 1;
-      if (pair_vote(bar_id, !ok)) {
-        pair_sync(bar_id);
-        return;
-      }
-      const float l_other = *xch(half ^ 1);
-      const float l_row = l + l_other;
+      float l_row = l;
+      if (!pair_total(*this, [&] { return c.wait(Cfg::BAR_O_FULL + ((g - 1) & 1), (g - 1) >> 1, WAIT_O_FULL); }, l_row)) return;
       tc_fence_after();
       const float inv_l = 1.0f / l_row;
       const bool in_range = row < p.q_len;
@@ -349,7 +341,7 @@ struct SplitSoftmax {
       if (half == 0 && p.lse != nullptr && in_range)
         p.lse[((int64_t)t.b * p.heads + t.h) * p.lse_stride + row] = m + log2f(l_row);
     }
-    if (pair_vote(bar_id, false)) pair_sync(bar_id);   // the partner failed where this warp did not
+    pair_finish(*this);
   }
 };
 
