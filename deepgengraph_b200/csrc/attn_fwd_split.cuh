@@ -43,12 +43,11 @@ struct SplitCfg {
   static constexpr int BAR_SCHED_FREE = BAR_SCHED + 2;       // [2] read by the softmax warps and the issuer
   static constexpr int BAR_DRAIN = BAR_SCHED_FREE + 2;
   static constexpr int NUM_BARS = BAR_DRAIN + 1;
-  // behind the tiles: barriers, [half][row] floats (maxima and sums handed between a row's two threads), a failure flag per pair of
-  // softmax warps, TMEM address, abort flag, two scheduler slots, skip flag
+  // behind the tiles: barriers, [half][row] floats (maxima and sums handed between a row's two threads), TMEM address, abort flag, two
+  // scheduler slots, skip flag
   static constexpr int OFF_BARS = Q_TILE_BYTES + SLOTS * STAGE_BYTES;
   static constexpr int OFF_XCH = OFF_BARS + (NUM_BARS * 8 + 15) / 16 * 16;
-  static constexpr int OFF_FAIL = OFF_XCH + 2 * BM * 4;
-  static constexpr int OFF_MISC = OFF_FAIL + 16;
+  static constexpr int OFF_MISC = OFF_XCH + 2 * BM * 4;
   static constexpr int SMEM_BYTES = OFF_MISC + 32 + 1024;    // +1024: manual alignment
   static_assert(SMEM_BYTES <= 232448, "shared memory budget exceeded");
 };
@@ -57,7 +56,6 @@ struct SplitCtx {
   uint8_t* smem;
   uint64_t* bars;
   float* xch;
-  volatile int* fail;
   volatile int* abort_flag;
   volatile int* sched;   // [2] item index or -1
   volatile int* skip;    // status word of the device at the start
@@ -84,16 +82,14 @@ __device__ __forceinline__ bool pair_vote(int id, bool pred) {
       : "memory");
   return r != 0;
 }
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
 
 // ------------------------------ softmax warps ------------------------------
 // Both threads of a row need the same reference maximum m (their P feed one accumulator), but m moves only in a tile's first block
 // and where a block's maximum exceeds it by more than 2^8 (lazy rescale).  So the common block costs one vote between the two warps
 // of a 32-row group; only after a vote for it are the maxima exchanged through shared memory.
 //
-// Steps and failure: attn_pair.h.  A warp whose bounded wait ran out sets the pair's flag, takes part in one more step with a true
-// vote and leaves; its partner leaves in that same step.  A warp that is done takes part in one last step.  No named barrier is ever
-// waited for alone.
+// Steps and failure: attn_pair.h.  A warp whose bounded wait ran out takes part in one more step and leaves; its partner leaves in
+// that same step.  A warp that is done takes part in one last step.  No named barrier is ever waited for alone.
 template <bool BF16, bool SOFTCAP>
 struct SplitSoftmax {
   using Cfg = SplitCfg;
@@ -111,11 +107,8 @@ struct SplitSoftmax {
 
   // the operations of attn_pair.h
   __device__ __forceinline__ bool vote(bool x) const { return pair_vote(bar_id, x); }
-  __device__ __forceinline__ void sync() const { pair_sync(bar_id); }
   __device__ __forceinline__ void put(float x) const { word(half) = x; }
   __device__ __forceinline__ float get() const { return word(half ^ 1); }
-  __device__ __forceinline__ void fail() const { c.fail[warp_q] = 1; }
-  __device__ __forceinline__ bool failed() const { return c.fail[warp_q] != 0; }
   __device__ __forceinline__ volatile float& word(int h) const { return c.xch[h * Cfg::BM + warp_q * 32 + lane]; }
 
   // One block of one row.  `g` counts the CTA's blocks, n those of the tile.  False: leave (no further step).
@@ -535,7 +528,6 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   c.smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   c.bars = reinterpret_cast<uint64_t*>(c.smem + Cfg::OFF_BARS);
   c.xch = reinterpret_cast<float*>(c.smem + Cfg::OFF_XCH);
-  c.fail = reinterpret_cast<volatile int*>(c.smem + Cfg::OFF_FAIL);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c.smem + Cfg::OFF_MISC);
   c.abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   c.sched = reinterpret_cast<volatile int*>(tmem_slot + 2);
@@ -548,7 +540,6 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const bool sched_free = i >= Cfg::BAR_SCHED_FREE && i < Cfg::BAR_SCHED_FREE + 2;
       mbar_init(&c.bars[i], p_full ? (uint32_t)Cfg::SOFTMAX_WARPS : sched_free ? (uint32_t)Cfg::SOFTMAX_WARPS + 1u : 1u);
     }
-    for (int i = 0; i < 4; ++i) c.fail[i] = 0;
     *c.abort_flag = 0;
     fence_mbar_init();
   }

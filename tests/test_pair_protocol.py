@@ -1,5 +1,6 @@
 """How the two warps that share a query tile's rows exchange maxima and sums (csrc/attn_pair.h), run on the host as two coroutines
-under many orders of their steps.  Every value read must be the one that the partner wrote for that step."""
+under many orders of their steps.  Every value read must be the one that the partner wrote for that step, and no warp may be left
+waiting in a barrier."""
 import os
 import subprocess
 
@@ -22,7 +23,7 @@ char stack[2][1 << 16];
 bool done[2], blocked[2];
 // what the two warps share
 int arrived, generation, delivered[2];
-bool ored, result, flag, aborted;
+bool ored, result, aborted;
 float word[2];
 // the problem: blocks per tile, a maximum and a sum for each block and half, one wait that runs out (or none)
 int blocks[kTiles], expiring_warp, expiring_wait;
@@ -50,11 +51,8 @@ struct Pair {
     while (generation == mine) yield(id);
     return result;
   }
-  void sync() const { vote(false); }
   void put(float x) const { yield(id); word[id] = x; }
   float get() const { yield(id); return word[id ^ 1]; }
-  void fail() const { yield(id); flag = true; }
-  bool failed() const { yield(id); return flag; }
 };
 
 // a bounded wait: runs out where the problem says so, and once the other warp has given up
@@ -106,7 +104,7 @@ void entry(int id) {
 int run_one(unsigned seed, bool failures) {
   rng.seed(seed);
   arrived = generation = 0;
-  ored = result = flag = aborted = false;
+  ored = result = aborted = false;
   expiring_warp = failures ? (int)(rng() % 2) : -1;
   expiring_wait = (int)(rng() % 16);
   for (int t = 0; t < kTiles; ++t) {
@@ -169,4 +167,9 @@ def program(tmp_path_factory):
 
 def test_every_value_read_belongs_to_its_step(program):
   waiting, wrong = map(int, subprocess.run([program, "0"], check=True, capture_output=True, text=True, timeout=300).stdout.split())
+  assert (waiting, wrong) == (0, 0)
+
+
+def test_a_wait_that_runs_out_ends_both_warps(program):
+  waiting, wrong = map(int, subprocess.run([program, "1"], check=True, capture_output=True, text=True, timeout=300).stdout.split())
   assert (waiting, wrong) == (0, 0)
