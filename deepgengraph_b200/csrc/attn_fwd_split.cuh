@@ -428,8 +428,10 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
 }
 
 // -------------------------------- MMA issuer --------------------------------
-// One warp, convergent control flow, an elected lane issues (umma_ss_if):
+// One warp, an elected lane issues (umma_ss_if):
 //   softmax(n) -> P -> [O += P V(n)] -> [S(n+SB) = Q K(n+SB)^T] -> softmax(n+SB)
+// The control flow is convergent unless a wait runs out: then one lane may have seen the abort flag and another the barrier's phase.
+// Inside of a tile nothing waits for the whole warp, and `ok` is voted on at the end of each tile, so all lanes leave together.
 template <bool BF16>
 __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams& p, const SchedParams& sp, int lane) {
   using Cfg = SplitCfg;
@@ -509,6 +511,7 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
       ring_i += PARTS;
       if (n + SB < nb) issue_s(gb + SB, n + SB == nb - 1);
     }
+    ok = __all_sync(0xffffffffu, ok);
     g0 += nb;
   }
   // every MMA issued above has retired before the CTA tears TMEM down
