@@ -52,6 +52,17 @@ struct SplitCfg {
   static_assert(SMEM_BYTES <= 232448, "shared memory budget exceeded");
 };
 
+// Blocks of one query tile, whose visible key range [lo, hi) is in half blocks: the first block starts at the first visible half, so
+// only the last one can be half a block.  For that one there is no second V stage, no P V of its second half and no work for the second
+// warpgroup.  In whole blocks only, short prompts and narrow windows paid for up to twice their keys (us, whole -> with a half block;
+// 16/8 heads): 64 tokens 7.28 -> 6.48, 8 x 40 heads of 64 tokens 15.8 -> 13.0, 8192 tokens with a window of 16 58.8 -> 52.2, of 16 with
+// soft-cap 68.6 -> 61.4; calls without a half block keep their times within 2 % (8 x 40 heads, 200 tokens, soft-cap 36.2 -> 36.4).
+struct SplitBlocks {
+  int count;
+  bool half_last;
+  __device__ __forceinline__ explicit SplitBlocks(const TileInfo& t) : count((t.hi - t.lo + 1) >> 1), half_last(((t.hi - t.lo) & 1) != 0) {}
+};
+
 struct SplitCtx {
   uint8_t* smem;
   uint64_t* bars;
@@ -111,6 +122,66 @@ struct SplitSoftmax {
   __device__ __forceinline__ float get() const { return word(half ^ 1); }
   __device__ __forceinline__ volatile float& word(int h) const { return c.xch[h * Cfg::BM + warp_q * 32 + lane]; }
 
+  // The reference maximum moves where a block's maximum asks for it: m, and l and O with it.  False: leave.
+  __device__ __forceinline__ bool agree(int n, int g, bool ok, float m_blk) {
+    const PairStep step = pair_block(*this, ok, n == 0 || m_blk - m > 8.0f, m_blk);   // exp2(x - m) stays <= 256
+    if (step == PairStep::kLeave) return false;
+    if (step == PairStep::kMoved) {
+      if (n == 0) {
+        m = fmaxf(m, m_blk);
+      } else {
+        float alpha = 1.0f;
+        bool rescale = false;
+        if (m_blk - m > 8.0f) {
+          alpha = ex2_approx(m - m_blk);
+          m = m_blk;
+          l *= alpha;
+          rescale = true;
+        }
+        if (__any_sync(0xffffffffu, rescale)) {   // the same in both warps: they hold the same rows
+          // P V(g-1): its barrier is exactly in or just past the awaited phase -- S(g) complete implies P V(g-2), and P V(g+1) waits
+          // for this thread's P(g).
+          if (!c.wait_warp(Cfg::BAR_O_FULL + ((g - 1) & 1), (g - 1) >> 1, WAIT_O_FULL)) {
+            pair_leave(*this);
+            return false;
+          }
+          tc_fence_after();
+          const float2 a2 = make_float2(alpha, alpha);
+#pragma unroll
+          for (int ch = 0; ch < D / 2 / 16; ++ch) {
+            uint32_t o[16];
+            tmem_ld16(o_addr + ch * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              const float2 r = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), a2);
+              o[i] = __float_as_uint(r.x);
+              o[i + 1] = __float_as_uint(r.y);
+            }
+            tmem_st16(o_addr + ch * 16, o);
+          }
+        }
+      }
+    }
+    return true;
+  }
+  __device__ __forceinline__ void deliver(int buf) const {
+    tmem_st_wait();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_P_FULL + buf]);
+  }
+
+  // A half block of the second warpgroup: no keys, but its half of O moves with the maximum.
+  __device__ __forceinline__ bool block_without_keys(int n, int g) {
+    const int buf = g % SB;
+    const bool ok = c.wait(Cfg::BAR_S_FULL + buf, g / SB, WAIT_S_FULL);
+    tc_fence_after();
+    if (!agree(n, g, ok, -INFINITY)) return false;
+    deliver(buf);
+    return true;
+  }
+
   // One block of one row.  `g` counts the CTA's blocks, n those of the tile.  False: leave (no further step).
   template <bool MASK>
   __device__ __forceinline__ bool block(int n, int g, int lo_c, int hi_c, float cmul) {
@@ -166,45 +237,7 @@ struct SplitSoftmax {
     } else {
       m_blk *= cmul;
     }
-    const PairStep step = pair_block(*this, ok, n == 0 || m_blk - m > 8.0f, m_blk);   // exp2(x - m) stays <= 256
-    if (step == PairStep::kLeave) return false;
-    if (step == PairStep::kMoved) {
-      if (n == 0) {
-        m = fmaxf(m, m_blk);
-      } else {
-        float alpha = 1.0f;
-        bool rescale = false;
-        if (m_blk - m > 8.0f) {
-          alpha = ex2_approx(m - m_blk);
-          m = m_blk;
-          l *= alpha;
-          rescale = true;
-        }
-        if (__any_sync(0xffffffffu, rescale)) {   // the same in both warps: they hold the same rows
-          // P V(g-1): its barrier is exactly in or just past the awaited phase -- S(g) complete implies P V(g-2), and P V(g+1) waits
-          // for this thread's P(g).
-          if (!c.wait_warp(Cfg::BAR_O_FULL + ((g - 1) & 1), (g - 1) >> 1, WAIT_O_FULL)) {
-            pair_leave(*this);
-            return false;
-          }
-          tc_fence_after();
-          const float2 a2 = make_float2(alpha, alpha);
-#pragma unroll
-          for (int ch = 0; ch < D / 2 / 16; ++ch) {
-            uint32_t o[16];
-            tmem_ld16(o_addr + ch * 16, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-              const float2 r = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), a2);
-              o[i] = __float_as_uint(r.x);
-              o[i + 1] = __float_as_uint(r.y);
-            }
-            tmem_st16(o_addr + ch * 16, o);
-          }
-        }
-      }
-    }
+    if (!agree(n, g, ok, m_blk)) return false;
     // P = exp2(x - m), packed to the 16-bit input type, written over the first half of the thread's own S columns
     const float2 c2 = make_float2(cmul, cmul), nm2 = make_float2(-m, -m);
     float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
@@ -263,10 +296,7 @@ struct SplitSoftmax {
       exp_pass(std::false_type{});
     }
     l += (acc0.x + acc0.y) + (acc1.x + acc1.y);
-    tmem_st_wait();
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_P_FULL + buf]);
+    deliver(buf);
     return true;
   }
 
@@ -282,7 +312,8 @@ struct SplitSoftmax {
       __syncwarp();
       if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_SCHED_FREE + (k & 1)]);   // slot may be rewritten for item k + 2
       if (item < 0) break;
-      const TileInfo t = decode_item(item, p, sp, Cfg::BN);
+      const TileInfo t = decode_item(item, p, sp, COLS);
+      const SplitBlocks blocks(t);
       const int row = t.q0 + warp_q * 32 + lane;
       m = -1.0e30f;   // finite, so that fully masked blocks stay NaN-free
       l = 0.f;
@@ -291,11 +322,16 @@ struct SplitSoftmax {
       const int lo_key = ((p.causal && p.window > 0) ? (row + p.delta - p.window + 1) : -(1 << 28)) - half * COLS;
       const int hi_first = p.causal ? min(t.q0 + p.delta, p.kv_len - 1) : p.kv_len - 1;
       const int lo_last = (p.causal && p.window > 0) ? (t.q0 + 127 + p.delta - p.window + 1) : -(1 << 28);
-      for (int j = t.lo; j < t.hi; ++j, ++g) {
-        const int n = j - t.lo, k0 = j * Cfg::BN;
+      const int with_keys = blocks.count - (half == 1 && blocks.half_last ? 1 : 0);
+      for (int n = 0; n < with_keys; ++n, ++g) {
+        const int k0 = t.lo * COLS + n * Cfg::BN;
         const bool need_mask = (hi_first - k0 < Cfg::BN - 1) || (lo_last - k0 > 0);
         const bool go = need_mask ? block<true>(n, g, lo_key - k0, hi_key - k0, cmul) : block<false>(n, g, 0, 0, cmul);
         if (!go) return;
+      }
+      if (with_keys < blocks.count) {
+        if (!block_without_keys(with_keys, g)) return;
+        ++g;
       }
       // Epilogue; the issuer is already computing the next tile's S meanwhile.  The next tile's first P V (which overwrites O) is
       // issued only after this warp has delivered that tile's first P, i.e. after the loads below have completed.
@@ -373,8 +409,9 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
       }
       break;
     }
-    const TileInfo t = decode_item(item, p, sp, Cfg::BN);
-    const int nb = t.hi - t.lo;
+    const TileInfo t = decode_item(item, p, sp, Cfg::V_KEYS);
+    const SplitBlocks blocks(t);
+    const int nb = blocks.count;
     if (k > 0) ok = c.wait(Cfg::BAR_Q_FREE, k - 1, WAIT_Q_FREE);
     if (!ok) break;
     mbar_expect_tx(&c.bars[Cfg::BAR_Q_FULL], Cfg::Q_TILE_BYTES);
@@ -385,6 +422,7 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
     auto load = [&](bool is_v, int n) {
 #pragma unroll
       for (int part = 0; part < Cfg::PARTS; ++part) {
+        if (is_v && part > 0 && blocks.half_last && n == nb - 1) return;
         const int slot = ring_i % SL, use = ring_i / SL;
         if (!ok || (use > 0 && !c.wait(Cfg::BAR_EMPTY + slot, use - 1, WAIT_K_EMPTY))) {
           ok = false;
@@ -393,7 +431,7 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
         uint64_t* full = &c.bars[Cfg::BAR_FULL + slot];
         uint8_t* dst = ring + slot * Cfg::STAGE_BYTES;
         mbar_expect_tx(full, Cfg::STAGE_BYTES);
-        const int key0 = (t.lo + n) * Cfg::BN;
+        const int key0 = t.lo * Cfg::V_KEYS + n * Cfg::BN;
         if (is_v) {
 #pragma unroll
           for (int ks = 0; ks < Cfg::KSUB; ++ks)
@@ -436,7 +474,6 @@ template <bool BF16>
 __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams& p, const SchedParams& sp, int lane) {
   using Cfg = SplitCfg;
   constexpr int SL = Cfg::SLOTS, D = Cfg::D, BN = Cfg::BN, BM = Cfg::BM, SB = Cfg::SB, PARTS = Cfg::PARTS;
-  constexpr uint32_t IDESC_S = make_idesc(BF16, BM, BN, false, false);
   constexpr uint32_t IDESC_PV = make_idesc(BF16, BM, D, false, true);
   // descriptor halves: the upper word is constant, the lower word is (address >> 4) plus a compile-time step
   const uint32_t desc_hi = smem_desc_hi(1024);
@@ -449,7 +486,10 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
   int ring_i = 0, g0 = 0;
   bool ok = true;
   auto wait_full = [&](int i) { return c.wait(Cfg::BAR_FULL + i % SL, i / SL, WAIT_K_FULL); };
-  auto issue_s = [&](int gb, bool last_of_tile) {
+  using Whole = std::integral_constant<int, PARTS>;
+  using Half = std::integral_constant<int, 1>;
+  auto issue_s = [&](auto parts_tag, int gb, bool last_of_tile) {
+    constexpr uint32_t IDESC_S = make_idesc(BF16, BM, Cfg::V_KEYS * decltype(parts_tag)::value, false, false);
     const uint32_t s_tmem = c.tmem_base + (gb % SB) * BN;
 #pragma unroll
     for (int part = 0; part < PARTS; ++part) {
@@ -471,10 +511,11 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
       if (part == PARTS - 1 && last_of_tile) umma_commit_if(elected, bars + 8 * Cfg::BAR_Q_FREE);   // no later MMA reads this Q
     }
   };
-  auto issue_pv = [&](int gb, bool first_of_tile) {
+  auto issue_pv = [&](auto parts_tag, int gb, bool first_of_tile) {
+    constexpr int parts = decltype(parts_tag)::value;
     const uint32_t p_tmem = c.tmem_base + (gb % SB) * BN;
 #pragma unroll
-    for (int part = 0; part < PARTS; ++part) {   // part = half: keys [64 part, 64 part + 64), P in columns [64 part, 64 part + 32)
+    for (int part = 0; part < parts; ++part) {   // part = half: keys [64 part, 64 part + 64), P in columns [64 part, 64 part + 32)
       const int slot = (ring_i + part) % SL;
       const uint32_t b0 = v_lo + (uint32_t)(slot * (Cfg::STAGE_BYTES >> 4));
 #pragma unroll
@@ -488,29 +529,36 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
     // one phase of a barrier is outstanding
     umma_commit_if(elected, bars + 8 * (Cfg::BAR_O_FULL + (gb & 1)));
   };
+  // P V of one block.  V first: it landed long ago, and nothing but the wait for P should stand before the products.
+  auto step_pv = [&](auto parts_tag, int gb, bool first_of_tile) {
+    constexpr int parts = decltype(parts_tag)::value;
+#pragma unroll
+    for (int part = 0; part < parts; ++part)
+      if (ok) ok = wait_full(ring_i + part);
+    if (ok) ok = c.wait(Cfg::BAR_P_FULL + gb % SB, gb / SB, WAIT_P_FULL);
+    if (!ok) return;
+    tc_fence_after();
+    issue_pv(parts_tag, gb, first_of_tile);
+    ring_i += parts;
+  };
   for (int k = 0; ok; ++k) {
     if (!c.wait_warp(Cfg::BAR_SCHED + (k & 1), k >> 1, WAIT_SCHED)) break;
     const int item = c.sched[k & 1];
     __syncwarp();
     if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_SCHED_FREE + (k & 1)]);
     if (item < 0) break;
-    const TileInfo t = decode_item(item, p, sp, BN);
-    const int nb = t.hi - t.lo;
+    const TileInfo t = decode_item(item, p, sp, Cfg::V_KEYS);
+    const SplitBlocks blocks(t);
+    const int nb = blocks.count, whole = nb - (blocks.half_last ? 1 : 0);
     ok = c.wait(Cfg::BAR_Q_FULL, k, WAIT_Q_FULL);
-    for (int n = 0; n < SB && n < nb && ok; ++n) issue_s(g0 + n, n == nb - 1);
-    for (int n = 0; n < nb && ok; ++n) {
-      const int gb = g0 + n;
-      // V first: it landed long ago, and nothing but the wait for P should stand before the P V products
-#pragma unroll
-      for (int part = 0; part < PARTS; ++part)
-        if (ok) ok = wait_full(ring_i + part);
-      if (ok) ok = c.wait(Cfg::BAR_P_FULL + gb % SB, gb / SB, WAIT_P_FULL);
-      if (!ok) break;
-      tc_fence_after();
-      issue_pv(gb, n == 0);
-      ring_i += PARTS;
-      if (n + SB < nb) issue_s(gb + SB, n + SB == nb - 1);
+    for (int n = 0; n < SB && n < whole && ok; ++n) issue_s(Whole{}, g0 + n, n == nb - 1);
+    if (whole < nb && whole < SB && ok) issue_s(Half{}, g0 + whole, true);
+    for (int n = 0; n < whole && ok; ++n) {
+      step_pv(Whole{}, g0 + n, n == 0);
+      if (ok && n + SB < nb) issue_s(Whole{}, g0 + n + SB, n + SB == nb - 1);
     }
+    // A half block by itself, so that the loop has no more to decide (there its S is computed whole, from keys that no row sees).
+    if (whole < nb && ok) step_pv(Half{}, g0 + whole, whole == 0);
     ok = __all_sync(0xffffffffu, ok);
     g0 += nb;
   }

@@ -51,3 +51,18 @@ def test_more_tiles_than_sms(cuda_device):
   got = [att.attn_fwd(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device)) for _ in range(2)]
   assert torch.equal(got[0], got[1])
   torch.testing.assert_close(got[0].float().cpu(), ref, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("q_len,extra", [(17, 0), (40, 24), (64, 1), (64, 128), (150, 42), (192, 0), (193, 0), (320, 0), (65, 256)])
+@pytest.mark.parametrize("softcap", [0.0, 30.0])
+def test_half_blocks(cuda_device, q_len, extra, softcap):
+  # a tile's last block has 64 keys (in the first, second or a later place) or, one key further, 128
+  q, k, v = _qkv(2, q_len, q_len + extra, 2, 1, torch.float16, q_len + extra)
+  _check(q, k, v, cuda_device, softcap=softcap)
+
+
+def test_a_half_block_can_move_the_maximum(cuda_device):
+  # the last 64 keys are the largest: the warpgroup that has none of them rescales its half of the output all the same
+  q, k, v = _qkv(1, 64, 320, 2, 2, torch.bfloat16, 3)
+  k[:, 256:] *= 6.0
+  _check(q, k, v, cuda_device)
