@@ -1,6 +1,7 @@
 """Helper of test_gpu_persistent_vs_one_tile.py: runs seeded random attention problems and prints one SHA-1 per
 problem (output + log-sum-exp bytes) as JSON.  Run as a child process so that the kernel variant -- chosen once
-per process from the environment -- can differ between two runs."""
+per process from the environment -- can differ between two runs.  At head_dim 256 both runs take the same kernel, so there the results
+are also compared with the oracle."""
 import hashlib
 import json
 import os
@@ -11,6 +12,7 @@ sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 import torch  # noqa: E402
 
 from deepgengraph_b200 import attention as att  # noqa: E402
+from oracle import reference_math as rm  # noqa: E402
 
 
 def cases(n, seed=1234):
@@ -45,6 +47,10 @@ def main(n):
       h = hashlib.sha1(out.cpu().view(torch.int16).numpy().tobytes() + lse.cpu().numpy().tobytes()).hexdigest()
       assert first is None or first == h, f"rerun differs for problem {ci}"
       first = h
+    if D == 256:
+      ref = rm.attention_ref(q, k, v, causal=True, window=window, softcap=softcap, want=("out", "lse2"))
+      torch.testing.assert_close(out.float(), ref["out"], rtol=2e-2, atol=2e-2, msg=lambda m: f"problem {ci}: {m}")
+      torch.testing.assert_close(lse, ref["lse2"], rtol=1e-3, atol=1e-3, msg=lambda m: f"problem {ci}: {m}")
     hashes.append(first)
   print("HASHES " + json.dumps(hashes))
 

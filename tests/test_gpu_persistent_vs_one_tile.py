@@ -1,6 +1,7 @@
 """The persistent attention kernel (CTAs walk many query tiles, barrier phases and rings carried across tiles,
 dynamic tile order) must produce the bits of the one-tile-per-CTA kernel (same per-tile arithmetic, static
-order) on random shapes: ragged lengths, grouped heads, windows, soft-cap, both head dims, both dtypes."""
+order) on random shapes: ragged lengths, grouped heads, windows, soft-cap, both head dims, both dtypes.  At head_dim 128 these are two
+kernels; at head_dim 256 the switch changes only the launch scheme of one, whose results _attn_hashes.py compares with the oracle."""
 import json
 import os
 import subprocess

@@ -28,7 +28,7 @@ KERNELS = dict(_kernels())
 
 
 def test_the_kernels_are_found():
-  assert {"attn_fwd_kernel", "attn_fwd_persist_kernel", "attn_decode_kernel", "attn_sweep_kernel", "kv_evict_regs_kernel",
+  assert {"attn_fwd_kernel", "attn_fwd_persist_kernel", "attn_fwd_split_kernel", "attn_decode_kernel", "attn_sweep_kernel", "kv_evict_regs_kernel",
           "rms_norm_block_kernel", "rotary_online_kernel"} | PLAIN_LAUNCHES <= set(KERNELS)
 
 
