@@ -1,4 +1,4 @@
-// Fused attention forward for sm_100a:  out = softmax(mask(softcap(q k^T * scale))) v.
+// Fused attention forward for sm_100a:  out = softmax(mask(softcap(q k^T * scale))) v, at head_dim 128 (256: attn_fwd_split.cuh).
 //
 // One CTA owns NQ query tiles of 128 rows of one (batch, head) and walks the key/value blocks that the
 // causal / sliding-window mask leaves visible.  Roles (warp-specialised):
@@ -32,18 +32,18 @@ struct FwdParams {
 
 // SB = S buffers per query tile in TMEM.  With SB = 2 the S tile of block j+1 is computed while the softmax of
 // block j runs, so a tile's softmax never waits for the tensor pipe in steady state.
-template <int D_, int BN_, int NQ_, int SB_>
+template <int BN_, int NQ_, int SB_>
 struct FwdCfg {
-  static constexpr int D = D_, BN = BN_, NQ = NQ_, SB = SB_;
+  static constexpr int D = 128, BN = BN_, NQ = NQ_, SB = SB_;
   static constexpr int BM = 128;
   static constexpr int KSUB = D / 64;                 // 64-element (128-byte) column blocks of a row
   static constexpr int Q_TILE_BYTES = BM * D * 2;
   static constexpr int KV_STAGE_BYTES = BN * D * 2;
   // one ring for K and V blocks (K(j) is item 2n, V(j) item 2n+1): as many slots as fit beside Q, at most 8
-  // head_dim 128 with one query tile per CTA: TMEM (256 of 512 columns) and shared memory are sized so that TWO
+  // With one query tile per CTA: TMEM (256 of 512 columns) and shared memory are sized so that TWO
   // CTAs share an SM.  The two are independent (own producer, own issuer, own K/V ring), so one CTA's prologue,
   // epilogue and softmax phases overlap the other's MMAs without any coupling between them.
-  static constexpr int CTAS_PER_SM = (NQ == 1 && D == 128) ? 2 : 1;
+  static constexpr int CTAS_PER_SM = NQ == 1 ? 2 : 1;
   static constexpr int SMEM_BUDGET = 232448 / CTAS_PER_SM - (CTAS_PER_SM > 1 ? 1024 : 0);   // 1 KB/CTA is reserved by the driver
   static constexpr int SLOTS_FIT = (SMEM_BUDGET - 2048 - NQ * Q_TILE_BYTES) / KV_STAGE_BYTES;
   static constexpr int SLOTS = SLOTS_FIT > 8 ? 8 : SLOTS_FIT;
@@ -325,33 +325,18 @@ constexpr int kPolyOf8 = B200_POLY_OF_8;
 // Exp-phase turn-taking between the two query tiles of a CTA (tuning switch).
 constexpr bool kTakeTurns = B200_TAKE_TURNS != 0;
 
-// One block of the online softmax for one row (thread).  MASK selects the edge-block variant.
-template <class Cfg, bool BF16, bool SOFTCAP, bool MASK>
-__device__ __forceinline__ bool fwd_softmax_block(const FwdCtx<Cfg, BF16>& c, const FwdParams& p, uint32_t s_addr,
-                                                  uint32_t o_addr, uint64_t* o_full, uint64_t* p_full, int n,
-                                                  int g, int lo_c, int hi_c, float cmul, float& m, float& l,
-                                                  uint64_t* turn_wait, int turn_parity, uint64_t* turn_pass,
-                                                  uint64_t* next_s_full = nullptr, int next_parity = 0,
-                                                  bool* next_ready = nullptr) {
-  constexpr int D = Cfg::D, BN = Cfg::BN;
-  const int lane = threadIdx.x & 31;
-  // (tuning builds stamp the first 64 blocks a CTA walks)
-  [[maybe_unused]] const int tl_base = (((int)(threadIdx.x >> 7)) * 64 + (g & 63)) * 8;
-  [[maybe_unused]] const bool tl_on = (threadIdx.x & 127) == 0 && g < 64;
-  if (tl_on) B200_TL(tl_base + 0);
-  uint32_t sr[BN / 32][32];
-#pragma unroll
-  for (int ch = 0; ch < BN / 32; ++ch) tmem_ld32(s_addr + ch * 32, sr[ch]);
-  tmem_ld_wait();
-  if (tl_on) B200_TL(tl_base + 1);
+// ---- one row (thread): its logits of a block in registers, COLS columns, masked outside [lo_c, hi_c] if MASK ----
 
-  // Row maximum of the block.  With a soft-cap the capped logit is a monotone function of the raw one, so the
-  // maximum is taken over the RAW values (no special-function work in this pass) and capped once; the pass also
-  // finds the largest |raw| so that the warp can vote for the polynomial-only exponential pass below.
+// Maximum in base-2 units, -inf if every column is masked.  With a soft-cap the capped logit is a monotone function of the raw one, so
+// the maximum is taken over the RAW values (no special-function work in this pass) and capped once; the pass also finds the largest
+// |raw| so that the warp can vote for the polynomial-only exponential pass.
+template <bool SOFTCAP, bool MASK, int COLS>
+__device__ __forceinline__ float row_maximum(uint32_t (&sr)[COLS / 32][32], int lo_c, int hi_c, const FwdParams& p, float cmul,
+                                             bool& cap_poly_only) {
   float mx0 = -INFINITY, mx1 = -INFINITY;
   [[maybe_unused]] float ab0 = 0.f, ab1 = 0.f;
 #pragma unroll
-  for (int ch = 0; ch < BN / 32; ++ch) {
+  for (int ch = 0; ch < COLS / 32; ++ch) {
 #pragma unroll
     for (int i = 0; i < 32; i += 4) {
       float v[4];
@@ -380,14 +365,151 @@ __device__ __forceinline__ bool fwd_softmax_block(const FwdCtx<Cfg, BF16>& c, co
       }
     }
   }
-  float m_blk = fmaxf(mx0, mx1);   // -inf when the whole row is masked inside this block
-  [[maybe_unused]] bool cap_poly_only = false;
+  const float mx = fmaxf(mx0, mx1);
   if constexpr (SOFTCAP) {
-    m_blk = m_blk == -INFINITY ? -INFINITY : softcap_tanh(m_blk * p.cap_in) * cmul;   // cap_out is folded into cmul
     cap_poly_only = !__any_sync(0xffffffffu, fmaxf(ab0, ab1) * p.cap_in > kCapPolyMax);
+    return mx == -INFINITY ? -INFINITY : softcap_tanh(mx * p.cap_in) * cmul;   // cap_out is folded into cmul
   } else {
-    m_blk *= cmul;
+    return mx * cmul;
   }
+}
+
+// P = exp2(x - m), packed to the 16-bit input type, written to TMEM from column p_addr on; returns the sum in fp32.
+// POLY_ONLY: every |raw / cap| of the warp's columns is <= 1.
+template <bool BF16, bool SOFTCAP, bool MASK, int COLS, bool POLY_ONLY>
+__device__ __forceinline__ float row_exponentials_pass(const uint32_t (&sr)[COLS / 32][32], uint32_t p_addr, int lo_c, int hi_c,
+                                                       const FwdParams& p, float cmul, float m) {
+  const float2 c2 = make_float2(cmul, cmul), nm2 = make_float2(-m, -m);
+  float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int ch = 0; ch < COLS / 32; ++ch) {
+    uint32_t pk[16];
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      // x = logit - m in base-2 units for four columns
+      float2 x0, x1;
+      const float2 s0 = make_float2(__uint_as_float(sr[ch][i + 0]), __uint_as_float(sr[ch][i + 1]));
+      const float2 s1 = make_float2(__uint_as_float(sr[ch][i + 2]), __uint_as_float(sr[ch][i + 3]));
+      if constexpr (SOFTCAP) {
+        const float2 a2 = make_float2(p.cap_in, p.cap_in);
+        const float2 y0 = fmul2(s0, a2), y1 = fmul2(s1, a2);
+        if constexpr (POLY_ONLY) {
+          x0 = ffma2(y0, softcap_r2(y0, cmul), nm2);
+          x1 = ffma2(y1, softcap_r2(y1, cmul), nm2);
+        } else {
+          x0 = ffma2(make_float2(softcap_tanh(y0.x), softcap_tanh(y0.y)), c2, nm2);
+          x1 = ffma2(make_float2(softcap_tanh(y1.x), softcap_tanh(y1.y)), c2, nm2);
+        }
+        if constexpr (MASK) {
+          const int col = ch * 32 + i;
+          if (col + 0 > hi_c || col + 0 < lo_c) x0.x = -INFINITY;
+          if (col + 1 > hi_c || col + 1 < lo_c) x0.y = -INFINITY;
+          if (col + 2 > hi_c || col + 2 < lo_c) x1.x = -INFINITY;
+          if (col + 3 > hi_c || col + 3 < lo_c) x1.y = -INFINITY;
+        }
+      } else {
+        x0 = ffma2(s0, c2, nm2);
+        x1 = ffma2(s1, c2, nm2);
+      }
+      // masked blocks hold -inf entries and stay on the special-function unit; elsewhere a fixed, interleaved
+      // subset of the column groups goes through the polynomial
+      if (!MASK && (((i / 4) * kPolyOf8) % 8) < kPolyOf8) {
+        x0 = exp2_poly2(x0);
+        x1 = exp2_poly2(x1);
+      } else {
+        x0.x = ex2_approx(x0.x);
+        x0.y = ex2_approx(x0.y);
+        x1.x = ex2_approx(x1.x);
+        x1.y = ex2_approx(x1.y);
+      }
+      acc0 = fadd2(acc0, x0);
+      acc1 = fadd2(acc1, x1);
+      pk[i / 2] = pack2<BF16>(x0.x, x0.y);
+      pk[i / 2 + 1] = pack2<BF16>(x1.x, x1.y);
+    }
+    tmem_st16(p_addr + ch * 16, pk);
+  }
+  return (acc0.x + acc0.y) + (acc1.x + acc1.y);
+}
+template <bool BF16, bool SOFTCAP, bool MASK, int COLS>
+__device__ __forceinline__ float row_exponentials(const uint32_t (&sr)[COLS / 32][32], uint32_t p_addr, int lo_c, int hi_c,
+                                                  const FwdParams& p, float cmul, float m, bool cap_poly_only) {
+  if constexpr (SOFTCAP) {
+    if (cap_poly_only) return row_exponentials_pass<BF16, SOFTCAP, MASK, COLS, true>(sr, p_addr, lo_c, hi_c, p, cmul, m);
+  }
+  return row_exponentials_pass<BF16, SOFTCAP, MASK, COLS, false>(sr, p_addr, lo_c, hi_c, p, cmul, m);
+}
+
+// O *= alpha for DIMS columns of the row's accumulator.
+template <int DIMS>
+__device__ __forceinline__ void row_rescale(uint32_t o_addr, float alpha) {
+  const float2 a2 = make_float2(alpha, alpha);
+#pragma unroll
+  for (int ch = 0; ch < DIMS / 16; ++ch) {
+    uint32_t o[16];
+    tmem_ld16(o_addr + ch * 16, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+      const float2 r = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), a2);
+      o[i] = __float_as_uint(r.x);
+      o[i + 1] = __float_as_uint(r.y);
+    }
+    tmem_st16(o_addr + ch * 16, o);
+  }
+}
+
+// O / l -> 16-bit -> global for DIMS columns of the row, from element `first` of `out` on (in_range: the row exists).
+template <bool BF16, int DIMS>
+__device__ __forceinline__ void row_store(uint32_t o_addr, void* out, int64_t first, float l, bool in_range) {
+  const float inv_l = 1.0f / l;
+  const bool wide_stores = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+  uint4* out_row = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(out) + first);
+#pragma unroll
+  for (int ch = 0; ch < DIMS / 32; ++ch) {
+    uint32_t o[32];
+    tmem_ld32(o_addr + ch * 32, o);
+    tmem_ld_wait();
+    if (in_range) {
+      // every lane writes its own row (rows are heads * D elements apart), so a store instruction costs one
+      // memory transaction per lane whatever its width: 32-byte stores halve the count
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        uint32_t w[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          w[e] = pack2<BF16>(__uint_as_float(o[v * 16 + 2 * e]) * inv_l, __uint_as_float(o[v * 16 + 2 * e + 1]) * inv_l);
+        if (wide_stores) {
+          st_global_v8(out_row + ch * 4 + v * 2, w);
+        } else {
+          out_row[ch * 4 + v * 2] = make_uint4(w[0], w[1], w[2], w[3]);
+          out_row[ch * 4 + v * 2 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
+        }
+      }
+    }
+  }
+}
+
+// One block of the online softmax for one row (thread).  MASK selects the edge-block variant.
+template <class Cfg, bool BF16, bool SOFTCAP, bool MASK>
+__device__ __forceinline__ bool fwd_softmax_block(const FwdCtx<Cfg, BF16>& c, const FwdParams& p, uint32_t s_addr,
+                                                  uint32_t o_addr, uint64_t* o_full, uint64_t* p_full, int n,
+                                                  int g, int lo_c, int hi_c, float cmul, float& m, float& l,
+                                                  uint64_t* turn_wait, int turn_parity, uint64_t* turn_pass) {
+  constexpr int D = Cfg::D, BN = Cfg::BN;
+  const int lane = threadIdx.x & 31;
+  // (tuning builds stamp the first 64 blocks a CTA walks)
+  [[maybe_unused]] const int tl_base = (((int)(threadIdx.x >> 7)) * 64 + (g & 63)) * 8;
+  [[maybe_unused]] const bool tl_on = (threadIdx.x & 127) == 0 && g < 64;
+  if (tl_on) B200_TL(tl_base + 0);
+  uint32_t sr[BN / 32][32];
+#pragma unroll
+  for (int ch = 0; ch < BN / 32; ++ch) tmem_ld32(s_addr + ch * 32, sr[ch]);
+  tmem_ld_wait();
+  if (tl_on) B200_TL(tl_base + 1);
+
+  bool cap_poly_only = false;
+  const float m_blk = row_maximum<SOFTCAP, MASK, BN>(sr, lo_c, hi_c, p, cmul, cap_poly_only);
   if (tl_on) B200_TL(tl_base + 2);
   float alpha = 1.0f;
   bool rescale = false;
@@ -408,93 +530,14 @@ __device__ __forceinline__ bool fwd_softmax_block(const FwdCtx<Cfg, BF16>& c, co
     // (g counts the P V products of this CTA: equal to n unless the CTA walks several tiles)
     if (!mbar_wait(o_full + ((g - 1) & 1), ((g - 1) >> 1) & 1, c.abort_flag, WAIT_O_FULL)) return false;
     tc_fence_after();
-    const float2 a2 = make_float2(alpha, alpha);
-#pragma unroll
-    for (int ch = 0; ch < D / 16; ++ch) {
-      uint32_t o[16];
-      tmem_ld16(o_addr + ch * 16, o);
-      tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 16; i += 2) {
-        const float2 r = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), a2);
-        o[i] = __float_as_uint(r.x);
-        o[i + 1] = __float_as_uint(r.y);
-      }
-      tmem_st16(o_addr + ch * 16, o);
-    }
+    row_rescale<D>(o_addr, alpha);
   }
   // The exponentials saturate the special-function unit, which the warp of the other query tile on this SM
   // sub-partition shares: the two take turns (see fwd_softmax), so that one tile's exponentials overlap the
   // other tile's MMAs instead of colliding with its exponentials.
   if (turn_wait != nullptr && !mbar_wait(turn_wait, turn_parity, c.abort_flag, WAIT_TURN)) return false;
-  // Early look at the next block's S barrier: shared-memory latency is ~10x higher while the S = Q K^T MMAs
-  // saturate the shared-memory port, so the probe is issued here and its result consumed after the exponentials.
-  if (next_s_full != nullptr) *next_ready = mbar_test_wait(next_s_full, next_parity);
-  // P = exp2(x - m), packed to the 16-bit input type, written over the first BN/2 columns of S
-  const float2 c2 = make_float2(cmul, cmul), nm2 = make_float2(-m, -m);
-  float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
-  // x = logit - m in base-2 units for four columns; POLY_ONLY: every |raw / cap| of the warp's block is <= 1
-  auto exponents = [&](auto poly_only_tag, int ch, int i, float2& x0, float2& x1) {
-    const float2 s0 = make_float2(__uint_as_float(sr[ch][i + 0]), __uint_as_float(sr[ch][i + 1]));
-    const float2 s1 = make_float2(__uint_as_float(sr[ch][i + 2]), __uint_as_float(sr[ch][i + 3]));
-    if constexpr (SOFTCAP) {
-      const float2 a2 = make_float2(p.cap_in, p.cap_in);
-      const float2 y0 = fmul2(s0, a2), y1 = fmul2(s1, a2);
-      if constexpr (decltype(poly_only_tag)::value) {
-        x0 = ffma2(y0, softcap_r2(y0, cmul), nm2);
-        x1 = ffma2(y1, softcap_r2(y1, cmul), nm2);
-      } else {
-        x0 = ffma2(make_float2(softcap_tanh(y0.x), softcap_tanh(y0.y)), c2, nm2);
-        x1 = ffma2(make_float2(softcap_tanh(y1.x), softcap_tanh(y1.y)), c2, nm2);
-      }
-      if constexpr (MASK) {
-        const int col = ch * 32 + i;
-        if (col + 0 > hi_c || col + 0 < lo_c) x0.x = -INFINITY;
-        if (col + 1 > hi_c || col + 1 < lo_c) x0.y = -INFINITY;
-        if (col + 2 > hi_c || col + 2 < lo_c) x1.x = -INFINITY;
-        if (col + 3 > hi_c || col + 3 < lo_c) x1.y = -INFINITY;
-      }
-    } else {
-      x0 = ffma2(s0, c2, nm2);
-      x1 = ffma2(s1, c2, nm2);
-    }
-  };
-  auto exp_pass = [&](auto poly_only_tag) {
-#pragma unroll
-    for (int ch = 0; ch < BN / 32; ++ch) {
-      uint32_t pk[16];
-#pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        float2 x0, x1;
-        exponents(poly_only_tag, ch, i, x0, x1);
-        // masked blocks hold -inf entries and stay on the special-function unit; elsewhere a fixed, interleaved
-        // subset of the column groups goes through the polynomial
-        if (!MASK && (((i / 4) * kPolyOf8) % 8) < kPolyOf8) {
-          x0 = exp2_poly2(x0);
-          x1 = exp2_poly2(x1);
-        } else {
-          x0.x = ex2_approx(x0.x);
-          x0.y = ex2_approx(x0.y);
-          x1.x = ex2_approx(x1.x);
-          x1.y = ex2_approx(x1.y);
-        }
-        acc0 = fadd2(acc0, x0);
-        acc1 = fadd2(acc1, x1);
-        pk[i / 2] = pack2<BF16>(x0.x, x0.y);
-        pk[i / 2 + 1] = pack2<BF16>(x1.x, x1.y);
-      }
-      tmem_st16(s_addr + ch * 16, pk);
-    }
-  };
-  if constexpr (SOFTCAP) {
-    if (cap_poly_only)
-      exp_pass(std::true_type{});
-    else
-      exp_pass(std::false_type{});
-  } else {
-    exp_pass(std::false_type{});
-  }
-  l += (acc0.x + acc0.y) + (acc1.x + acc1.y);
+  // P over the first BN/2 columns of S
+  l += row_exponentials<BF16, SOFTCAP, MASK, BN>(sr, s_addr, lo_c, hi_c, p, cmul, m, cap_poly_only);
   if (turn_pass != nullptr) {
     __syncwarp();
     if (lane == 0) mbar_arrive(turn_pass);
@@ -576,44 +619,18 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<Cfg, BF16>& c, const Fw
   if (!mbar_wait(o_full + (last & 1), (last >> 1) & 1, c.abort_flag, WAIT_O_FULL)) return;
   tc_fence_after();
   if ((threadIdx.x & 127) == 0) B200_TL((3 * 64 + 62) * 8 + 3);   // last P V complete
-  const float inv_l = 1.0f / l;
   const bool in_range = row < p.q_len;
-  const bool wide_stores = (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
-  uint4* out_row = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
-                                            (((int64_t)c.b * p.q_len + row) * p.heads + c.h) * (int64_t)D);
-#pragma unroll
-  for (int ch = 0; ch < D / 32; ++ch) {
-    uint32_t o[32];
-    tmem_ld32(o_addr + ch * 32, o);
-    tmem_ld_wait();
-    if (in_range) {
-      // every lane writes its own row (rows are heads * D elements apart), so a store instruction costs one
-      // memory transaction per lane whatever its width: 32-byte stores halve the count
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        uint32_t w[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          w[e] = pack2<BF16>(__uint_as_float(o[v * 16 + 2 * e]) * inv_l, __uint_as_float(o[v * 16 + 2 * e + 1]) * inv_l);
-        if (wide_stores) {
-          st_global_v8(out_row + ch * 4 + v * 2, w);
-        } else {
-          out_row[ch * 4 + v * 2] = make_uint4(w[0], w[1], w[2], w[3]);
-          out_row[ch * 4 + v * 2 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
-        }
-      }
-    }
-  }
+  row_store<BF16, D>(o_addr, p.out, (((int64_t)c.b * p.q_len + row) * p.heads + c.h) * (int64_t)D, l, in_range);
   if ((threadIdx.x & 127) == 0) B200_TL((3 * 64 + 62) * 8 + 4);   // output stored
   if (p.lse != nullptr && in_range) p.lse[((int64_t)c.b * p.heads + c.h) * p.lse_stride + row] = m + log2f(l);
 }
 
 // ----------------------------------- kernel ----------------------------------
-template <int D, int BN, int NQ, int SB, bool BF16, bool SOFTCAP>
-__global__ void __launch_bounds__(FwdCfg<D, BN, NQ, SB>::THREADS, FwdCfg<D, BN, NQ, SB>::CTAS_PER_SM)
+template <int BN, int NQ, int SB, bool BF16, bool SOFTCAP>
+__global__ void __launch_bounds__(FwdCfg<BN, NQ, SB>::THREADS, FwdCfg<BN, NQ, SB>::CTAS_PER_SM)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
-  using Cfg = FwdCfg<D, BN, NQ, SB>;
+  using Cfg = FwdCfg<BN, NQ, SB>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
@@ -716,11 +733,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 }
 
 // --------------------------------- host side ---------------------------------
-template <int D, int BN, int NQ, int SB, bool BF16, bool SOFTCAP>
+template <int BN, int NQ, int SB, bool BF16, bool SOFTCAP>
 int launch_attn_fwd_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                         cudaStream_t stream) {
-  using Cfg = FwdCfg<D, BN, NQ, SB>;
-  auto kern = attn_fwd_kernel<D, BN, NQ, SB, BF16, SOFTCAP>;
+  using Cfg = FwdCfg<BN, NQ, SB>;
+  auto kern = attn_fwd_kernel<BN, NQ, SB, BF16, SOFTCAP>;
   static thread_local int configured_dev = -1;
   int dev = 0;
   B200_CUDA_TRY(cudaGetDevice(&dev));
@@ -735,7 +752,7 @@ int launch_attn_fwd_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
 }
 
 // persistent variant (attn_fwd_persist.cuh)
-template <int D_, bool BF16, bool SOFTCAP>
+template <bool BF16, bool SOFTCAP>
 int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                             cudaStream_t stream);
 
@@ -811,26 +828,19 @@ inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v,
   if ((rc = make_bshd_tensor_map(&tv, v, batch, kv_len, kv_heads, head_dim, bn, bf16, st.v_token, st.v_batch)) != B200_OK)
     return rc;
 
-#define B200_FWD_DISPATCH(D_, BN_, NQ_, SB_)                                                                 \
-  (bf16 ? (cap ? launch_attn_fwd_cfg<D_, BN_, NQ_, SB_, true, true>(tq, tk, tv, p, stream)                   \
-               : launch_attn_fwd_cfg<D_, BN_, NQ_, SB_, true, false>(tq, tk, tv, p, stream))                 \
-        : (cap ? launch_attn_fwd_cfg<D_, BN_, NQ_, SB_, false, true>(tq, tk, tv, p, stream)                  \
-               : launch_attn_fwd_cfg<D_, BN_, NQ_, SB_, false, false>(tq, tk, tv, p, stream)))
   // Default: the persistent kernel, whose CTAs walk query tiles handed out by an atomic counter, two CTAs per SM.  (The other
   // kernel also supports NQ = 2 -- two tiles sharing one K/V stream in a single CTA; two independent CTAs per SM measured 13 %
   // faster at seq 4096.)
-#define B200_PERSIST_DISPATCH(D_)                                                                    \
-  (bf16 ? (cap ? launch_attn_fwd_persist<D_, true, true>(tq, tk, tv, p, stream)                       \
-               : launch_attn_fwd_persist<D_, true, false>(tq, tk, tv, p, stream))                     \
-        : (cap ? launch_attn_fwd_persist<D_, false, true>(tq, tk, tv, p, stream)                      \
-               : launch_attn_fwd_persist<D_, false, false>(tq, tk, tv, p, stream)))
-  if (!one_tile_per_cta && B200_BN128 == 64 && B200_SB128 == 2) return B200_PERSIST_DISPATCH(128);
 #ifdef B200_NQ128
-  return B200_FWD_DISPATCH(128, B200_BN128, B200_NQ128, B200_SB128);
+  constexpr int NQ = B200_NQ128;
 #else
-  return B200_FWD_DISPATCH(128, B200_BN128, 1, B200_SB128);
+  constexpr int NQ = 1;
 #endif
-#undef B200_PERSIST_DISPATCH
+#define B200_FWD_DISPATCH(launch, ...)                                                                          \
+  (bf16 ? (cap ? launch<__VA_ARGS__ true, true>(tq, tk, tv, p, stream) : launch<__VA_ARGS__ true, false>(tq, tk, tv, p, stream))   \
+        : (cap ? launch<__VA_ARGS__ false, true>(tq, tk, tv, p, stream) : launch<__VA_ARGS__ false, false>(tq, tk, tv, p, stream)))
+  if (!one_tile_per_cta && B200_BN128 == 64 && B200_SB128 == 2) return B200_FWD_DISPATCH(launch_attn_fwd_persist, );
+  return B200_FWD_DISPATCH(launch_attn_fwd_cfg, B200_BN128, NQ, B200_SB128, );
 #undef B200_FWD_DISPATCH
 }
 

@@ -1,6 +1,6 @@
 // Persistent variant of the attention forward kernel at head_dim 128, two CTAs per SM (head_dim 256: attn_fwd_split.cuh).
 //
-// Same tiling, TMEM plan and warp roles as attn_fwd_kernel<D, 64, 1, 2> (one 128-row query tile at a time, two
+// Same tiling, TMEM plan and warp roles as attn_fwd_kernel<64, 1, 2> (one 128-row query tile at a time, two
 // S buffers), but the grid is CTAS_PER_SM x #SM CTAs that each walk a sequence of query tiles:
 //   * tiles are handed out by an atomic counter, (batch, head) units in L2-sized groups and tile-major,
 //     heaviest tile first inside a group (see decode_item), so the SMs drain evenly;
@@ -55,9 +55,8 @@ __device__ __forceinline__ TileInfo decode_item(int item, const FwdParams& p, co
   return t;
 }
 
-template <int D_>
-struct PersistCfg : FwdCfg<D_, 64, 1, 2> {
-  using Base = FwdCfg<D_, 64, 1, 2>;
+struct PersistCfg : FwdCfg<64, 1, 2> {
+  using Base = FwdCfg<64, 1, 2>;
   static constexpr int SOFTMAX_WARPS = 4;
   static constexpr int THREADS_P = (SOFTMAX_WARPS + 2) * 32;
   static constexpr int BAR_SCHED = Base::NUM_BARS;        // [2] tile descriptor slot k % 2 published
@@ -68,11 +67,11 @@ struct PersistCfg : FwdCfg<D_, 64, 1, 2> {
   static_assert(SMEM_BYTES_P <= Base::SMEM_BUDGET, "shared memory budget exceeded");
 };
 
-template <int D_, bool BF16, bool SOFTCAP>
-__global__ void __launch_bounds__(PersistCfg<D_>::THREADS_P, PersistCfg<D_>::CTAS_PER_SM)
+template <bool BF16, bool SOFTCAP>
+__global__ void __launch_bounds__(PersistCfg::THREADS_P, PersistCfg::CTAS_PER_SM)
 attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                         const __grid_constant__ CUtensorMap tm_v, const FwdParams p, const SchedParams sp) {
-  using Cfg = PersistCfg<D_>;
+  using Cfg = PersistCfg;
   constexpr int SL = Cfg::SLOTS, D = Cfg::D, BN = Cfg::BN, BM = Cfg::BM, SB = Cfg::SB;
   constexpr int PRODUCER_WARP = Cfg::SOFTMAX_WARPS;
   extern __shared__ uint8_t smem_raw[];
@@ -179,35 +178,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       if (!mbar_wait(o_full + (last & 1), (last >> 1) & 1, c.abort_flag, WAIT_O_FULL)) break;
       tc_fence_after();
       if (threadIdx.x == 0 && k < 8) B200_TL((3 * 64 + 48 + k) * 8 + 1);
-      const float inv_l = 1.0f / l;
       const bool in_range = row < p.q_len;
-      const bool wide_stores = (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
-      uint4* out_row = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
-                                                (((int64_t)t.b * p.q_len + row) * p.heads + t.h) * (int64_t)D);
-#pragma unroll
-      for (int ch = 0; ch < D / 32; ++ch) {
-        uint32_t o[32];
-        tmem_ld32(o_addr + ch * 32, o);
-        tmem_ld_wait();
-        if (threadIdx.x == 0 && k < 8 && ch < 4) B200_TL((3 * 64 + 48 + k) * 8 + 3 + ch);   // chunk ch loaded
-        if (in_range) {
-          // every lane writes its own row (rows are heads * D elements apart), so a store instruction costs one
-          // memory transaction per lane whatever its width: 32-byte stores halve the count
-#pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            uint32_t w[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              w[e] = pack2<BF16>(__uint_as_float(o[v * 16 + 2 * e]) * inv_l, __uint_as_float(o[v * 16 + 2 * e + 1]) * inv_l);
-            if (wide_stores) {
-              st_global_v8(out_row + ch * 4 + v * 2, w);
-            } else {
-              out_row[ch * 4 + v * 2] = make_uint4(w[0], w[1], w[2], w[3]);
-              out_row[ch * 4 + v * 2 + 1] = make_uint4(w[4], w[5], w[6], w[7]);
-            }
-          }
-        }
-      }
+      row_store<BF16, D>(o_addr, p.out, (((int64_t)t.b * p.q_len + row) * p.heads + t.h) * (int64_t)D, l, in_range);
       if (p.lse != nullptr && in_range) p.lse[((int64_t)t.b * p.heads + t.h) * p.lse_stride + row] = m + log2f(l);
       if (threadIdx.x == 0 && k < 8) B200_TL((3 * 64 + 48 + k) * 8 + 2);
       blocks_done = g;
@@ -480,11 +452,11 @@ inline int sched_params(SchedParams* sp, const FwdParams& p, int head_dim, bool 
   return B200_OK;
 }
 
-template <int D_, bool BF16, bool SOFTCAP>
+template <bool BF16, bool SOFTCAP>
 int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
                             cudaStream_t stream) {
-  using Cfg = PersistCfg<D_>;
-  auto kern = attn_fwd_persist_kernel<D_, BF16, SOFTCAP>;
+  using Cfg = PersistCfg;
+  auto kern = attn_fwd_persist_kernel<BF16, SOFTCAP>;
   static thread_local int configured_dev = -1;
   int dev = 0;
   B200_CUDA_TRY(cudaGetDevice(&dev));
@@ -493,7 +465,7 @@ int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const 
     configured_dev = dev;
   }
   SchedParams sp;
-  const int rc = sched_params(&sp, p, D_, true);
+  const int rc = sched_params(&sp, p, Cfg::D, true);
   if (rc != B200_OK) return rc;
   const int grid = std::min(sp.total_items, Cfg::CTAS_PER_SM * sm_count());
   B200_CUDA_TRY(launch_kernel(kern, grid, Cfg::THREADS_P, Cfg::SMEM_BYTES_P, stream, 1, tq, tk, tv, p, sp));

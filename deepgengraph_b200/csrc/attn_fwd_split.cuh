@@ -146,20 +146,7 @@ struct SplitSoftmax {
             return false;
           }
           tc_fence_after();
-          const float2 a2 = make_float2(alpha, alpha);
-#pragma unroll
-          for (int ch = 0; ch < D / 2 / 16; ++ch) {
-            uint32_t o[16];
-            tmem_ld16(o_addr + ch * 16, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-              const float2 r = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), a2);
-              o[i] = __float_as_uint(r.x);
-              o[i + 1] = __float_as_uint(r.y);
-            }
-            tmem_st16(o_addr + ch * 16, o);
-          }
+          row_rescale<D / 2>(o_addr, alpha);
         }
       }
     }
@@ -194,108 +181,11 @@ struct SplitSoftmax {
     for (int ch = 0; ch < COLS / 32; ++ch) tmem_ld32(s_addr + ch * 32, sr[ch]);
     tmem_ld_wait();
 
-    // Maximum of the thread's 64 logits.  With a soft-cap the capped logit is a monotone function of the raw one, so the maximum
-    // is taken over the RAW values (no special-function work in this pass) and capped once; the pass also finds the largest
-    // |raw| so that the warp can vote for the polynomial-only exponential pass below.
-    float mx0 = -INFINITY, mx1 = -INFINITY;
-    [[maybe_unused]] float ab0 = 0.f, ab1 = 0.f;
-#pragma unroll
-    for (int ch = 0; ch < COLS / 32; ++ch) {
-#pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        float v[4];
-        [[maybe_unused]] float va[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          float s = __uint_as_float(sr[ch][i + u]);
-          [[maybe_unused]] float sa = s;
-          if constexpr (MASK) {
-            const int col = ch * 32 + i + u;
-            if (col > hi_c || col < lo_c) {
-              s = -INFINITY;
-              sa = 0.f;
-            }
-            // (with a soft-cap the registers keep the raw value: the exponential pass masks by column again)
-            if constexpr (!SOFTCAP) sr[ch][i + u] = __float_as_uint(s);
-          }
-          v[u] = s;
-          if constexpr (SOFTCAP) va[u] = sa;
-        }
-        mx0 = fmax3(mx0, v[0], v[1]);
-        mx1 = fmax3(mx1, v[2], v[3]);
-        if constexpr (SOFTCAP) {
-          ab0 = fmax3_abs(ab0, va[0], va[1]);
-          ab1 = fmax3_abs(ab1, va[2], va[3]);
-        }
-      }
-    }
-    float m_blk = fmaxf(mx0, mx1);   // -inf when all 64 are masked
-    [[maybe_unused]] bool cap_poly_only = false;
-    if constexpr (SOFTCAP) {
-      m_blk = m_blk == -INFINITY ? -INFINITY : softcap_tanh(m_blk * p.cap_in) * cmul;   // cap_out is folded into cmul
-      cap_poly_only = !__any_sync(0xffffffffu, fmaxf(ab0, ab1) * p.cap_in > kCapPolyMax);
-    } else {
-      m_blk *= cmul;
-    }
+    bool cap_poly_only = false;
+    const float m_blk = row_maximum<SOFTCAP, MASK, COLS>(sr, lo_c, hi_c, p, cmul, cap_poly_only);
     if (!agree(n, g, ok, m_blk)) return false;
-    // P = exp2(x - m), packed to the 16-bit input type, written over the first half of the thread's own S columns
-    const float2 c2 = make_float2(cmul, cmul), nm2 = make_float2(-m, -m);
-    float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
-    // x = logit - m in base-2 units for four columns; POLY_ONLY: every |raw / cap| of the warp's columns is <= 1
-    auto exponents = [&](auto poly_only_tag, int ch, int i, float2& x0, float2& x1) {
-      const float2 s0 = make_float2(__uint_as_float(sr[ch][i + 0]), __uint_as_float(sr[ch][i + 1]));
-      const float2 s1 = make_float2(__uint_as_float(sr[ch][i + 2]), __uint_as_float(sr[ch][i + 3]));
-      if constexpr (SOFTCAP) {
-        const float2 a2 = make_float2(p.cap_in, p.cap_in);
-        const float2 y0 = fmul2(s0, a2), y1 = fmul2(s1, a2);
-        if constexpr (decltype(poly_only_tag)::value) {
-          x0 = ffma2(y0, softcap_r2(y0, cmul), nm2);
-          x1 = ffma2(y1, softcap_r2(y1, cmul), nm2);
-        } else {
-          x0 = ffma2(make_float2(softcap_tanh(y0.x), softcap_tanh(y0.y)), c2, nm2);
-          x1 = ffma2(make_float2(softcap_tanh(y1.x), softcap_tanh(y1.y)), c2, nm2);
-        }
-        if constexpr (MASK) {
-          const int col = ch * 32 + i;
-          if (col + 0 > hi_c || col + 0 < lo_c) x0.x = -INFINITY;
-          if (col + 1 > hi_c || col + 1 < lo_c) x0.y = -INFINITY;
-          if (col + 2 > hi_c || col + 2 < lo_c) x1.x = -INFINITY;
-          if (col + 3 > hi_c || col + 3 < lo_c) x1.y = -INFINITY;
-        }
-      } else {
-        x0 = ffma2(s0, c2, nm2);
-        x1 = ffma2(s1, c2, nm2);
-      }
-    };
-    auto exp_pass = [&](auto poly_only_tag) {
-#pragma unroll
-      for (int ch = 0; ch < COLS / 32; ++ch) {
-        uint32_t pk[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          float2 x0, x1;
-          exponents(poly_only_tag, ch, i, x0, x1);
-          x0.x = ex2_approx(x0.x);
-          x0.y = ex2_approx(x0.y);
-          x1.x = ex2_approx(x1.x);
-          x1.y = ex2_approx(x1.y);
-          acc0 = fadd2(acc0, x0);
-          acc1 = fadd2(acc1, x1);
-          pk[i / 2] = pack2<BF16>(x0.x, x0.y);
-          pk[i / 2 + 1] = pack2<BF16>(x1.x, x1.y);
-        }
-        tmem_st16(s_addr + ch * 16, pk);
-      }
-    };
-    if constexpr (SOFTCAP) {
-      if (cap_poly_only)
-        exp_pass(std::true_type{});
-      else
-        exp_pass(std::false_type{});
-    } else {
-      exp_pass(std::false_type{});
-    }
-    l += (acc0.x + acc0.y) + (acc1.x + acc1.y);
+    // P over the first half of the thread's own S columns
+    l += row_exponentials<BF16, SOFTCAP, MASK, COLS>(sr, s_addr, lo_c, hi_c, p, cmul, m, cap_poly_only);
     deliver(buf);
     return true;
   }
@@ -338,34 +228,8 @@ struct SplitSoftmax {
       float l_row = l;
       if (!pair_total(*this, [&] { return c.wait(Cfg::BAR_O_FULL + ((g - 1) & 1), (g - 1) >> 1, WAIT_O_FULL); }, l_row)) return;
       tc_fence_after();
-      const float inv_l = 1.0f / l_row;
       const bool in_range = row < p.q_len;
-      const bool wide_stores = (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
-      uint4* out_row = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
-                                                (((int64_t)t.b * p.q_len + row) * p.heads + t.h) * (int64_t)D + half * (D / 2));
-#pragma unroll
-      for (int ch = 0; ch < D / 2 / 32; ++ch) {
-        uint32_t o[32];
-        tmem_ld32(o_addr + ch * 32, o);
-        tmem_ld_wait();
-        if (in_range) {
-          // every lane writes its own row (rows are heads * D elements apart), so a store instruction costs one
-          // memory transaction per lane whatever its width: 32-byte stores halve the count
-#pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            uint32_t x[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              x[e] = pack2<BF16>(__uint_as_float(o[v * 16 + 2 * e]) * inv_l, __uint_as_float(o[v * 16 + 2 * e + 1]) * inv_l);
-            if (wide_stores) {
-              st_global_v8(out_row + ch * 4 + v * 2, x);
-            } else {
-              out_row[ch * 4 + v * 2] = make_uint4(x[0], x[1], x[2], x[3]);
-              out_row[ch * 4 + v * 2 + 1] = make_uint4(x[4], x[5], x[6], x[7]);
-            }
-          }
-        }
-      }
+      row_store<BF16, D / 2>(o_addr, p.out, (((int64_t)t.b * p.q_len + row) * p.heads + t.h) * (int64_t)D + half * (D / 2), l_row, in_range);
       tc_fence_before();
       if (half == 0 && p.lse != nullptr && in_range)
         p.lse[((int64_t)t.b * p.heads + t.h) * p.lse_stride + row] = m + log2f(l_row);

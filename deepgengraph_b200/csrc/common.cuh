@@ -169,19 +169,6 @@ __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&w)[8]) 
                : "memory");
 }
 
-// Non-blocking probe (try_wait may suspend the thread for a while when the phase is still open).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // Bounded wait.  `abort_flag` is a CTA-shared word: once any thread of the CTA
 // has given up, every other wait of that CTA returns false quickly, so that all
 // roles fall through to the common tear-down (TMEM is always released).
