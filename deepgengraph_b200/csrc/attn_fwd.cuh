@@ -121,7 +121,7 @@ __device__ __forceinline__ void fwd_producer(const FwdCtx<Cfg, BF16>& c, const C
   bool ok = true;
   auto load = [&](bool is_v, int n) {
     const int i = issued, slot = i % SL, use = i / SL;
-    if (use > 0 && !mbar_wait(&c.bars[Cfg::BAR_EMPTY + slot], (use - 1) & 1, c.abort_flag, WAIT_K_EMPTY)) {
+    if (use > 0 && !mbar_wait(&c.bars[Cfg::BAR_EMPTY + slot], (use - 1) & 1, c.abort_flag, is_v ? WAIT_V_EMPTY : WAIT_K_EMPTY)) {
       ok = false;
       return;
     }

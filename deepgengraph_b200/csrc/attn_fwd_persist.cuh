@@ -223,7 +223,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         const int nb = t.hi - t.lo;
         auto load = [&](bool is_v, int n) {
           const int slot = ring_i % SL, use = ring_i / SL;
-          if (use > 0 && !mbar_wait(&c.bars[Cfg::BAR_EMPTY + slot], (use - 1) & 1, c.abort_flag, WAIT_K_EMPTY)) {
+          if (use > 0 && !mbar_wait(&c.bars[Cfg::BAR_EMPTY + slot], (use - 1) & 1, c.abort_flag,
+                                    is_v ? WAIT_V_EMPTY : WAIT_K_EMPTY)) {
             ok = false;
             return;
           }

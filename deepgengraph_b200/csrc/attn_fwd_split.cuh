@@ -288,7 +288,7 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
       for (int part = 0; part < Cfg::PARTS; ++part) {
         if (is_v && part > 0 && blocks.half_last && n == nb - 1) return;
         const int slot = ring_i % SL, use = ring_i / SL;
-        if (!ok || (use > 0 && !c.wait(Cfg::BAR_EMPTY + slot, use - 1, WAIT_K_EMPTY))) {
+        if (!ok || (use > 0 && !c.wait(Cfg::BAR_EMPTY + slot, use - 1, is_v ? WAIT_V_EMPTY : WAIT_K_EMPTY))) {
           ok = false;
           return;
         }
@@ -349,7 +349,7 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
   const uint32_t elected = elect_one(), bars = smem_u32(c.bars);
   int ring_i = 0, g0 = 0;
   bool ok = true;
-  auto wait_full = [&](int i) { return c.wait(Cfg::BAR_FULL + i % SL, i / SL, WAIT_K_FULL); };
+  auto wait_full = [&](int i, int code) { return c.wait(Cfg::BAR_FULL + i % SL, i / SL, code); };
   using Whole = std::integral_constant<int, PARTS>;
   using Half = std::integral_constant<int, 1>;
   auto issue_s = [&](auto parts_tag, int gb, bool last_of_tile) {
@@ -358,7 +358,7 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
 #pragma unroll
     for (int part = 0; part < PARTS; ++part) {
       const int slot = ring_i % SL;
-      if (ok) ok = wait_full(ring_i);
+      if (ok) ok = wait_full(ring_i, WAIT_K_FULL);
       ++ring_i;
       if (!ok) return;
       tc_fence_after();
@@ -398,7 +398,7 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
     constexpr int parts = decltype(parts_tag)::value;
 #pragma unroll
     for (int part = 0; part < parts; ++part)
-      if (ok) ok = wait_full(ring_i + part);
+      if (ok) ok = wait_full(ring_i + part, WAIT_V_FULL);
     if (ok) ok = c.wait(Cfg::BAR_P_FULL + gb % SB, gb / SB, WAIT_P_FULL);
     if (!ok) return;
     tc_fence_after();

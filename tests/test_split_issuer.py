@@ -32,3 +32,10 @@ def test_the_issue_helpers_take_no_step_of_the_whole_warp():
   helpers, _ = _issuer()
   helpers = helpers[helpers.index("auto wait_full = "):]
   assert not re.search(WHOLE_WARP, helpers)
+
+
+def test_an_expired_wait_for_v_is_reported_as_one_for_v():
+  text = open(os.path.join(CSRC, "attn_fwd_split.cuh")).read()
+  assert "is_v ? WAIT_V_EMPTY : WAIT_K_EMPTY" in text                                        # the producer's one wait
+  full = dict(re.findall(r"wait_full\((ring_i(?: \+ part)?), (\w+)\)", text))                # the issuer's two
+  assert full == {"ring_i": "WAIT_K_FULL", "ring_i + part": "WAIT_V_FULL"}
