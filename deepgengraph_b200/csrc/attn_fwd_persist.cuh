@@ -430,10 +430,12 @@ inline int sched_params(SchedParams* sp, const FwdParams& p, int head_dim, bool 
   sp->total_items = p.batch * p.heads * sp->n_q_tiles;
   // Group size.  Where all of K and V stay in L2 (126 MB) beside q and out, one group: the whole launch then runs heaviest
   // tile first and ends on the lightest.  Else as many units as have a quarter of L2 of K/V, at least 1 and at most 32.  K/V
-  // of a head count once for the query heads that share it.  Measured, groups -> one group (bf16, causal, us): 2 x 12 heads,
-  // 3000 tokens, head_dim 256 (74 MB) 114.5 -> 101.8; 4 x 32/8 heads, 1024 tokens (17 MB) 47.5 -> 45.9; 2 x 32/8, 777
-  // queries, 3001 keys (25 MB) 85.9 -> 84.1; 8 x 32, 512 tokens (67 MB) 37.3 -> 36.4; but 32 heads, 8192 tokens (134 MB)
-  // 454.9 -> 469.7 and 4 x 32, 4096 tokens (268 MB) 494.5 -> 559.6.
+  // of a head count once for the query heads that share it.  Measured, groups -> one group (bf16, causal, us), head_dim 128:
+  // 4 x 32/8 heads, 1024 tokens (17 MB) 47.5 -> 45.9; 2 x 32/8, 777 queries, 3001 keys (25 MB) 85.9 -> 84.1; 8 x 32, 512 tokens
+  // (67 MB) 37.3 -> 36.4; but 32 heads, 8192 tokens (134 MB) 454.9 -> 469.7 and 4 x 32, 4096 tokens (268 MB) 494.5 -> 559.6.
+  // head_dim 256, groups of 4 / 8 / one group: 4 x 16/8 heads, 1500 tokens (49 MB) 80.6 / 78.6 / 76.4; 2 x 12, 3000 tokens (74 MB)
+  // 103.0 / 99.1 / 100.5; the rule's groups -> one group: 2 x 16, 4096 tokens (134 MB) 218.6 -> 236.3; 4 x 12, 3000 tokens (147 MB)
+  // 196.9 -> 214.5; 4 x 16/8, 6000 tokens (196 MB) 881 -> 942.
   {
     const int64_t kv_bytes_per_head = (int64_t)2 * p.kv_len * head_dim * 2;
     const int units = p.batch * p.heads, group = p.heads / p.kv_heads;

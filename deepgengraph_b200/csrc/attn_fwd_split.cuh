@@ -5,14 +5,14 @@
 // TMEM (512 columns): two S buffers of 128 (the 16-bit P of a thread's 64 keys overwrites the first half of its own 64 columns), O 256.
 //
 // What bounds it and why this shape.  Per block of 128 keys the tensor pipe needs 16 x 64 clk for S and 8 x 128 for P V, 2048 in all,
-// the special-function unit 1024, and with the soft-cap the softmax is issue-bound on top.  With 64-key blocks and one softmax
-// warpgroup a block cost every hand-over (S -> softmax -> P -> P V) twice as often, and one warp per SM sub-partition could not keep
-// up with the soft-cap: 1771 clk per 64 keys, where the first form of this kernel took 3058 per 128 (2832 without the soft-cap, 630 of
-// them the issuer's barrier polls).  S with N = 128 runs at the full rate with Q in shared memory (N = 64: 48 instead of 32 clk), so
-// Q needs no TMEM and both S buffers hold 128 keys.
-// Measured, before -> now (one box, bf16, idle GPU / in a loop under the power cap): 16/8 heads, 8192 tokens, window 4096, soft-cap 50:
-// 379 -> 347 / 422 -> 385 us; 500 queries on 4000 keys, soft-cap: 66.6 -> 57 / 65 -> 55; causal without soft-cap, 8192 tokens:
-// 412 -> 409 / 456 -> 454.
+// the special-function unit 1024; a block takes 3130 clk with the soft-cap and 2900 without (a launch of 85.6 blocks per SM, everything
+// included): no pipe is full, the chain S -> softmax -> P -> P V of one tile is what is left.  With 64-key blocks and one softmax
+// warpgroup a block cost every hand-over of that chain twice as often, and one warp per SM sub-partition could not keep up with the
+// soft-cap.  S with N = 128 runs at the full rate with Q in shared memory (N = 64: 48 instead of 32 clk), so Q needs no TMEM and both S
+// buffers hold 128 keys.
+// Measured, 64-key blocks -> now (one box, bf16, us, idle GPU): 16/8 heads, 8192 tokens, window 4096, soft-cap 50: 376 -> 330; 500 queries
+// on 4000 keys, 32/8 heads: 52.4 -> 50.7, with soft-cap 64.9 -> 53.8; 16/8 heads, causal, 8192 tokens 402 -> 391, 1024 tokens 19.1 -> 18.3,
+// with soft-cap 23.0 -> 19.7, 64 tokens 6.6 -> 6.7.  In a loop under the power cap: window 4096, soft-cap 447 -> 396.
 #pragma once
 
 #include "attn_fwd_persist.cuh"
