@@ -222,10 +222,10 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<Cfg, BF16>& c) {
     const bool act = j >= lo && j < hi;
     if (elect_one()) B200_TL((3 * 64 + (n & 63)) * 8 + T * 4 + 2);
     if (act && !q_ready) {
-      ok = mbar_wait(&c.bars[Cfg::BAR_Q_FULL + T], 0, c.abort_flag, WAIT_Q_FULL);
+      ok = mbar_wait_warp(&c.bars[Cfg::BAR_Q_FULL + T], 0, c.abort_flag, WAIT_Q_FULL);
       q_ready = true;
     }
-    ok = ok && mbar_wait(&c.bars[Cfg::BAR_FULL + slot], ph, c.abort_flag, WAIT_K_FULL);
+    ok = ok && mbar_wait_warp(&c.bars[Cfg::BAR_FULL + slot], ph, c.abort_flag, WAIT_K_FULL);
     if (!ok) return;
     tc_fence_after();
     if (elect_one()) {
@@ -255,13 +255,13 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<Cfg, BF16>& c) {
     const bool act_k = has_k && jk >= lo && jk < hi;
     const int nt = jv - lo, buf = nt % SB;
     if (elect_one()) B200_TL((3 * 64 + (n & 63)) * 8 + T * 4 + 0);
-    ok = mbar_wait(&c.bars[Cfg::BAR_FULL + vslot], vph, c.abort_flag, WAIT_V_FULL);
-    if (ok && has_k) ok = mbar_wait(&c.bars[Cfg::BAR_FULL + kslot], kph, c.abort_flag, WAIT_K_FULL);
+    ok = mbar_wait_warp(&c.bars[Cfg::BAR_FULL + vslot], vph, c.abort_flag, WAIT_V_FULL);
+    if (ok && has_k) ok = mbar_wait_warp(&c.bars[Cfg::BAR_FULL + kslot], kph, c.abort_flag, WAIT_K_FULL);
     if (ok && act_k && !q_ready) {
-      ok = mbar_wait(&c.bars[Cfg::BAR_Q_FULL + T], 0, c.abort_flag, WAIT_Q_FULL);
+      ok = mbar_wait_warp(&c.bars[Cfg::BAR_Q_FULL + T], 0, c.abort_flag, WAIT_Q_FULL);
       q_ready = true;
     }
-    if (ok && act_v) ok = mbar_wait(&c.bars[Cfg::BAR_P_FULL + T * SB + buf], (nt / SB) & 1, c.abort_flag, WAIT_P_FULL);
+    if (ok && act_v) ok = mbar_wait_warp(&c.bars[Cfg::BAR_P_FULL + T * SB + buf], (nt / SB) & 1, c.abort_flag, WAIT_P_FULL);
     if (!ok) return;
     tc_fence_after();
     if (elect_one()) {
@@ -281,7 +281,7 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<Cfg, BF16>& c) {
   // every MMA issued above has retired before the CTA tears TMEM down
   if (elect_one()) umma_commit(&c.bars[Cfg::BAR_DRAIN + T]);
   __syncwarp();
-  mbar_wait(&c.bars[Cfg::BAR_DRAIN + T], 0, c.abort_flag, WAIT_DRAIN);
+  mbar_wait_warp(&c.bars[Cfg::BAR_DRAIN + T], 0, c.abort_flag, WAIT_DRAIN);
 }
 
 // ------------------------------ softmax warpgroup ----------------------------
@@ -528,14 +528,14 @@ __device__ __forceinline__ bool fwd_softmax_block(const FwdCtx<Cfg, BF16>& c, co
     // P V(n-2) too, and P V(n+1) cannot start before this thread delivers P(n): the barrier is exactly in or
     // just past the awaited phase.
     // (g counts the P V products of this CTA: equal to n unless the CTA walks several tiles)
-    if (!mbar_wait(o_full + ((g - 1) & 1), ((g - 1) >> 1) & 1, c.abort_flag, WAIT_O_FULL)) return false;
+    if (!mbar_wait_warp(o_full + ((g - 1) & 1), ((g - 1) >> 1) & 1, c.abort_flag, WAIT_O_FULL)) return false;
     tc_fence_after();
     row_rescale<D>(o_addr, alpha);
   }
   // The exponentials saturate the special-function unit, which the warp of the other query tile on this SM
   // sub-partition shares: the two take turns (see fwd_softmax), so that one tile's exponentials overlap the
   // other tile's MMAs instead of colliding with its exponentials.
-  if (turn_wait != nullptr && !mbar_wait(turn_wait, turn_parity, c.abort_flag, WAIT_TURN)) return false;
+  if (turn_wait != nullptr && !mbar_wait_warp(turn_wait, turn_parity, c.abort_flag, WAIT_TURN)) return false;
   // P over the first BN/2 columns of S
   l += row_exponentials<BF16, SOFTCAP, MASK, BN>(sr, s_addr, lo_c, hi_c, p, cmul, m, cap_poly_only);
   if (turn_pass != nullptr) {
@@ -590,7 +590,7 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<Cfg, BF16>& c, const Fw
     const int n = j - rng.lo, buf = n % SB;
     const uint32_t s_addr = s_addr0 + buf * BN;
     uint64_t* p_full = &c.bars[Cfg::BAR_P_FULL + t * SB + buf];
-    if (!mbar_wait(&c.bars[Cfg::BAR_S_FULL + t * SB + buf], (n / SB) & 1, c.abort_flag, WAIT_S_FULL)) return;
+    if (!mbar_wait_warp(&c.bars[Cfg::BAR_S_FULL + t * SB + buf], (n / SB) & 1, c.abort_flag, WAIT_S_FULL)) return;
     tc_fence_after();
     // a block needs element masks only if some row of the tile sees it partially
     const bool need_mask = (hi_first - j * BN < BN - 1) || (lo_last - j * BN > 0);
@@ -616,7 +616,7 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<Cfg, BF16>& c, const Fw
   // epilogue: O / l -> 16-bit -> global (BSHD), base-2 LSE for the score passes
   if ((threadIdx.x & 127) == 0) B200_TL((3 * 64 + 62) * 8 + 2);   // last block's P delivered
   const int last = rng.hi - rng.lo - 1;
-  if (!mbar_wait(o_full + (last & 1), (last >> 1) & 1, c.abort_flag, WAIT_O_FULL)) return;
+  if (!mbar_wait_warp(o_full + (last & 1), (last >> 1) & 1, c.abort_flag, WAIT_O_FULL)) return;
   tc_fence_after();
   if ((threadIdx.x & 127) == 0) B200_TL((3 * 64 + 62) * 8 + 3);   // last P V complete
   const bool in_range = row < p.q_len;

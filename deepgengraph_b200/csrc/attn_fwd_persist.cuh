@@ -137,7 +137,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const float cmul = SOFTCAP ? p.cap_out : p.scale_log2;
     int g = 0;   // blocks processed by this CTA so far (S / P buffer = g % SB, barrier phases follow g)
     for (int k = 0;; ++k) {
-      if (!mbar_wait(&c.bars[Cfg::BAR_SCHED + (k & 1)], (k >> 1) & 1, c.abort_flag, WAIT_SCHED)) break;
+      if (!mbar_wait_warp(&c.bars[Cfg::BAR_SCHED + (k & 1)], (k >> 1) & 1, c.abort_flag, WAIT_SCHED)) break;
       const int item = sched[k & 1];
       __syncwarp();
       if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_SCHED_FREE + (k & 1)]);   // slot may be rewritten for tile k + 2
@@ -155,7 +155,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         const uint32_t s_addr = lane_addr + buf * BN;
         uint64_t* p_full = &c.bars[Cfg::BAR_P_FULL + buf];
         if (threadIdx.x == 0 && g < 64) B200_TL((g & 63) * 8 + 5);
-        ok = mbar_wait(&c.bars[Cfg::BAR_S_FULL + buf], (g / SB) & 1, c.abort_flag, WAIT_S_FULL);
+        ok = mbar_wait_warp(&c.bars[Cfg::BAR_S_FULL + buf], (g / SB) & 1, c.abort_flag, WAIT_S_FULL);
         if (!ok) break;
         if (threadIdx.x == 0 && g < 64) B200_TL((g & 63) * 8 + 6);
         tc_fence_after();
@@ -175,7 +175,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       const int last = g - 1;
       // (tuning builds: slots (3 * 64 + 48 + tile) * 8 + {0: last P delivered, 1: last P V complete, 2: output stored})
       if (threadIdx.x == 0 && k < 8) B200_TL((3 * 64 + 48 + k) * 8 + 0);
-      if (!mbar_wait(o_full + (last & 1), (last >> 1) & 1, c.abort_flag, WAIT_O_FULL)) break;
+      if (!mbar_wait_warp(o_full + (last & 1), (last >> 1) & 1, c.abort_flag, WAIT_O_FULL)) break;
       tc_fence_after();
       if (threadIdx.x == 0 && k < 8) B200_TL((3 * 64 + 48 + k) * 8 + 1);
       const bool in_range = row < p.q_len;
@@ -293,19 +293,19 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     int ring_i = 0, g0 = 0;   // ring items consumed, blocks issued before this tile
     bool ok = true;
     for (int k = 0; ok; ++k) {
-      if (!mbar_wait(&c.bars[Cfg::BAR_SCHED + (k & 1)], (k >> 1) & 1, c.abort_flag, WAIT_SCHED)) break;
+      if (!mbar_wait_warp(&c.bars[Cfg::BAR_SCHED + (k & 1)], (k >> 1) & 1, c.abort_flag, WAIT_SCHED)) break;
       const int item = sched[k & 1];
       __syncwarp();
       if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_SCHED_FREE + (k & 1)]);
       if (item < 0) break;
       const TileInfo t = decode_item(item, p, sp, BN);
       const int nb = t.hi - t.lo;
-      ok = mbar_wait(&c.bars[Cfg::BAR_Q_FULL], k & 1, c.abort_flag, WAIT_Q_FULL);
+      ok = mbar_wait_warp(&c.bars[Cfg::BAR_Q_FULL], k & 1, c.abort_flag, WAIT_Q_FULL);
       // S of the first SB blocks
       for (int n = 0; n < SB && n < nb && ok; ++n) {
         const int slot = ring_i % SL, ph = (ring_i / SL) & 1;
         ++ring_i;
-        ok = mbar_wait(&c.bars[Cfg::BAR_FULL + slot], ph, c.abort_flag, WAIT_K_FULL);
+        ok = mbar_wait_warp(&c.bars[Cfg::BAR_FULL + slot], ph, c.abort_flag, WAIT_K_FULL);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
@@ -323,7 +323,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       // while the four P V MMAs execute.
       int vslot = ring_i % SL, vph = (ring_i / SL) & 1;
       ++ring_i;
-      if (ok) ok = mbar_wait(&c.bars[Cfg::BAR_FULL + vslot], vph, c.abort_flag, WAIT_V_FULL);   // V(0)
+      if (ok) ok = mbar_wait_warp(&c.bars[Cfg::BAR_FULL + vslot], vph, c.abort_flag, WAIT_V_FULL);   // V(0)
       for (int n = 0; n < nb && ok; ++n) {
         const bool has_k = n + SB < nb;
         const int kslot = ring_i % SL, kph = (ring_i / SL) & 1;
@@ -333,7 +333,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         if (has_v) ++ring_i;
         const int gb = g0 + n;
         if (lane == 0 && gb < 64) B200_TL((3 * 64 + (gb & 63)) * 8 + 0);
-        ok = mbar_wait(&c.bars[Cfg::BAR_P_FULL + (gb % SB)], (gb / SB) & 1, c.abort_flag, WAIT_P_FULL);
+        ok = mbar_wait_warp(&c.bars[Cfg::BAR_P_FULL + (gb % SB)], (gb / SB) & 1, c.abort_flag, WAIT_P_FULL);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
@@ -343,8 +343,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
           if (gb < 64) B200_TL((2 * 64 + (gb & 63)) * 8 + 1);
         }
         __syncwarp();
-        if (has_k) ok = mbar_wait(&c.bars[Cfg::BAR_FULL + kslot], kph, c.abort_flag, WAIT_K_FULL);
-        if (ok && has_v) ok = mbar_wait(&c.bars[Cfg::BAR_FULL + nvslot], nvph, c.abort_flag, WAIT_V_FULL);
+        if (has_k) ok = mbar_wait_warp(&c.bars[Cfg::BAR_FULL + kslot], kph, c.abort_flag, WAIT_K_FULL);
+        if (ok && has_v) ok = mbar_wait_warp(&c.bars[Cfg::BAR_FULL + nvslot], nvph, c.abort_flag, WAIT_V_FULL);
         if (!ok) break;
         tc_fence_after();
         if (has_k) {
@@ -367,9 +367,9 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         const int kslot = ring_i % SL, kph = (ring_i / SL) & 1;
         if (has_k) ++ring_i;
         const int gb = g0 + n;
-        ok = mbar_wait(&c.bars[Cfg::BAR_FULL + vslot], vph, c.abort_flag, WAIT_V_FULL);
-        if (ok && has_k) ok = mbar_wait(&c.bars[Cfg::BAR_FULL + kslot], kph, c.abort_flag, WAIT_K_FULL);
-        if (ok) ok = mbar_wait(&c.bars[Cfg::BAR_P_FULL + (gb % SB)], (gb / SB) & 1, c.abort_flag, WAIT_P_FULL);
+        ok = mbar_wait_warp(&c.bars[Cfg::BAR_FULL + vslot], vph, c.abort_flag, WAIT_V_FULL);
+        if (ok && has_k) ok = mbar_wait_warp(&c.bars[Cfg::BAR_FULL + kslot], kph, c.abort_flag, WAIT_K_FULL);
+        if (ok) ok = mbar_wait_warp(&c.bars[Cfg::BAR_P_FULL + (gb % SB)], (gb / SB) & 1, c.abort_flag, WAIT_P_FULL);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
@@ -386,7 +386,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // every MMA issued above has retired before the CTA tears TMEM down
     if (elect_one()) umma_commit(&c.bars[Cfg::BAR_DRAIN]);
     __syncwarp();
-    mbar_wait(&c.bars[Cfg::BAR_DRAIN], 0, c.abort_flag, WAIT_DRAIN);
+    mbar_wait_warp(&c.bars[Cfg::BAR_DRAIN], 0, c.abort_flag, WAIT_DRAIN);
   }
 
   tc_fence_before();

@@ -76,7 +76,7 @@ struct SplitCtx {
     return mbar_wait(&bars[bar], parity & 1, abort_flag, code);
   }
   __device__ __forceinline__ bool wait_warp(int bar, int parity, int code) const {   // one outcome for the whole warp
-    return __all_sync(0xffffffffu, wait(bar, parity, code));
+    return mbar_wait_warp(&bars[bar], parity & 1, abort_flag, code);
   }
 };
 

@@ -263,11 +263,11 @@ __device__ __forceinline__ void sweep_mma(const SweepCtx<Cfg>& c, int n_items) {
   constexpr uint32_t IDESC = make_idesc(BF16, 128, BX, false, false);
   const uint32_t desc_hi = smem_desc_hi(1024);
   const uint32_t a_lo = smem_desc_lo(smem_u32(c.sA), 16), x_lo = smem_desc_lo(smem_u32(c.sX), 16);
-  bool ok = mbar_wait(&c.bars[Cfg::BAR_A_FULL], 0, c.abort_flag, WAIT_Q_FULL);
+  bool ok = mbar_wait_warp(&c.bars[Cfg::BAR_A_FULL], 0, c.abort_flag, WAIT_Q_FULL);
   for (int n = 0; n < n_items && ok; ++n) {
     const int st = n % ST, tb = n & 1, tuse = n >> 1;
-    if (tuse > 0) ok = mbar_wait(&c.bars[Cfg::BAR_T_EMPTY + tb], (tuse - 1) & 1, c.abort_flag, WAIT_T_EMPTY);
-    ok = ok && mbar_wait(&c.bars[Cfg::BAR_X_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_X_FULL);
+    if (tuse > 0) ok = mbar_wait_warp(&c.bars[Cfg::BAR_T_EMPTY + tb], (tuse - 1) & 1, c.abort_flag, WAIT_T_EMPTY);
+    ok = ok && mbar_wait_warp(&c.bars[Cfg::BAR_X_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_X_FULL);
     if (!ok) break;
     tc_fence_after();
     if (elect_one()) {
@@ -397,9 +397,11 @@ __device__ __forceinline__ void sweep_compute_colsum(const SweepCtx<Cfg>& c, con
     [[maybe_unused]] const bool tl_on = threadIdx.x == 0;
     [[maybe_unused]] const int tl_base = (n & 63) * 8;
     if (tl_on) B200_TL(tl_base + 0);
-    if (!mbar_wait(&c.bars[Cfg::BAR_T_FULL + tb], (n >> 1) & 1, c.abort_flag, WAIT_T_FULL)) return;
+    // (one vote for both waits: mbar_wait_warp)
+    if (!__all_sync(0xffffffffu, mbar_wait(&c.bars[Cfg::BAR_T_FULL + tb], (n >> 1) & 1, c.abort_flag, WAIT_T_FULL) &&
+                                     mbar_wait(&c.bars[Cfg::BAR_N_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_N_FULL)))
+      return;
     if (tl_on) B200_TL(tl_base + 1);
-    if (!mbar_wait(&c.bars[Cfg::BAR_N_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_N_FULL)) return;
     tc_fence_after();
     if (tl_on) B200_TL(tl_base + 2);
     const uint8_t* nst = c.sN + st * Cfg::N_STAGE_STRIDE;
@@ -499,8 +501,9 @@ __device__ __forceinline__ void sweep_compute_colsum_grouped(const SweepCtx<Cfg>
   int blk = c.blk_lo, hh = 0;
   for (int n = 0; n < n_items; ++n) {
     const int st = n % ST, tb = n & 1;
-    if (!mbar_wait(&c.bars[Cfg::BAR_T_FULL + tb], (n >> 1) & 1, c.abort_flag, WAIT_T_FULL)) return;
-    if (!mbar_wait(&c.bars[Cfg::BAR_N_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_N_FULL)) return;
+    if (!__all_sync(0xffffffffu, mbar_wait(&c.bars[Cfg::BAR_T_FULL + tb], (n >> 1) & 1, c.abort_flag, WAIT_T_FULL) &&
+                                     mbar_wait(&c.bars[Cfg::BAR_N_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_N_FULL)))
+      return;
     tc_fence_after();
     const float* lse_s = reinterpret_cast<const float*>(c.sN + st * Cfg::N_STAGE_STRIDE + Cfg::NOISE_BYTES);
     const int i0 = blk * BX;
@@ -574,9 +577,10 @@ __device__ __forceinline__ void sweep_compute_rowlse(const SweepCtx<Cfg>& c, con
 
   for (int blk = c.blk_lo; blk < c.blk_hi; ++blk) {
     const int n = blk - c.blk_lo, st = n % ST, tb = n & 1;
-    if (!mbar_wait(&c.bars[Cfg::BAR_T_FULL + tb], (n >> 1) & 1, c.abort_flag, WAIT_T_FULL)) return;
+    bool ok = mbar_wait(&c.bars[Cfg::BAR_T_FULL + tb], (n >> 1) & 1, c.abort_flag, WAIT_T_FULL);
     if constexpr (Cfg::N_STAGE_BYTES > 0)
-      if (!mbar_wait(&c.bars[Cfg::BAR_N_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_N_FULL)) return;
+      ok = ok && mbar_wait(&c.bars[Cfg::BAR_N_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_N_FULL);
+    if (!__all_sync(0xffffffffu, ok)) return;
     tc_fence_after();
     [[maybe_unused]] const uint8_t* nst = c.sN + st * Cfg::N_STAGE_STRIDE;
     const int hi_c = hi_key - blk * BX;

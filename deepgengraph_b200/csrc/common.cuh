@@ -196,6 +196,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_slow(bar, parity, abort_flag, code);
 }
 
+// For a whole warp: one outcome for all of its lanes.  Lane by lane, one could see the abort flag where another sees the phase; the
+// first would leave its role, and the next step that takes the whole warp (elect.sync, a vote) would wait for it without limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, abort_flag, code));
+}
+
 // Brings the line of `p` into L2, without reading it: a load that follows costs a round trip to L2 instead of one to HBM.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
