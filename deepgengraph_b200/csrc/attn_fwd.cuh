@@ -753,8 +753,8 @@ int launch_attn_fwd_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
 
 // persistent variant (attn_fwd_persist.cuh)
 template <bool BF16, bool SOFTCAP>
-int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
-                            cudaStream_t stream);
+int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
+                            const FwdParams& p, cudaStream_t stream);
 
 // head_dim 256 (attn_fwd_split.cuh)
 struct AttnStrides;
@@ -836,12 +836,18 @@ inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v,
 #else
   constexpr int NQ = 1;
 #endif
-#define B200_FWD_DISPATCH(launch, ...)                                                                          \
-  (bf16 ? (cap ? launch<__VA_ARGS__ true, true>(tq, tk, tv, p, stream) : launch<__VA_ARGS__ true, false>(tq, tk, tv, p, stream))   \
-        : (cap ? launch<__VA_ARGS__ false, true>(tq, tk, tv, p, stream) : launch<__VA_ARGS__ false, false>(tq, tk, tv, p, stream)))
-  if (!one_tile_per_cta && B200_BN128 == 64 && B200_SB128 == 2) return B200_FWD_DISPATCH(launch_attn_fwd_persist, );
-  return B200_FWD_DISPATCH(launch_attn_fwd_cfg, B200_BN128, NQ, B200_SB128, );
-#undef B200_FWD_DISPATCH
+  if (!one_tile_per_cta && B200_BN128 == 64 && B200_SB128 == 2) {
+    CUtensorMap to;   // a warp stores 32 rows
+    if ((rc = make_bshd_tensor_map(&to, out, batch, q_len, heads, head_dim, 32, bf16)) != B200_OK) return rc;
+    return bf16 ? (cap ? launch_attn_fwd_persist<true, true>(tq, tk, tv, to, p, stream)
+                       : launch_attn_fwd_persist<true, false>(tq, tk, tv, to, p, stream))
+                : (cap ? launch_attn_fwd_persist<false, true>(tq, tk, tv, to, p, stream)
+                       : launch_attn_fwd_persist<false, false>(tq, tk, tv, to, p, stream));
+  }
+  return bf16 ? (cap ? launch_attn_fwd_cfg<B200_BN128, NQ, B200_SB128, true, true>(tq, tk, tv, p, stream)
+                     : launch_attn_fwd_cfg<B200_BN128, NQ, B200_SB128, true, false>(tq, tk, tv, p, stream))
+              : (cap ? launch_attn_fwd_cfg<B200_BN128, NQ, B200_SB128, false, true>(tq, tk, tv, p, stream)
+                     : launch_attn_fwd_cfg<B200_BN128, NQ, B200_SB128, false, false>(tq, tk, tv, p, stream));
 }
 
 inline int attn_fwd_impl(const void* q, const void* k, const void* v, void* out, float* lse, int batch, int q_len,

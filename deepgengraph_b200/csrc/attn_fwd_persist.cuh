@@ -55,6 +55,7 @@ __device__ __forceinline__ TileInfo decode_item(int item, const FwdParams& p, co
   return t;
 }
 
+template <bool SOFTCAP>
 struct PersistCfg : FwdCfg<64, 1, 2> {
   using Base = FwdCfg<64, 1, 2>;
   static constexpr int SOFTMAX_WARPS = 4;
@@ -63,23 +64,64 @@ struct PersistCfg : FwdCfg<64, 1, 2> {
   static constexpr int BAR_Q_FREE = BAR_SCHED + 2;        // last S MMA of a tile retired: Q buffer reusable
   static constexpr int BAR_SCHED_FREE = BAR_Q_FREE + 1;   // [2] descriptor slot read by all its consumers
   static constexpr int NUM_BARS_P = BAR_SCHED_FREE + 2;
-  static constexpr int SMEM_BYTES_P = Base::SMEM_TILES + NUM_BARS_P * 8 + 64 + 1024;
+  // Without a soft-cap the output goes through 4 KB of staging per softmax warp (32 rows x 64 columns) to bulk stores, and the first loads
+  // are issued before the set-up is over.  32 query heads, bf16, us per call, before -> with the bulk stores -> with both: 4 x 256
+  // tokens, 8 K/V heads 9.89 -> 9.46 -> 9.13; 4 x 1024 tokens, 8 K/V heads 44.5 -> 43.1 -> 42.5; 128 tokens 6.66 -> 6.65 -> 6.47;
+  // 512 tokens 10.94 -> 10.96 -> 10.71; 2048 tokens 37.1 -> 36.7 -> 35.5; 4 x 4096 tokens 499 -> 499 -> 486 (idle GPU).
+  // With a soft-cap the compiler schedules the longer softmax worse around either (2 x 4096 tokens 327 -> 338, 2048 tokens 52.2 -> 54.5,
+  // 159 -> 160 registers), so that kernel stores its rows directly and loads after the set-up.
+  static constexpr bool STAGED = !SOFTCAP;
+  // Behind Q, the ring and the staging: barriers, a few words.  Without static shared memory, dynamic shared memory starts at a
+  // multiple of 1024 bytes.
+  static constexpr int STAGE_OUT_BYTES = 32 * 128;
+  static constexpr int OFF_BARS = Base::SMEM_TILES + (STAGED ? SOFTMAX_WARPS * STAGE_OUT_BYTES : 0);
+  static constexpr int SMEM_BYTES_P = OFF_BARS + NUM_BARS_P * 8 + 64 + (STAGED ? 0 : 1024);
   static_assert(SMEM_BYTES_P <= Base::SMEM_BUDGET, "shared memory budget exceeded");
 };
 
+// O / l of a warp's 32 rows -> 16-bit -> global, 64 columns at a time: every lane writes its row (128 bytes, the swizzle of the tensor map)
+// to the warp's staging tile, one lane stores the tile.  The lanes' rows are heads * D elements apart in memory, so that plain stores
+// cost a transaction per lane and 32 bytes.
+template <bool BF16>
+__device__ __forceinline__ void row_store_bulk(uint32_t o_addr, uint8_t* stage, const CUtensorMap* tm_o, const TileInfo& t, int row0,
+                                               int q_len, int lane, float l) {
+  const float inv_l = 1.0f / l;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t o[2][32];
+    tmem_ld32(o_addr + half * 64, o[0]);
+    tmem_ld32(o_addr + half * 64 + 32, o[1]);
+    if (lane == 0) bulk_wait_read();   // the tile's last store has read it
+    tmem_ld_wait();
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        w[e] = pack2<BF16>(__uint_as_float(o[v / 4][(v % 4) * 8 + 2 * e]) * inv_l, __uint_as_float(o[v / 4][(v % 4) * 8 + 2 * e + 1]) * inv_l);
+      *reinterpret_cast<uint4*>(stage + lane * 128 + ((v ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0 && row0 < q_len) {   // (rows beyond q_len are cut off)
+      tma_store_4d(tm_o, stage, half * 64, t.h, row0, t.b);
+      bulk_commit();
+    }
+  }
+}
+
 template <bool BF16, bool SOFTCAP>
-__global__ void __launch_bounds__(PersistCfg::THREADS_P, PersistCfg::CTAS_PER_SM)
+__global__ void __launch_bounds__(PersistCfg<SOFTCAP>::THREADS_P, PersistCfg<SOFTCAP>::CTAS_PER_SM)
 attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                        const __grid_constant__ CUtensorMap tm_v, const FwdParams p, const SchedParams sp) {
-  using Cfg = PersistCfg;
+                        const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const FwdParams p,
+                        const SchedParams sp) {
+  using Cfg = PersistCfg<SOFTCAP>;
   constexpr int SL = Cfg::SLOTS, D = Cfg::D, BN = Cfg::BN, BM = Cfg::BM, SB = Cfg::SB;
   constexpr int PRODUCER_WARP = Cfg::SOFTMAX_WARPS;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = Cfg::STAGED ? smem_raw : reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 
-  // A launch that follows an expired wait on this device drains immediately (the status word stays set until the
-  // host reads it).
-  __shared__ int s_skip;
   if (threadIdx.x == 32) prefetch_l2(&g_device_status);   // read after the wait below
 
   [[maybe_unused]] const uint64_t cta_start_ns = global_timer_ns();
@@ -89,13 +131,25 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   FwdCtx<Cfg, BF16> c;
   c.sQ = smem;
   c.sKV = c.sQ + Cfg::Q_TILE_BYTES;
-  c.bars = reinterpret_cast<uint64_t*>(c.sKV + SL * Cfg::KV_STAGE_BYTES);
+  c.bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BARS);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c.bars + Cfg::NUM_BARS_P);
   c.abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* s_skip = reinterpret_cast<volatile int*>(tmem_slot + 4);
   volatile int* sched = reinterpret_cast<volatile int*>(tmem_slot + 2);   // [2] item index or -1
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
+  // The producer initialises the barriers, so that its first loads need not wait for the rest of the block.
+  if (!Cfg::STAGED && warp == PRODUCER_WARP && lane == 0) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
+  if (Cfg::STAGED ? (warp == PRODUCER_WARP && lane == 0) : threadIdx.x == 0) {
+    if (Cfg::STAGED) {
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_v);
+    }
 #pragma unroll
     for (int i = 0; i < Cfg::NUM_BARS_P; ++i) {
       const bool is_p_full = (i >= Cfg::BAR_P_FULL && i < Cfg::BAR_P_FULL + SB);   // every softmax warp
@@ -106,15 +160,31 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     *c.abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == PRODUCER_WARP && lane == 0) {
-    tma_prefetch_desc(&tm_q);
-    tma_prefetch_desc(&tm_k);
-    tma_prefetch_desc(&tm_v);
-  }
+  TileInfo first_tile;   // (producer)
+  if (Cfg::STAGED && warp == PRODUCER_WARP) first_tile = decode_item(blockIdx.x, p, sp, BN);   // the grid has no more CTAs than items
   // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
   // to allocate columns of its own, and what it wrote is visible only now.
   pdl_wait();
-  if (threadIdx.x == 32) s_skip = *reinterpret_cast<volatile int*>(&g_device_status);
+  // Q and the first K block of the first tile are on their way while tensor memory is allocated and the status word comes in.
+  auto load_q = [&](const TileInfo& t) {
+    mbar_expect_tx(&c.bars[Cfg::BAR_Q_FULL], Cfg::Q_TILE_BYTES);
+#pragma unroll
+    for (int ks = 0; ks < Cfg::KSUB; ++ks)
+      tma_load_4d(c.sQ + ks * (BM * 128), &tm_q, &c.bars[Cfg::BAR_Q_FULL], ks * 64, t.h, t.q0, t.b);
+  };
+  auto load_kv = [&](const TileInfo& t, bool is_v, int n, int slot) {
+    uint64_t* full = &c.bars[Cfg::BAR_FULL + slot];
+    uint8_t* dst = c.sKV + slot * Cfg::KV_STAGE_BYTES;
+    mbar_expect_tx(full, Cfg::KV_STAGE_BYTES);
+#pragma unroll
+    for (int ks = 0; ks < Cfg::KSUB; ++ks)
+      tma_load_4d(dst + ks * (BN * 128), is_v ? &tm_v : &tm_k, full, ks * 64, t.hk, (t.lo + n) * BN, t.b);
+  };
+  if (Cfg::STAGED && warp == PRODUCER_WARP && lane == 0) {
+    load_q(first_tile);
+    load_kv(first_tile, false, 0, 0);
+  }
+  if (threadIdx.x == 32) *s_skip = *reinterpret_cast<volatile int*>(&g_device_status);
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
@@ -123,7 +193,15 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   __syncthreads();
   tc_fence_after();
   c.tmem_base = *tmem_slot;
-  if (s_skip != 0) {   // (the tile counter is untouched: the host zeroes it when it clears the status word)
+  // A launch that follows an expired wait on this device drains immediately (the status word stays set until the host reads it; the tile
+  // counter is untouched: the host zeroes it when it clears the word).
+  if (*s_skip != 0) {
+    if (Cfg::STAGED && warp == PRODUCER_WARP && lane == 0) {
+      const uint64_t t0 = global_timer_ns();   // the two loads above land before the CTA exits (bounded, 20 ms)
+      for (int bar : {Cfg::BAR_Q_FULL, Cfg::BAR_FULL})
+        while (!mbar_try_wait(&c.bars[bar], 0) && global_timer_ns() - t0 < 20000000ull) {
+        }
+    }
     if (warp == 0) tmem_dealloc(c.tmem_base, Cfg::TMEM_COLS);
     return;
   }
@@ -179,15 +257,19 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       tc_fence_after();
       if (threadIdx.x == 0 && k < 8) B200_TL((3 * 64 + 48 + k) * 8 + 1);
       const bool in_range = row < p.q_len;
-      row_store<BF16, D>(o_addr, p.out, (((int64_t)t.b * p.q_len + row) * p.heads + t.h) * (int64_t)D, l, in_range);
+      if constexpr (!Cfg::STAGED)
+        row_store<BF16, D>(o_addr, p.out, (((int64_t)t.b * p.q_len + row) * p.heads + t.h) * (int64_t)D, l, in_range);
+      else
+        row_store_bulk<BF16>(o_addr, smem + Cfg::SMEM_TILES + warp * Cfg::STAGE_OUT_BYTES, &tm_o, t, t.q0 + warp_q * 32, p.q_len, lane, l);
       if (p.lse != nullptr && in_range) p.lse[((int64_t)t.b * p.heads + t.h) * p.lse_stride + row] = m + log2f(l);
       if (threadIdx.x == 0 && k < 8) B200_TL((3 * 64 + 48 + k) * 8 + 2);
       blocks_done = g;
     }
+    if (Cfg::STAGED && lane == 0) bulk_wait_read();   // (the stores themselves end with the kernel)
   } else if (warp == PRODUCER_WARP) {
     // --------------------------- TMA producer + tile scheduler ---------------------------
     if (lane == 0) {
-      int ring_i = 0;   // K/V ring items issued so far (continuous across tiles)
+      int ring_i = Cfg::STAGED ? 1 : 0;   // K/V ring items issued so far (continuous across tiles)
       bool ok = true;
       for (int k = 0; ok; ++k) {
         // the first tile of a CTA is its own index (no round trip to the counter before the first load is issued)
@@ -216,10 +298,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         const TileInfo t = decode_item(item, p, sp, BN);
         if (k > 0) ok = mbar_wait(&c.bars[Cfg::BAR_Q_FREE], (k - 1) & 1, c.abort_flag, WAIT_Q_FREE);
         if (!ok) break;
-        mbar_expect_tx(&c.bars[Cfg::BAR_Q_FULL], Cfg::Q_TILE_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < Cfg::KSUB; ++ks)
-          tma_load_4d(c.sQ + ks * (BM * 128), &tm_q, &c.bars[Cfg::BAR_Q_FULL], ks * 64, t.h, t.q0, t.b);
+        if (k > 0 || !Cfg::STAGED) load_q(t);
+        // K(0 .. SB-1), V(0), K(SB), V(1), ...
         const int nb = t.hi - t.lo;
         auto load = [&](bool is_v, int n) {
           const int slot = ring_i % SL, use = ring_i / SL;
@@ -228,18 +308,21 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             ok = false;
             return;
           }
-          uint64_t* full = &c.bars[Cfg::BAR_FULL + slot];
-          uint8_t* dst = c.sKV + slot * Cfg::KV_STAGE_BYTES;
-          mbar_expect_tx(full, Cfg::KV_STAGE_BYTES);
-#pragma unroll
-          for (int ks = 0; ks < Cfg::KSUB; ++ks)
-            tma_load_4d(dst + ks * (BN * 128), is_v ? &tm_v : &tm_k, full, ks * 64, t.hk, (t.lo + n) * BN, t.b);
+          load_kv(t, is_v, n, slot);
           ++ring_i;
         };
-        for (int n = 0; n < SB && n < nb && ok; ++n) load(false, n);
-        for (int n = 0; n < nb && ok; ++n) {
-          load(true, n);
-          if (ok && n + SB < nb) load(false, n + SB);
+        if constexpr (Cfg::STAGED) {   // (one loop for both: 1024 tokens 17.6 us, with the two loops below 17.8)
+          int next_k = k == 0 ? 1 : 0, next_v = 0;
+          while (ok && next_v < nb) {
+            const bool is_v = next_k == nb || next_k - next_v == SB;
+            load(is_v, is_v ? next_v++ : next_k++);
+          }
+        } else {
+          for (int n = 0; n < SB && n < nb && ok; ++n) load(false, n);
+          for (int n = 0; n < nb && ok; ++n) {
+            load(true, n);
+            if (ok && n + SB < nb) load(false, n + SB);
+          }
         }
       }
       if (!ok || *c.abort_flag != 0) {
@@ -248,8 +331,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         for (int slot = 0; slot < SL; ++slot) {
           if (ring_i <= slot) continue;
           const int last = slot + ((ring_i - 1 - slot) / SL) * SL;
-          while (!mbar_try_wait(&c.bars[Cfg::BAR_FULL + slot], (last / SL) & 1) &&
-                 global_timer_ns() - t0 < 20000000ull) {
+          while (!mbar_try_wait(&c.bars[Cfg::BAR_FULL + slot], (last / SL) & 1) && global_timer_ns() - t0 < 20000000ull) {
           }
         }
       }
@@ -456,9 +538,9 @@ inline int sched_params(SchedParams* sp, const FwdParams& p, int head_dim, bool 
 }
 
 template <bool BF16, bool SOFTCAP>
-int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p,
-                            cudaStream_t stream) {
-  using Cfg = PersistCfg;
+int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
+                            const FwdParams& p, cudaStream_t stream) {
+  using Cfg = PersistCfg<SOFTCAP>;
   auto kern = attn_fwd_persist_kernel<BF16, SOFTCAP>;
   static thread_local int configured_dev = -1;
   int dev = 0;
@@ -471,7 +553,7 @@ int launch_attn_fwd_persist(const CUtensorMap& tq, const CUtensorMap& tk, const 
   const int rc = sched_params(&sp, p, Cfg::D, true);
   if (rc != B200_OK) return rc;
   const int grid = std::min(sp.total_items, Cfg::CTAS_PER_SM * sm_count());
-  B200_CUDA_TRY(launch_kernel(kern, grid, Cfg::THREADS_P, Cfg::SMEM_BYTES_P, stream, 1, tq, tk, tv, p, sp));
+  B200_CUDA_TRY(launch_kernel(kern, grid, Cfg::THREADS_P, Cfg::SMEM_BYTES_P, stream, 1, tq, tk, tv, to, p, sp));
   return B200_OK;
 }
 
