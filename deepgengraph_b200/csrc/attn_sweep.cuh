@@ -116,6 +116,12 @@ struct SweepCfg {
   static_assert(!GEN || MODE != SWEEP_COLSUM, "only the KeyFormer sweeps use noise");
   static constexpr bool NOISE = MODE != SWEEP_COLSUM && !GEN;   // noise TENSOR streamed through the auxiliary ring
   static constexpr bool LSE_IN = MODE != SWEEP_KF_ROWLSE;
+  // Ring depths of the streamed operand (XST) and of what the compute warps read (NST).  With a noise tensor the sweep is bound by its
+  // read, and what is in flight follows the noise stages: three of 32 KB beside one of the 16 KB operand (refilled as soon as its MMAs
+  // are done, more than a tile before it is needed again) just leave room for two CTAs per SM.
+  // KeyFormer calls with a noise tensor, two stages of each -> three and one (bf16, us): 2 x 32 heads, 2048 tokens 312.9 -> 305.5;
+  // 12 heads, 2048 tokens 109.9 -> 100.3; 32 heads, 1000 tokens 67.6 -> 62.7; 32 heads, 512 tokens 38.1 -> 36.5.
+  static constexpr int XST = NOISE ? 1 : STAGES, NST = NOISE ? 3 : STAGES;
   // BX = 64: the stationary tile lives in TMEM (64 columns beside the two 64-column product tiles) and is the
   // A operand of the MMAs, which then read only the streamed operand from shared memory -- with both operands
   // in shared memory the M128 x N64 MMAs ask for 192 B/clk of a 128 B/clk port, and every shared-memory access
@@ -127,7 +133,9 @@ struct SweepCfg {
   static constexpr int NOISE_BYTES = NOISE ? BM * BX * 4 : 0;
   static constexpr int LSE_BYTES = LSE_IN ? BX * 4 : 0;
   static constexpr int N_STAGE_BYTES = NOISE_BYTES + LSE_BYTES;       // auxiliary ring read by the compute warps
-  static constexpr int N_STAGE_STRIDE = (N_STAGE_BYTES + 1023) / 1024 * 1024;
+  static constexpr int N_STAGE_STRIDE = NOISE ? NOISE_BYTES : (N_STAGE_BYTES + 1023) / 1024 * 1024;
+  static constexpr int LSE_STRIDE = NOISE ? LSE_BYTES : N_STAGE_STRIDE;
+  static constexpr int LSE_RING_BYTES = NOISE ? NST * LSE_BYTES : 0;   // behind the noise stages; without noise a stage is its normalisers
   static constexpr int TMEM_COLS = A_TMEM ? 256 : 2 * BX;               // two product tiles (+ the stationary tile)
   static constexpr int COMPUTE_WARPS = 4 * CWG;
   static constexpr int THREADS = (COMPUTE_WARPS + 2) * 32;   // + TMA producer warp + MMA issuer warp
@@ -137,17 +145,19 @@ struct SweepCfg {
   static_assert(BX / 32 % CWG == 0, "every compute warpgroup takes whole 32-column chunks");
   static constexpr int BAR_A_FULL = 0;
   static constexpr int BAR_X_FULL = 1;
-  static constexpr int BAR_X_EMPTY = BAR_X_FULL + STAGES;
-  static constexpr int BAR_N_FULL = BAR_X_EMPTY + STAGES;
-  static constexpr int BAR_N_EMPTY = BAR_N_FULL + STAGES;
-  static constexpr int BAR_T_FULL = BAR_N_EMPTY + STAGES;   // [2]
+  static constexpr int BAR_X_EMPTY = BAR_X_FULL + XST;
+  static constexpr int BAR_N_FULL = BAR_X_EMPTY + XST;
+  static constexpr int BAR_N_EMPTY = BAR_N_FULL + NST;
+  static constexpr int BAR_T_FULL = BAR_N_EMPTY + NST;      // [2]
   static constexpr int BAR_T_EMPTY = BAR_T_FULL + 2;        // [2]
   static constexpr int BAR_DRAIN = BAR_T_EMPTY + 2;
   static constexpr int BAR_COMBINE = BAR_DRAIN + 1;         // second compute warpgroup's sums are in shared memory
   static constexpr int NUM_BARS = BAR_COMBINE + 1;
-  static constexpr int COMBINE_BYTES = CWG == 2 ? 2 * 128 * 4 : 0;   // second warpgroup's partial sums
-  static constexpr int SMEM_BYTES = A_BYTES + STAGES * X_STAGE_BYTES + STAGES * N_STAGE_STRIDE + COMBINE_BYTES +
-                                    NUM_BARS * 8 + 16 + 1024;
+  // second warpgroup's partial sums; with noise they take the place of the streamed operand, whose last MMA is over by then
+  static constexpr int COMBINE_BYTES = CWG == 2 && !NOISE ? 2 * 128 * 4 : 0;
+  static constexpr int SMEM_BYTES = A_BYTES + XST * X_STAGE_BYTES + NST * N_STAGE_STRIDE + LSE_RING_BYTES + COMBINE_BYTES +
+                                    NUM_BARS * 8 + 16;
+  static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 233472, "shared memory budget exceeded");   // 1 KB per CTA is reserved
 };
 
 template <class Cfg>
@@ -155,6 +165,7 @@ struct SweepCtx {
   uint8_t* sA;
   uint8_t* sX;
   uint8_t* sN;
+  uint8_t* sL;       // row normalisers, LSE_STRIDE bytes apart
   float* sCombine;   // [2][128], two compute warpgroups only
   uint64_t* bars;
   volatile int* abort_flag;
@@ -171,7 +182,7 @@ struct SweepCtx {
 template <class Cfg, bool GROUPED>
 __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const SweepParams& p, const CUtensorMap* tm_a,
                                                const CUtensorMap* tm_x, const CUtensorMap* tm_n) {
-  constexpr int ST = Cfg::STAGES, BX = Cfg::BX;
+  constexpr int XST = Cfg::XST, NST = Cfg::NST, BX = Cfg::BX;
   static_assert(!GROUPED || (Cfg::A_TMEM && !Cfg::NOISE), "grouped sweep: stationary tile in TMEM, no noise");
   if constexpr (!Cfg::A_TMEM) {
     mbar_expect_tx(&c.bars[Cfg::BAR_A_FULL], Cfg::A_BYTES);
@@ -186,27 +197,28 @@ __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const Swe
   const int n_items = (c.blk_hi - c.blk_lo) * group;
   for (int n = 0; n < n_items; ++n) {
     const int blk = c.blk_lo + (GROUPED ? n / group : n);
-    const int st = n % ST, use = n / ST;
+    const int xs = n % XST, xuse = n / XST;
     // head of the streamed operand, and the row of the normaliser table that goes with it
     const int x_head = GROUPED ? c.h * group + (n - (blk - c.blk_lo) * group)
                                : (Cfg::MODE == SWEEP_KF_ROWLSE ? c.h / p.kv_group : c.h);
     const int lse_row = GROUPED ? c.b * p.heads + x_head : c.bh;
-    if (use > 0 && !mbar_wait(&c.bars[Cfg::BAR_X_EMPTY + st], (use - 1) & 1, c.abort_flag, WAIT_X_EMPTY)) {
+    if (xuse > 0 && !mbar_wait(&c.bars[Cfg::BAR_X_EMPTY + xs], (xuse - 1) & 1, c.abort_flag, WAIT_X_EMPTY)) {
       ok = false;
       break;
     }
-    mbar_expect_tx(&c.bars[Cfg::BAR_X_FULL + st], Cfg::X_STAGE_BYTES);
+    mbar_expect_tx(&c.bars[Cfg::BAR_X_FULL + xs], Cfg::X_STAGE_BYTES);
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks)
-      tma_load_4d(c.sX + st * Cfg::X_STAGE_BYTES + ks * (BX * 128), tm_x, &c.bars[Cfg::BAR_X_FULL + st], ks * 64,
+      tma_load_4d(c.sX + xs * Cfg::X_STAGE_BYTES + ks * (BX * 128), tm_x, &c.bars[Cfg::BAR_X_FULL + xs], ks * 64,
                   x_head, blk * BX, c.b);
     if constexpr (Cfg::N_STAGE_BYTES > 0) {
+      const int st = n % NST, use = n / NST;
       if (use > 0 && !mbar_wait(&c.bars[Cfg::BAR_N_EMPTY + st], (use - 1) & 1, c.abort_flag, WAIT_N_EMPTY)) {
         ok = false;
         n_issued = n;  // X(n) issued, N(n) not
         break;
       }
-      uint8_t* dst = c.sN + st * Cfg::N_STAGE_STRIDE;
+      [[maybe_unused]] uint8_t* dst = c.sN + st * Cfg::N_STAGE_STRIDE;
       mbar_expect_tx(&c.bars[Cfg::BAR_N_FULL + st], Cfg::N_STAGE_BYTES);
       if constexpr (Cfg::NOISE) {
         // exp_rand viewed as a [B*H*q_len, kv_len] fp32 matrix; panels of 32 columns
@@ -229,7 +241,7 @@ __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const Swe
         const float* src = p.lse + (int64_t)lse_row * p.lse_stride + blk * BX;
         asm volatile(
             "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-            ::"r"(smem_u32(dst + Cfg::NOISE_BYTES)), "l"(src), "r"((uint32_t)Cfg::LSE_BYTES),
+            ::"r"(smem_u32(c.sL + st * Cfg::LSE_STRIDE)), "l"(src), "r"((uint32_t)Cfg::LSE_BYTES),
               "r"(smem_u32(&c.bars[Cfg::BAR_N_FULL + st]))
             : "memory");
       }
@@ -241,13 +253,15 @@ __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const Swe
     const uint64_t t0 = global_timer_ns();
     while (!mbar_try_wait(&c.bars[Cfg::BAR_A_FULL], 0) && global_timer_ns() - t0 < 20000000ull) {
     }
-    for (int st = 0; st < ST; ++st) {
-      const int u = (n_issued - 1 - st) >= 0 ? (n_issued - 1 - st) / ST : -1;
+    for (int st = 0; st < XST; ++st) {
+      const int u = (n_issued - 1 - st) >= 0 ? (n_issued - 1 - st) / XST : -1;
       while (u >= 0 && !mbar_try_wait(&c.bars[Cfg::BAR_X_FULL + st], u & 1) && global_timer_ns() - t0 < 20000000ull) {
       }
-      if constexpr (Cfg::N_STAGE_BYTES > 0) {
-        while (u >= 0 && !mbar_try_wait(&c.bars[Cfg::BAR_N_FULL + st], u & 1) &&
-               global_timer_ns() - t0 < 20000000ull) {
+    }
+    if constexpr (Cfg::N_STAGE_BYTES > 0) {
+      for (int st = 0; st < NST; ++st) {
+        const int u = (n_issued - 1 - st) >= 0 ? (n_issued - 1 - st) / NST : -1;
+        while (u >= 0 && !mbar_try_wait(&c.bars[Cfg::BAR_N_FULL + st], u & 1) && global_timer_ns() - t0 < 20000000ull) {
         }
       }
     }
@@ -259,7 +273,7 @@ __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const Swe
 // datapath); one elected lane issues.
 template <class Cfg, bool BF16>
 __device__ __forceinline__ void sweep_mma(const SweepCtx<Cfg>& c, int n_items) {
-  constexpr int ST = Cfg::STAGES, BX = Cfg::BX;
+  constexpr int ST = Cfg::XST, BX = Cfg::BX;
   constexpr uint32_t IDESC = make_idesc(BF16, 128, BX, false, false);
   const uint32_t desc_hi = smem_desc_hi(1024);
   const uint32_t a_lo = smem_desc_lo(smem_u32(c.sA), 16), x_lo = smem_desc_lo(smem_u32(c.sX), 16);
@@ -304,7 +318,7 @@ __device__ __forceinline__ void sweep_mma(const SweepCtx<Cfg>& c, int n_items) {
 // ------------------------- compute: per-key column sums -----------------------
 template <class Cfg, bool SOFTCAP, int AUX>
 __device__ __forceinline__ void sweep_compute_colsum(const SweepCtx<Cfg>& c, const SweepParams& p, int chunk) {
-  constexpr int ST = Cfg::STAGES, BX = Cfg::BX;
+  constexpr int ST = Cfg::NST, BX = Cfg::BX;
   constexpr bool KF = Cfg::MODE == SWEEP_KF_COLSUM;
   const int warp_q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   const int key = c.a0 + warp_q * 32 + lane;
@@ -405,7 +419,7 @@ __device__ __forceinline__ void sweep_compute_colsum(const SweepCtx<Cfg>& c, con
     tc_fence_after();
     if (tl_on) B200_TL(tl_base + 2);
     const uint8_t* nst = c.sN + st * Cfg::N_STAGE_STRIDE;
-    const float* lse_s = reinterpret_cast<const float*>(nst + Cfg::NOISE_BYTES);
+    const float* lse_s = reinterpret_cast<const float*>(c.sL + st * Cfg::LSE_STRIDE);
     const float* noise_col = reinterpret_cast<const float*>(nst + warp_q * (BX * 128)) + lane;  // + i * 32
     const int i0 = blk * BX;
     const int lo_c = i_lo - i0, hi_c = i_hi - i0;
@@ -479,7 +493,7 @@ __device__ __forceinline__ void sweep_compute_colsum(const SweepCtx<Cfg>& c, con
 // them into its accumulators after the last head of the group.
 template <class Cfg, bool SOFTCAP, int AUX>
 __device__ __forceinline__ void sweep_compute_colsum_grouped(const SweepCtx<Cfg>& c, const SweepParams& p, int chunk) {
-  constexpr int ST = Cfg::STAGES, BX = Cfg::BX;
+  constexpr int ST = Cfg::NST, BX = Cfg::BX;
   static_assert(BX == 64, "the grouped sweep keeps one 64-query block of running sums in registers");
   const int warp_q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   const int key = c.a0 + warp_q * 32 + lane;
@@ -505,7 +519,7 @@ __device__ __forceinline__ void sweep_compute_colsum_grouped(const SweepCtx<Cfg>
                                      mbar_wait(&c.bars[Cfg::BAR_N_FULL + st], (n / ST) & 1, c.abort_flag, WAIT_N_FULL)))
       return;
     tc_fence_after();
-    const float* lse_s = reinterpret_cast<const float*>(c.sN + st * Cfg::N_STAGE_STRIDE + Cfg::NOISE_BYTES);
+    const float* lse_s = reinterpret_cast<const float*>(c.sL + st * Cfg::LSE_STRIDE);
     const int i0 = blk * BX;
     const int lo_c = i_lo - i0, hi_c = i_hi - i0;
     const float keep = hh == 0 ? 0.f : 1.f;   // the first head of a group starts the running sums afresh
@@ -562,7 +576,7 @@ __device__ __forceinline__ void sweep_compute_colsum_grouped(const SweepCtx<Cfg>
 // --------------------- compute: per-query log-sum-exp of z --------------------
 template <class Cfg>
 __device__ __forceinline__ void sweep_compute_rowlse(const SweepCtx<Cfg>& c, const SweepParams& p) {
-  constexpr int ST = Cfg::STAGES, BX = Cfg::BX;
+  constexpr int ST = Cfg::NST, BX = Cfg::BX;
   const int warp_q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   const int r_local = warp_q * 32 + lane;
   const int row = c.a0 + r_local;
@@ -663,11 +677,7 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                   const __grid_constant__ CUtensorMap tm_n, const SweepParams p) {
   using Cfg = SweepCfg<MODE, BX, STAGES, CWG, GEN>;
   constexpr int CW = Cfg::COMPUTE_WARPS;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  // A launch that follows an expired wait on this device drains immediately (the status word stays
-  // set until the host reads it), so that one stuck kernel cannot stall a whole queue of launches.
-  __shared__ int s_skip;
+  extern __shared__ __align__(1024) uint8_t smem[];   // (no static shared memory: it starts at a multiple of 1024)
   // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
   // to allocate columns of its own, and what it wrote is visible only now.  It comes first of all, because a launch has several
   // waves of CTAs: those of the later ones load the word while they set up.
@@ -681,11 +691,14 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   SweepCtx<Cfg> c;
   c.sA = smem;
   c.sX = c.sA + Cfg::A_BYTES;
-  c.sN = c.sX + STAGES * Cfg::X_STAGE_BYTES;
-  c.sCombine = reinterpret_cast<float*>(c.sN + STAGES * Cfg::N_STAGE_STRIDE);
-  c.bars = reinterpret_cast<uint64_t*>(c.sN + STAGES * Cfg::N_STAGE_STRIDE + Cfg::COMBINE_BYTES);
+  c.sN = c.sX + Cfg::XST * Cfg::X_STAGE_BYTES;
+  c.sL = Cfg::NOISE ? c.sN + Cfg::NST * Cfg::N_STAGE_STRIDE : c.sN;
+  uint8_t* behind = c.sN + Cfg::NST * Cfg::N_STAGE_STRIDE + Cfg::LSE_RING_BYTES;
+  c.sCombine = reinterpret_cast<float*>(Cfg::NOISE ? c.sX : behind);
+  c.bars = reinterpret_cast<uint64_t*>(behind + Cfg::COMBINE_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c.bars + Cfg::NUM_BARS);
   c.abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* s_skip = reinterpret_cast<volatile int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunk = blockIdx.z;
@@ -725,7 +738,7 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll
     for (int i = 0; i < Cfg::NUM_BARS; ++i) {
       // arrivals per phase: every compute warp releases a product buffer / an auxiliary stage
-      const bool warp_count = (i >= Cfg::BAR_N_EMPTY && i < Cfg::BAR_N_EMPTY + STAGES) ||
+      const bool warp_count = (i >= Cfg::BAR_N_EMPTY && i < Cfg::BAR_N_EMPTY + Cfg::NST) ||
                               (i >= Cfg::BAR_T_EMPTY && i < Cfg::BAR_T_EMPTY + 2);
       const bool four = (Cfg::A_TMEM && i == Cfg::BAR_A_FULL) || i == Cfg::BAR_COMBINE;
       mbar_init(&c.bars[i], warp_count ? (uint32_t)Cfg::COMPUTE_WARPS : four ? 4u : 1u);
@@ -742,12 +755,14 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
-  if (threadIdx.x == 0) s_skip = status_now;
+  if (threadIdx.x == 0) *s_skip = status_now;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   c.tmem_base = *tmem_slot;
-  if (s_skip != 0) {
+  // A launch that follows an expired wait on this device drains immediately (the status word stays
+  // set until the host reads it), so that one stuck kernel cannot stall a whole queue of launches.
+  if (*s_skip != 0) {
     if (warp == 0) tmem_dealloc(c.tmem_base, Cfg::TMEM_COLS);
     return;
   }
@@ -856,8 +871,7 @@ constexpr int kSweepChunkBlocks = B200_SWEEP_CHUNK;
 #ifndef B200_COLSUM_STAGES
 #define B200_COLSUM_STAGES 2
 #endif
-// KeyFormer sweeps: two ring stages of 8 KB (streamed operand) + 32 KB (noise) keep a CTA at 83 KB of shared memory, so
-// that two CTAs share an SM (measured at config 4: 430 -> 322 us against three stages and one CTA per SM)
+// ring stages of the KeyFormer sweeps without a noise tensor and of the grouped sweep (with one: SweepCfg)
 #ifndef B200_KF_STAGES
 #define B200_KF_STAGES 2
 #endif
