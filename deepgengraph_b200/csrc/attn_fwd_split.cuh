@@ -2,15 +2,19 @@
 //   warps 0-3, 4-7   softmax: warpgroup h takes keys [64 h, 64 h + 64) of every block; thread = row = TMEM lane
 //   warp  8          TMA producer of Q, K and V, tile scheduler
 //   warp  9          MMA issuer: S = Q K^T (operands in shared memory), O += P V (P read from TMEM)
-// TMEM (512 columns): two S buffers of 128 (the 16-bit P of a thread's 64 keys overwrites the first half of its own 64 columns), O 256.
+// TMEM (512 columns): S 128, two buffers of 64 for the 16-bit P, O 256.
 //
 // What bounds it and why this shape.  Per block of 128 keys the tensor pipe needs 16 x 64 clk for S and 8 x 128 for P V, 2048 in all,
 // the special-function unit 1024; a block takes 3130 clk with the soft-cap and 2900 without (a launch of 85.6 blocks per SM, everything
-// included): no pipe is full, the chain S -> softmax -> P -> P V of one tile is what is left.  With 64-key blocks and one softmax
+// included): no pipe is full, the chain S -> softmax -> P -> P V of one tile is what is left, and in long launches the power limit.
+// S is free as soon as the softmax warps have it in registers, so that S(n+1) is computed under the softmax of block n and before
+// P V(n).  With two S buffers, in which P took S's place, S(n+2) had to wait for P V(n) (us, before -> now, bf16, no soft-cap): 16/8 heads,
+// causal, 1024 tokens 18.23 -> 18.02, 4096 tokens 110.5 -> 106.5, 8192 tokens 405.2 -> 398.7; 500 queries on 4000 keys, 32/8 heads 50.9 ->
+// 49.9; 4 x 1500 tokens 80.5 -> 78.9; with the soft-cap, where the softmax is longer, equal.  With 64-key blocks and one softmax
 // warpgroup a block cost every hand-over of that chain twice as often, and one warp per SM sub-partition could not keep up with the
-// soft-cap.  S with N = 128 runs at the full rate with Q in shared memory (N = 64: 48 instead of 32 clk), so Q needs no TMEM and both S
-// buffers hold 128 keys.
-// Measured, 64-key blocks -> now (one box, bf16, us, idle GPU): 16/8 heads, 8192 tokens, window 4096, soft-cap 50: 376 -> 330; 500 queries
+// soft-cap.  S with N = 128 runs at the full rate with Q in shared memory (N = 64: 48 instead of 32 clk), so Q needs no TMEM and S
+// holds 128 keys.
+// Measured, 64-key blocks -> 128-key blocks (one box, bf16, us, idle GPU): 16/8 heads, 8192 tokens, window 4096, soft-cap 50: 376 -> 330; 500 queries
 // on 4000 keys, 32/8 heads: 52.4 -> 50.7, with soft-cap 64.9 -> 53.8; 16/8 heads, causal, 8192 tokens 402 -> 391, 1024 tokens 19.1 -> 18.3,
 // with soft-cap 23.0 -> 19.7, 64 tokens 6.6 -> 6.7.  In a loop under the power cap: window 4096, soft-cap 447 -> 396.
 #pragma once
@@ -21,22 +25,23 @@
 namespace b200 {
 
 struct SplitCfg {
-  static constexpr int D = 256, BM = 128, BN = 128, SB = 2;
+  static constexpr int D = 256, BM = 128, BN = 128, PB = 2;   // PB: P buffers
   static constexpr int COLS = BN / 2;                // keys of a softmax thread
   static constexpr int KSUB = D / 64;                // 64-element (128-byte) column blocks of a row
   static constexpr int Q_TILE_BYTES = BM * D * 2;
   // One ring of 32 KB stages.  A K block is two stages of 128 keys x 128 dims, a V block two of 64 keys x 256 dims: each stage is a
   // complete operand of a run of eight (four) MMAs.
   static constexpr int STAGE_BYTES = 32768, PARTS = 2, V_KEYS = BN / PARTS, SLOTS = 5;
-  static constexpr int O_COL = SB * BN, TMEM_COLS = 512;
+  static constexpr int P_COL = BN, O_COL = P_COL + PB * BN / 2, TMEM_COLS = 512;
   static_assert(O_COL + D == TMEM_COLS, "TMEM plan");
   static constexpr int SOFTMAX_WARPS = 8, PRODUCER_WARP = 8, THREADS = 320;
   // barriers
   static constexpr int BAR_Q_FULL = 0;
   static constexpr int BAR_Q_FREE = 1;                       // last S of a tile retired
-  static constexpr int BAR_S_FULL = 2;                       // [SB]
-  static constexpr int BAR_P_FULL = BAR_S_FULL + SB;         // [SB] eight softmax warps
-  static constexpr int BAR_O_FULL = BAR_P_FULL + SB;         // [2] P V of block g completes barrier g % 2
+  static constexpr int BAR_S_FULL = 2;
+  static constexpr int BAR_S_FREE = 3;                       // S is in the registers of the eight softmax warps
+  static constexpr int BAR_P_FULL = 4;                       // [PB] eight softmax warps
+  static constexpr int BAR_O_FULL = BAR_P_FULL + PB;         // [2] P V of block g completes barrier g % 2
   static constexpr int BAR_FULL = BAR_O_FULL + 2;            // [SLOTS]
   static constexpr int BAR_EMPTY = BAR_FULL + SLOTS;         // [SLOTS]
   static constexpr int BAR_SCHED = BAR_EMPTY + SLOTS;        // [2] item of slot k % 2 published
@@ -104,7 +109,7 @@ __device__ __forceinline__ bool pair_vote(int id, bool pred) {
 template <bool BF16, bool SOFTCAP>
 struct SplitSoftmax {
   using Cfg = SplitCfg;
-  static constexpr int D = Cfg::D, COLS = Cfg::COLS, SB = Cfg::SB;
+  static constexpr int D = Cfg::D, COLS = Cfg::COLS, PB = Cfg::PB;
   const SplitCtx& c;
   const FwdParams& p;
   const int half, warp_q, lane, bar_id;
@@ -159,11 +164,18 @@ struct SplitSoftmax {
     if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_P_FULL + buf]);
   }
 
+  __device__ __forceinline__ void release_s() const {
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&c.bars[Cfg::BAR_S_FREE]);
+  }
+
   // A half block of the second warpgroup: no keys, but its half of O moves with the maximum.
   __device__ __forceinline__ bool block_without_keys(int n, int g) {
-    const int buf = g % SB;
-    const bool ok = c.wait(Cfg::BAR_S_FULL + buf, g / SB, WAIT_S_FULL);
+    const int buf = g % PB;
+    const bool ok = c.wait(Cfg::BAR_S_FULL, g, WAIT_S_FULL);
     tc_fence_after();
+    release_s();
     if (!agree(n, g, ok, -INFINITY)) return false;
     deliver(buf);
     return true;
@@ -172,20 +184,21 @@ struct SplitSoftmax {
   // One block of one row.  `g` counts the CTA's blocks, n those of the tile.  False: leave (no further step).
   template <bool MASK>
   __device__ __forceinline__ bool block(int n, int g, int lo_c, int hi_c, float cmul) {
-    const int buf = g % SB;
-    const uint32_t s_addr = lane_addr + buf * Cfg::BN + half * COLS;
-    const bool ok = c.wait(Cfg::BAR_S_FULL + buf, g / SB, WAIT_S_FULL);
+    const int buf = g % PB;
+    const uint32_t s_addr = lane_addr + half * COLS;
+    const uint32_t p_addr = lane_addr + Cfg::P_COL + buf * (Cfg::BN / 2) + half * (COLS / 2);
+    const bool ok = c.wait(Cfg::BAR_S_FULL, g, WAIT_S_FULL);
     tc_fence_after();
     uint32_t sr[COLS / 32][32];
 #pragma unroll
     for (int ch = 0; ch < COLS / 32; ++ch) tmem_ld32(s_addr + ch * 32, sr[ch]);
     tmem_ld_wait();
+    release_s();
 
     bool cap_poly_only = false;
     const float m_blk = row_maximum<SOFTCAP, MASK, COLS>(sr, lo_c, hi_c, p, cmul, cap_poly_only);
     if (!agree(n, g, ok, m_blk)) return false;
-    // P over the first half of the thread's own S columns
-    l += row_exponentials<BF16, SOFTCAP, MASK, COLS>(sr, s_addr, lo_c, hi_c, p, cmul, m, cap_poly_only);
+    l += row_exponentials<BF16, SOFTCAP, MASK, COLS>(sr, p_addr, lo_c, hi_c, p, cmul, m, cap_poly_only);
     deliver(buf);
     return true;
   }
@@ -239,7 +252,7 @@ struct SplitSoftmax {
 };
 
 // ------------------------------- TMA producer -------------------------------
-// One thread.  Ring stages in the order the issuer consumes them: K(0 .. SB-1), then V(n), K(n+SB) for n = 0, 1, ...
+// One thread.  Ring stages in the order the issuer consumes them: K(0), then K(n+1), V(n) for n = 0, 1, ...
 template <bool PERSISTENT>
 __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                                                const CUtensorMap* tm_v, const FwdParams& p, const SchedParams& sp) {
@@ -308,10 +321,10 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
         ++ring_i;
       }
     };
-    for (int n = 0; n < Cfg::SB && n < nb && ok; ++n) load(false, n);
+    load(false, 0);
     for (int n = 0; n < nb && ok; ++n) {
-      load(true, n);
-      if (ok && n + Cfg::SB < nb) load(false, n + Cfg::SB);
+      if (n + 1 < nb) load(false, n + 1);
+      if (ok) load(true, n);
     }
   }
   if (!ok || *c.abort_flag != 0) {
@@ -331,13 +344,15 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
 
 // -------------------------------- MMA issuer --------------------------------
 // One warp, an elected lane issues (umma_ss_if):
-//   softmax(n) -> P -> [O += P V(n)] -> [S(n+SB) = Q K(n+SB)^T] -> softmax(n+SB)
+//   [S(n+1) = Q K(n+1)^T] [O += P V(n)] [S(n+2)] ...
+// S(n+1) needs only S(n) in the softmax warps' registers, so it is there when they are done with block n.  P V(n) stays before S(n+2):
+// a softmax warp that sees S(n+2) may overwrite P(n).
 // The control flow is convergent unless a wait runs out: then one lane may have seen the abort flag and another the barrier's phase.
 // Inside of a tile nothing waits for the whole warp, and `ok` is voted on at the end of each tile, so all lanes leave together.
 template <bool BF16>
 __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams& p, const SchedParams& sp, int lane) {
   using Cfg = SplitCfg;
-  constexpr int SL = Cfg::SLOTS, D = Cfg::D, BN = Cfg::BN, BM = Cfg::BM, SB = Cfg::SB, PARTS = Cfg::PARTS;
+  constexpr int SL = Cfg::SLOTS, D = Cfg::D, BN = Cfg::BN, BM = Cfg::BM, PB = Cfg::PB, PARTS = Cfg::PARTS;
   constexpr uint32_t IDESC_PV = make_idesc(BF16, BM, D, false, true);
   // descriptor halves: the upper word is constant, the lower word is (address >> 4) plus a compile-time step
   const uint32_t desc_hi = smem_desc_hi(1024);
@@ -354,11 +369,12 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
   using Half = std::integral_constant<int, 1>;
   auto issue_s = [&](auto parts_tag, int gb, bool last_of_tile) {
     constexpr uint32_t IDESC_S = make_idesc(BF16, BM, Cfg::V_KEYS * decltype(parts_tag)::value, false, false);
-    const uint32_t s_tmem = c.tmem_base + (gb % SB) * BN;
+    const uint32_t s_tmem = c.tmem_base;
 #pragma unroll
     for (int part = 0; part < PARTS; ++part) {
       const int slot = ring_i % SL;
       if (ok) ok = wait_full(ring_i, WAIT_K_FULL);
+      if (part == 0 && ok && gb > 0) ok = c.wait(Cfg::BAR_S_FREE, gb - 1, WAIT_S_FREE);
       ++ring_i;
       if (!ok) return;
       tc_fence_after();
@@ -370,21 +386,21 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
         const uint32_t b_off = (uint32_t)(((kk / 4) * (BN * 128) + (kk % 4) * 32) >> 4);
         umma_ss_if<IDESC_S>(elected, s_tmem, q_lo + a_off, b0 + b_off, desc_hi, ka == 0 ? 0u : 1u);
       }
-      if (part == PARTS - 1) umma_commit_if(elected, bars + 8 * (Cfg::BAR_S_FULL + gb % SB));
+      if (part == PARTS - 1) umma_commit_if(elected, bars + 8 * Cfg::BAR_S_FULL);
       umma_commit_if(elected, bars + 8 * (Cfg::BAR_EMPTY + slot));
       if (part == PARTS - 1 && last_of_tile) umma_commit_if(elected, bars + 8 * Cfg::BAR_Q_FREE);   // no later MMA reads this Q
     }
   };
   auto issue_pv = [&](auto parts_tag, int gb, bool first_of_tile) {
     constexpr int parts = decltype(parts_tag)::value;
-    const uint32_t p_tmem = c.tmem_base + (gb % SB) * BN;
+    const uint32_t p_tmem = c.tmem_base + Cfg::P_COL + (gb % PB) * (BN / 2);
 #pragma unroll
-    for (int part = 0; part < parts; ++part) {   // part = half: keys [64 part, 64 part + 64), P in columns [64 part, 64 part + 32)
+    for (int part = 0; part < parts; ++part) {   // part = half: keys [64 part, 64 part + 64), P in columns [32 part, 32 part + 32)
       const int slot = (ring_i + part) % SL;
       const uint32_t b0 = v_lo + (uint32_t)(slot * (Cfg::STAGE_BYTES >> 4));
 #pragma unroll
       for (int kk = 0; kk < Cfg::V_KEYS / 16; ++kk) {
-        const uint32_t a = p_tmem + part * Cfg::COLS + kk * 8, b = b0 + (uint32_t)(kk * (2048 >> 4));
+        const uint32_t a = p_tmem + part * (Cfg::COLS / 2) + kk * 8, b = b0 + (uint32_t)(kk * (2048 >> 4));
         umma_ts_if<IDESC_PV>(elected, o_tmem, a, b, desc_hi, (part == 0 && kk == 0 && first_of_tile) ? 0u : 1u);
       }
       umma_commit_if(elected, bars + 8 * (Cfg::BAR_EMPTY + slot));
@@ -399,7 +415,7 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
 #pragma unroll
     for (int part = 0; part < parts; ++part)
       if (ok) ok = wait_full(ring_i + part, WAIT_V_FULL);
-    if (ok) ok = c.wait(Cfg::BAR_P_FULL + gb % SB, gb / SB, WAIT_P_FULL);
+    if (ok) ok = c.wait(Cfg::BAR_P_FULL + gb % PB, gb / PB, WAIT_P_FULL);
     if (!ok) return;
     tc_fence_after();
     issue_pv(parts_tag, gb, first_of_tile);
@@ -415,13 +431,14 @@ __device__ __forceinline__ void split_issuer(const SplitCtx& c, const FwdParams&
     const SplitBlocks blocks(t);
     const int nb = blocks.count, whole = nb - (blocks.half_last ? 1 : 0);
     ok = c.wait(Cfg::BAR_Q_FULL, k, WAIT_Q_FULL);
-    for (int n = 0; n < SB && n < whole && ok; ++n) issue_s(Whole{}, g0 + n, n == nb - 1);
-    if (whole < nb && whole < SB && ok) issue_s(Half{}, g0 + whole, true);
-    for (int n = 0; n < whole && ok; ++n) {
-      step_pv(Whole{}, g0 + n, n == 0);
-      if (ok && n + SB < nb) issue_s(Whole{}, g0 + n + SB, n + SB == nb - 1);
+    if (whole > 0 && ok) issue_s(Whole{}, g0, nb == 1);
+    for (int n = 0; n + 1 < whole && ok; ++n) {
+      issue_s(Whole{}, g0 + n + 1, n + 2 == nb);
+      if (ok) step_pv(Whole{}, g0 + n, n == 0);
     }
-    // A half block by itself, so that the loop has no more to decide (there its S is computed whole, from keys that no row sees).
+    // The last whole block and the half block are not in the loop, so that it has no more to decide.
+    if (whole < nb && ok) issue_s(Half{}, g0 + whole, true);
+    if (whole > 0 && ok) step_pv(Whole{}, g0 + whole - 1, whole == 1);
     if (whole < nb && ok) step_pv(Half{}, g0 + whole, whole == 0);
     ok = __all_sync(0xffffffffu, ok);
     g0 += nb;
@@ -451,9 +468,9 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int i = 0; i < Cfg::NUM_BARS; ++i) {
-      const bool p_full = i >= Cfg::BAR_P_FULL && i < Cfg::BAR_P_FULL + Cfg::SB;
+      const bool p_full = i >= Cfg::BAR_P_FULL && i < Cfg::BAR_P_FULL + Cfg::PB;
       const bool sched_free = i >= Cfg::BAR_SCHED_FREE && i < Cfg::BAR_SCHED_FREE + 2;
-      mbar_init(&c.bars[i], p_full ? (uint32_t)Cfg::SOFTMAX_WARPS : sched_free ? (uint32_t)Cfg::SOFTMAX_WARPS + 1u : 1u);
+      mbar_init(&c.bars[i], p_full || i == Cfg::BAR_S_FREE ? (uint32_t)Cfg::SOFTMAX_WARPS : sched_free ? (uint32_t)Cfg::SOFTMAX_WARPS + 1u : 1u);
     }
     *c.abort_flag = 0;
     fence_mbar_init();

@@ -105,7 +105,8 @@ enum WaitCode : int {
   WAIT_TURN = 16,     // exp-phase turn-taking between the two query tiles
   WAIT_SELFTEST = 17, // b200_selftest_bounded_wait
   WAIT_SCHED = 18,    // persistent attention: next tile descriptor
-  WAIT_Q_FREE = 19    // persistent attention: Q buffer released by the previous tile
+  WAIT_Q_FREE = 19,   // persistent attention: Q buffer released by the previous tile
+  WAIT_S_FREE = 20    // attention at head_dim 256: S in the softmax warps' registers
 };
 
 // ---------------------------------------------------------------------------
