@@ -33,13 +33,6 @@ enum SweepMode : int { SWEEP_COLSUM = 0, SWEEP_KF_COLSUM = 1, SWEEP_KF_ROWLSE = 
 // second per-key statistic of the column-sum sweep: none, sum of p^2 (RoCo), or the Corm flag
 enum SweepAux : int { AUX_NONE = 0, AUX_SQUARES = 1, AUX_CORM = 2 };
 
-// Of every 8 groups of 4 columns of an unmasked block, this many take their exponentials from the FMA-pipe
-// polynomial instead of the special-function unit (column-sum sweeps).
-#ifndef B200_SWEEP_POLY_OF_8
-#define B200_SWEEP_POLY_OF_8 0
-#endif
-constexpr int kSweepPolyOf8 = B200_SWEEP_POLY_OF_8;
-
 // ---------------------------------------------------------------------------------------------
 // In-kernel noise for the KeyFormer sweeps (no counterpart in the reference, whose modules take the noise as a
 // [B, H, Sq, Skv] fp32 tensor, kernels/kf.py:19,36-37, drawn by the caller, kf.py:48 / models/kf.py:44).
@@ -339,17 +332,19 @@ __device__ __forceinline__ void sweep_compute_colsum(const SweepCtx<Cfg>& c, con
                         const float* noise_col, int lo_c, int hi_c, float qbase, int i0) {
     constexpr bool MASK = decltype(mask_tag)::value;
     [[maybe_unused]] constexpr bool cap_poly_only = decltype(cap_tag)::value;
-    const float2 c2 = make_float2(cmul, cmul);
+    // The negative exponents are formed: L (and the logarithm of the noise) are then operands as they are, and the sign is a modifier
+    // of the exponential.  Packed operands have none: negating them costs an instruction per element.
+    const float2 c2 = make_float2(-cmul, -cmul);
 #pragma unroll
     for (int i = 0; i < 32; i += 4) {
       const float4 L = *reinterpret_cast<const float4*>(lse_s + ch * 32 + i);
       float sv[4] = {__uint_as_float(sr[i]), __uint_as_float(sr[i + 1]), __uint_as_float(sr[i + 2]),
                      __uint_as_float(sr[i + 3])};
       if constexpr (SOFTCAP) softcap4(sv, p.cap_in, p.cap_out, cap_poly_only);
-      float2 e0, e1;
+      float2 e0, e1;   // -(exponents)
       if constexpr (KF) {
         const float2 it2 = make_float2(p.inv_tau, p.inv_tau);
-        float g[4];
+        float g[4];   // log2 of the noise
         if constexpr (Cfg::GEN) {
           // One generator call yields the noise of ONE query against four consecutive keys, while this thread needs
           // one key against four consecutive queries: the four lanes of a quad (keys 4k .. 4k+3) each generate one of
@@ -363,29 +358,18 @@ __device__ __forceinline__ void sweep_compute_colsum(const SweepCtx<Cfg>& c, con
           for (int sft = 0; sft < 4; ++sft) r[sft] = __shfl_sync(0xffffffffu, o[sft], (lane & ~3) | (int)(cpos ^ sft));
           xor_permute4(r, cpos);
 #pragma unroll
-          for (int u = 0; u < 4; ++u) g[u] = -kf_gen_log2_exp_rand(r[u]);
+          for (int u = 0; u < 4; ++u) g[u] = kf_gen_log2_exp_rand(r[u]);
         } else {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) g[u] = -lg2_approx(noise_col[(ch * 32 + i + u) * 32]);
+          for (int u = 0; u < 4; ++u) g[u] = lg2_approx(noise_col[(ch * 32 + i + u) * 32]);
         }
-        e0 = ffma2(ffma2(make_float2(sv[0], sv[1]), c2, make_float2(g[0], g[1])), it2, make_float2(-L.x, -L.y));
-        e1 = ffma2(ffma2(make_float2(sv[2], sv[3]), c2, make_float2(g[2], g[3])), it2, make_float2(-L.z, -L.w));
+        e0 = ffma2(ffma2(make_float2(sv[0], sv[1]), c2, make_float2(g[0], g[1])), it2, make_float2(L.x, L.y));
+        e1 = ffma2(ffma2(make_float2(sv[2], sv[3]), c2, make_float2(g[2], g[3])), it2, make_float2(L.z, L.w));
       } else {
-        e0 = ffma2(make_float2(sv[0], sv[1]), c2, make_float2(-L.x, -L.y));
-        e1 = ffma2(make_float2(sv[2], sv[3]), c2, make_float2(-L.z, -L.w));
+        e0 = ffma2(make_float2(sv[0], sv[1]), c2, make_float2(L.x, L.y));
+        e1 = ffma2(make_float2(sv[2], sv[3]), c2, make_float2(L.z, L.w));
       }
-      float pr[4];
-      // A fixed, interleaved subset of the column groups of unmasked blocks takes its exponentials from the cubic
-      // polynomial on the FMA pipe (exp2_poly2, relative error 7.5e-5): the sweep issues one exponential per
-      // element and nothing else of weight, so the special-function unit (16 results per clock per SM) is its
-      // bound; the share is kSweepPolyOf8 / 8.
-      if (!MASK && (((i / 4) * kSweepPolyOf8) % 8) < kSweepPolyOf8) {
-        e0 = exp2_poly2(e0);
-        e1 = exp2_poly2(e1);
-        pr[0] = e0.x, pr[1] = e0.y, pr[2] = e1.x, pr[3] = e1.y;
-      } else {
-        pr[0] = ex2_approx(e0.x), pr[1] = ex2_approx(e0.y), pr[2] = ex2_approx(e1.x), pr[3] = ex2_approx(e1.y);
-      }
+      float pr[4] = {ex2_approx(-e0.x), ex2_approx(-e0.y), ex2_approx(-e1.x), ex2_approx(-e1.y)};
       if constexpr (MASK) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -584,6 +568,7 @@ __device__ __forceinline__ void sweep_compute_rowlse(const SweepCtx<Cfg>& c, con
   const float cz = p.scale_log2 * p.inv_tau;
   float m = -1.0e30f, l = 0.f;
   const int hi_key = p.causal ? min(row + p.delta, p.kv_len - 1) : p.kv_len - 1;
+  const int hi_first = p.causal ? min(c.a0 + p.delta, p.kv_len - 1) : p.kv_len - 1;   // of the tile's first row
   // with two compute warpgroups each takes half of the block's key columns: a row's running (maximum, sum) is then
   // split over two threads and merged once at the end
   constexpr int NCH = BX / 32 / Cfg::CWG;
@@ -599,14 +584,16 @@ __device__ __forceinline__ void sweep_compute_rowlse(const SweepCtx<Cfg>& c, con
     [[maybe_unused]] const uint8_t* nst = c.sN + st * Cfg::N_STAGE_STRIDE;
     const int hi_c = hi_key - blk * BX;
     float z[NCH * 32];
-    float mx = -INFINITY;
-#pragma unroll
-    for (int cc = 0; cc < NCH; ++cc) {
+    float mx0 = -INFINITY, mx1 = -INFINITY;
+    // z = x / tau - log2(noise) / tau of 32 keys; MASK: some row of the tile does not see all of the block's keys
+    auto chunk = [&](auto mask_tag, int cc) {
+      constexpr bool MASK = decltype(mask_tag)::value;
       const int ch = ch0 + cc;
       uint32_t sr[32];
       tmem_ld32(lane_addr + tb * BX + ch * 32, sr);
       tmem_ld_wait();
       [[maybe_unused]] const uint8_t* panel = nst + ch * (128 * 128) + r_local * 128;
+      const float2 cz2 = make_float2(cz, cz), nit2 = make_float2(-p.inv_tau, -p.inv_tau);
 #pragma unroll
       for (int q4 = 0; q4 < 8; ++q4) {
         float lg[4];   // log2(exp_rand) of this query against four consecutive keys
@@ -620,15 +607,30 @@ __device__ __forceinline__ void sweep_compute_rowlse(const SweepCtx<Cfg>& c, con
           const float4 er = *reinterpret_cast<const float4*>(panel + ((q4 ^ (r_local & 7)) << 4));
           lg[0] = lg2_approx(er.x), lg[1] = lg2_approx(er.y), lg[2] = lg2_approx(er.z), lg[3] = lg2_approx(er.w);
         }
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u += 2) {
+          const float2 x = make_float2(__uint_as_float(sr[q4 * 4 + u]), __uint_as_float(sr[q4 * 4 + u + 1]));
+          const float2 r = ffma2(x, cz2, fmul2(make_float2(lg[u], lg[u + 1]), nit2));
+          v[u] = r.x, v[u + 1] = r.y;
+        }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int col = ch * 32 + q4 * 4 + u;
-          float v = fmaf(__uint_as_float(sr[q4 * 4 + u]), cz, -lg[u] * p.inv_tau);
-          if (col > hi_c) v = -INFINITY;
-          z[cc * 32 + q4 * 4 + u] = v;
-          mx = fmaxf(mx, v);
+          if constexpr (MASK)
+            if (ch * 32 + q4 * 4 + u > hi_c) v[u] = -INFINITY;
+          z[cc * 32 + q4 * 4 + u] = v[u];
         }
+        mx0 = fmax3(mx0, v[0], v[1]);
+        mx1 = fmax3(mx1, v[2], v[3]);
       }
+    };
+    const bool need_mask = hi_first < blk * BX + BX - 1;
+#pragma unroll
+    for (int cc = 0; cc < NCH; ++cc) {
+      if (need_mask)
+        chunk(std::true_type{}, cc);
+      else
+        chunk(std::false_type{}, cc);
     }
     tc_fence_before();
     __syncwarp();
@@ -636,13 +638,15 @@ __device__ __forceinline__ void sweep_compute_rowlse(const SweepCtx<Cfg>& c, con
       mbar_arrive(&c.bars[Cfg::BAR_T_EMPTY + tb]);
       if constexpr (Cfg::N_STAGE_BYTES > 0) mbar_arrive(&c.bars[Cfg::BAR_N_EMPTY + st]);
     }
-    const float m_new = fmaxf(m, mx);
-    float s0 = 0.f, s1 = 0.f;
+    const float m_new = fmaxf(m, fmaxf(mx0, mx1));
+    const float2 nm2 = make_float2(-m_new, -m_new);
+    float2 sum = make_float2(0.f, 0.f);   // of the even and of the odd keys
 #pragma unroll
     for (int i = 0; i < NCH * 32; i += 2) {
-      s0 += ex2_approx(z[i] - m_new);
-      s1 += ex2_approx(z[i + 1] - m_new);
+      const float2 e = fadd2(make_float2(z[i], z[i + 1]), nm2);
+      sum = fadd2(sum, make_float2(ex2_approx(e.x), ex2_approx(e.y)));
     }
+    const float s0 = sum.x, s1 = sum.y;
     l = l * ex2_approx(m - m_new) + (s0 + s1);
     m = m_new;
   }
