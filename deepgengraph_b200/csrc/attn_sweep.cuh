@@ -184,8 +184,7 @@ __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const Swe
       tma_load_4d(c.sA + ks * (Cfg::BM * 128), tm_a, &c.bars[Cfg::BAR_A_FULL], ks * 64,
                   Cfg::MODE == SWEEP_KF_ROWLSE ? c.h : c.h / p.kv_group, c.a0, c.b);
   }
-  bool ok = true;
-  int n_issued = 0;
+  int x_issued = 0, n_issued = 0;   // items whose streamed operand, and whose noise and normalisers, are on their way
   const int group = GROUPED ? p.kv_group : 1;
   const int n_items = (c.blk_hi - c.blk_lo) * group;
   for (int n = 0; n < n_items; ++n) {
@@ -195,22 +194,17 @@ __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const Swe
     const int x_head = GROUPED ? c.h * group + (n - (blk - c.blk_lo) * group)
                                : (Cfg::MODE == SWEEP_KF_ROWLSE ? c.h / p.kv_group : c.h);
     const int lse_row = GROUPED ? c.b * p.heads + x_head : c.bh;
-    if (xuse > 0 && !mbar_wait(&c.bars[Cfg::BAR_X_EMPTY + xs], (xuse - 1) & 1, c.abort_flag, WAIT_X_EMPTY)) {
-      ok = false;
+    if (xuse > 0 && !mbar_wait(&c.bars[Cfg::BAR_X_EMPTY + xs], (xuse - 1) & 1, c.abort_flag, WAIT_X_EMPTY))
       break;
-    }
     mbar_expect_tx(&c.bars[Cfg::BAR_X_FULL + xs], Cfg::X_STAGE_BYTES);
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks)
       tma_load_4d(c.sX + xs * Cfg::X_STAGE_BYTES + ks * (BX * 128), tm_x, &c.bars[Cfg::BAR_X_FULL + xs], ks * 64,
                   x_head, blk * BX, c.b);
+    x_issued = n + 1;
     if constexpr (Cfg::N_STAGE_BYTES > 0) {
       const int st = n % NST, use = n / NST;
-      if (use > 0 && !mbar_wait(&c.bars[Cfg::BAR_N_EMPTY + st], (use - 1) & 1, c.abort_flag, WAIT_N_EMPTY)) {
-        ok = false;
-        n_issued = n;  // X(n) issued, N(n) not
-        break;
-      }
+      if (use > 0 && !mbar_wait(&c.bars[Cfg::BAR_N_EMPTY + st], (use - 1) & 1, c.abort_flag, WAIT_N_EMPTY)) break;
       [[maybe_unused]] uint8_t* dst = c.sN + st * Cfg::N_STAGE_STRIDE;
       mbar_expect_tx(&c.bars[Cfg::BAR_N_FULL + st], Cfg::N_STAGE_BYTES);
       if constexpr (Cfg::NOISE) {
@@ -241,13 +235,15 @@ __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const Swe
     }
     n_issued = n + 1;
   }
-  if (!ok || *c.abort_flag != 0) {
-    // abort path: let our own bulk copies land before the CTA exits (bounded, 20 ms)
+  // Our own bulk copies land before the CTA exits (bounded, 20 ms): nobody else waits for them after a wait that ran out, or where the
+  // launch drains.
+  {
     const uint64_t t0 = global_timer_ns();
-    while (!mbar_try_wait(&c.bars[Cfg::BAR_A_FULL], 0) && global_timer_ns() - t0 < 20000000ull) {
-    }
+    if constexpr (!Cfg::A_TMEM)
+      while (!mbar_try_wait(&c.bars[Cfg::BAR_A_FULL], 0) && global_timer_ns() - t0 < 20000000ull) {
+      }
     for (int st = 0; st < XST; ++st) {
-      const int u = (n_issued - 1 - st) >= 0 ? (n_issued - 1 - st) / XST : -1;
+      const int u = (x_issued - 1 - st) >= 0 ? (x_issued - 1 - st) / XST : -1;
       while (u >= 0 && !mbar_try_wait(&c.bars[Cfg::BAR_X_FULL + st], u & 1) && global_timer_ns() - t0 < 20000000ull) {
       }
     }
@@ -738,7 +734,7 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     return;
   }
 
-  if (threadIdx.x == 0) {
+  auto init_barriers = [&] {
 #pragma unroll
     for (int i = 0; i < Cfg::NUM_BARS; ++i) {
       // arrivals per phase: every compute warp releases a product buffer / an auxiliary stage
@@ -749,29 +745,54 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
     *c.abort_flag = 0;
     fence_mbar_init();
+  };
+  // EARLY: the producer initialises the barriers and goes straight on to its loads; the other warps meet once tensor memory is there and
+  // the status word has come in.  For the plain column sums only (us per call with the forward, bf16, H2O / RoCo: 12 heads, 128 tokens
+  // 11.94 / 12.30 -> 11.60 / 11.98; 32 heads, 512 tokens 20.35 / 20.84 -> 20.01 / 20.53, 1501 tokens 48.3 / 49.0 -> 47.6 / 48.4; 4 x 16
+  // heads, 1024 tokens 47.1 / 47.8 -> 46.5 / 47.1): the KeyFormer sweeps, bound by what they stream, lose 1 % (99.5 -> 100.8) and spill.
+  constexpr bool EARLY = MODE == SWEEP_COLSUM && !SOFTCAP;
+  if constexpr (EARLY) {
+    if (warp == CW) {
+      if (lane == 0) {
+        tma_prefetch_desc(&tm_a);
+        tma_prefetch_desc(&tm_x);
+        init_barriers();
+      }
+      __syncwarp();
+      asm volatile("barrier.cta.arrive 1, %0;" ::"n"(Cfg::THREADS) : "memory");
+    } else {
+      if (warp == 0) {
+        tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+        tmem_relinquish();
+      }
+      if (threadIdx.x == 0) *s_skip = status_now;
+      tc_fence_before();
+      asm volatile("barrier.cta.sync 1, %0;" ::"n"(Cfg::THREADS) : "memory");
+      tc_fence_after();
+      c.tmem_base = *tmem_slot;
+    }
+  } else {
+    if (threadIdx.x == 0) init_barriers();
+    if (warp == CW && lane == 0) {
+      tma_prefetch_desc(&tm_a);
+      tma_prefetch_desc(&tm_x);
+      if constexpr (Cfg::NOISE) tma_prefetch_desc(&tm_n);
+    }
+    if (warp == 0) {
+      tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+      tmem_relinquish();
+    }
+    if (threadIdx.x == 0) *s_skip = status_now;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    c.tmem_base = *tmem_slot;
   }
-  if (warp == CW && lane == 0) {
-    tma_prefetch_desc(&tm_a);
-    tma_prefetch_desc(&tm_x);
-    if constexpr (Cfg::NOISE) tma_prefetch_desc(&tm_n);
-  }
-  if (warp == 0) {
-    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
-    tmem_relinquish();
-  }
-  if (threadIdx.x == 0) *s_skip = status_now;
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  c.tmem_base = *tmem_slot;
   // A launch that follows an expired wait on this device drains immediately (the status word stays
   // set until the host reads it), so that one stuck kernel cannot stall a whole queue of launches.
-  if (*s_skip != 0) {
-    if (warp == 0) tmem_dealloc(c.tmem_base, Cfg::TMEM_COLS);
-    return;
-  }
-
-  if (warp < CW) {
+  if ((!EARLY || warp != CW) && *s_skip != 0) {
+    *c.abort_flag = WAIT_DRAIN;   // an early producer gives up, too
+  } else if (warp < CW) {
     if constexpr (Cfg::A_TMEM) if (warp < 4) {
       // thread r copies row r of the stationary tile (256 contiguous bytes) from global memory into TMEM lane r;
       // a 32-bit TMEM column holds two consecutive 16-bit elements, which is the order they have in memory
