@@ -252,6 +252,29 @@ struct SplitSoftmax {
 };
 
 // ------------------------------- TMA producer -------------------------------
+__device__ __forceinline__ void split_load_q(const SplitCtx& c, const CUtensorMap* tm_q, const TileInfo& t) {
+  using Cfg = SplitCfg;
+  mbar_expect_tx(&c.bars[Cfg::BAR_Q_FULL], Cfg::Q_TILE_BYTES);
+#pragma unroll
+  for (int ks = 0; ks < Cfg::KSUB; ++ks)
+    tma_load_4d(c.smem + ks * (Cfg::BM * 128), tm_q, &c.bars[Cfg::BAR_Q_FULL], ks * 64, t.h, t.q0, t.b);
+}
+__device__ __forceinline__ void split_load_k(const SplitCtx& c, const CUtensorMap* tm_k, const TileInfo& t, int slot, int n, int part) {
+  using Cfg = SplitCfg;
+  uint64_t* full = &c.bars[Cfg::BAR_FULL + slot];
+  mbar_expect_tx(full, Cfg::STAGE_BYTES);
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks)
+    tma_load_4d(c.smem + Cfg::Q_TILE_BYTES + slot * Cfg::STAGE_BYTES + ks * (Cfg::BN * 128), tm_k, full, part * 128 + ks * 64, t.hk,
+                t.lo * Cfg::V_KEYS + n * Cfg::BN, t.b);
+}
+// Q and the first K block of the CTA's first tile, before the set-up of the CTA is over.
+__device__ __forceinline__ void split_first_loads(const SplitCtx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k, const TileInfo& t) {
+  split_load_q(c, tm_q, t);
+#pragma unroll
+  for (int part = 0; part < SplitCfg::PARTS; ++part) split_load_k(c, tm_k, t, part, 0, part);
+}
+
 // One thread.  Ring stages in the order the issuer consumes them: K(0), then K(n+1), V(n) for n = 0, 1, ...
 template <bool PERSISTENT>
 __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
@@ -259,7 +282,7 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
   using Cfg = SplitCfg;
   constexpr int SL = Cfg::SLOTS;
   uint8_t* ring = c.smem + Cfg::Q_TILE_BYTES;
-  int ring_i = 0, tiles = 0;   // stages and Q tiles issued so far
+  int ring_i = Cfg::PARTS, tiles = 1;   // stages and Q tiles issued so far (split_first_loads)
   bool ok = true;
   for (int k = 0; ok; ++k) {
     // the first tile of a CTA is its own index (no round trip to the counter before the first load is issued)
@@ -289,13 +312,12 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
     const TileInfo t = decode_item(item, p, sp, Cfg::V_KEYS);
     const SplitBlocks blocks(t);
     const int nb = blocks.count;
-    if (k > 0) ok = c.wait(Cfg::BAR_Q_FREE, k - 1, WAIT_Q_FREE);
-    if (!ok) break;
-    mbar_expect_tx(&c.bars[Cfg::BAR_Q_FULL], Cfg::Q_TILE_BYTES);
-#pragma unroll
-    for (int ks = 0; ks < Cfg::KSUB; ++ks)
-      tma_load_4d(c.smem + ks * (Cfg::BM * 128), tm_q, &c.bars[Cfg::BAR_Q_FULL], ks * 64, t.h, t.q0, t.b);
-    ++tiles;
+    if (k > 0) {
+      ok = c.wait(Cfg::BAR_Q_FREE, k - 1, WAIT_Q_FREE);
+      if (!ok) break;
+      split_load_q(c, tm_q, t);
+      ++tiles;
+    }
     auto load = [&](bool is_v, int n) {
 #pragma unroll
       for (int part = 0; part < Cfg::PARTS; ++part) {
@@ -306,22 +328,19 @@ __device__ __forceinline__ void split_producer(const SplitCtx& c, const CUtensor
           return;
         }
         uint64_t* full = &c.bars[Cfg::BAR_FULL + slot];
-        uint8_t* dst = ring + slot * Cfg::STAGE_BYTES;
-        mbar_expect_tx(full, Cfg::STAGE_BYTES);
-        const int key0 = t.lo * Cfg::V_KEYS + n * Cfg::BN;
         if (is_v) {
+          mbar_expect_tx(full, Cfg::STAGE_BYTES);
 #pragma unroll
           for (int ks = 0; ks < Cfg::KSUB; ++ks)
-            tma_load_4d(dst + ks * (Cfg::V_KEYS * 128), tm_v, full, ks * 64, t.hk, key0 + part * Cfg::V_KEYS, t.b);
+            tma_load_4d(ring + slot * Cfg::STAGE_BYTES + ks * (Cfg::V_KEYS * 128), tm_v, full, ks * 64, t.hk,
+                        t.lo * Cfg::V_KEYS + n * Cfg::BN + part * Cfg::V_KEYS, t.b);
         } else {
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks)
-            tma_load_4d(dst + ks * (Cfg::BN * 128), tm_k, full, part * 128 + ks * 64, t.hk, key0, t.b);
+          split_load_k(c, tm_k, t, slot, n, part);
         }
         ++ring_i;
       }
     };
-    load(false, 0);
+    if (k > 0) load(false, 0);
     for (int n = 0; n < nb && ok; ++n) {
       if (n + 1 < nb) load(false, n + 1);
       if (ok) load(true, n);
@@ -465,7 +484,12 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   c.sched = reinterpret_cast<volatile int*>(tmem_slot + 2);
   c.skip = reinterpret_cast<volatile int*>(tmem_slot + 4);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
+  // The producer initialises the barriers, so that its first loads need not wait for the rest of the block.
+  const bool producer = warp == Cfg::PRODUCER_WARP && lane == 0;
+  if (producer) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
 #pragma unroll
     for (int i = 0; i < Cfg::NUM_BARS; ++i) {
       const bool p_full = i >= Cfg::BAR_P_FULL && i < Cfg::BAR_P_FULL + Cfg::PB;
@@ -475,14 +499,12 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     *c.abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == Cfg::PRODUCER_WARP && lane == 0) {
-    tma_prefetch_desc(&tm_q);
-    tma_prefetch_desc(&tm_k);
-    tma_prefetch_desc(&tm_v);
-  }
+  TileInfo first_tile;
+  if (producer) first_tile = decode_item(blockIdx.x, p, sp, Cfg::V_KEYS);   // the grid has no more CTAs than items
   // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
   // to allocate columns of its own, and what it wrote is visible only now.
   pdl_wait();
+  if (producer) split_first_loads(c, &tm_q, &tm_k, first_tile);
   if (threadIdx.x == 32) *c.skip = *reinterpret_cast<volatile int*>(&g_device_status);
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
@@ -503,6 +525,11 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     } else {
       split_issuer<BF16>(c, p, sp, lane);
     }
+  } else if (producer) {   // the loads above land before the CTA exits (bounded, 20 ms)
+    const uint64_t t0 = global_timer_ns();
+    for (int bar : {Cfg::BAR_Q_FULL, Cfg::BAR_FULL, Cfg::BAR_FULL + 1})
+      while (!mbar_try_wait(&c.bars[bar], 0) && global_timer_ns() - t0 < 20000000ull) {
+      }
   }
   tc_fence_before();
   __syncthreads();
