@@ -181,6 +181,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       tma_load_4d(dst + ks * (BN * 128), is_v ? &tm_v : &tm_k, full, ks * 64, t.hk, (t.lo + n) * BN, t.b);
   };
   if (Cfg::STAGED && warp == PRODUCER_WARP && lane == 0) {
+    fence_proxy_async_global();
     load_q(first_tile);
     load_kv(first_tile, false, 0, 0);
   }
@@ -265,7 +266,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       if (threadIdx.x == 0 && k < 8) B200_TL((3 * 64 + 48 + k) * 8 + 2);
       blocks_done = g;
     }
-    if (Cfg::STAGED && lane == 0) bulk_wait_read();   // (the stores themselves end with the kernel)
+    if (Cfg::STAGED && lane == 0) bulk_wait();   // before the kernel's end lets its successor read them
   } else if (warp == PRODUCER_WARP) {
     // --------------------------- TMA producer + tile scheduler ---------------------------
     if (lane == 0) {

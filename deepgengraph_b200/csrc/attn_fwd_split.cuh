@@ -504,7 +504,10 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
   // to allocate columns of its own, and what it wrote is visible only now.
   pdl_wait();
-  if (producer) split_first_loads(c, &tm_q, &tm_k, first_tile);
+  if (producer) {
+    fence_proxy_async_global();
+    split_first_loads(c, &tm_q, &tm_k, first_tile);
+  }
   if (threadIdx.x == 32) *c.skip = *reinterpret_cast<volatile int*>(&g_device_status);
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);

@@ -757,6 +757,7 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         tma_prefetch_desc(&tm_a);
         tma_prefetch_desc(&tm_x);
         init_barriers();
+        fence_proxy_async_global();
       }
       __syncwarp();
       asm volatile("barrier.cta.arrive 1, %0;" ::"n"(Cfg::THREADS) : "memory");

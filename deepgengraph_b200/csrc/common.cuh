@@ -209,6 +209,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 
 // programmatic dependent launch (see launch_kernel below)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// for the thread that issues bulk copies right behind pdl_wait: what the predecessor wrote with ordinary stores comes before them
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies, global -> shared, completion on an mbarrier)
@@ -241,6 +243,7 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* tmap, const void
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }   // sources are free
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }             // stores are done
 
 // ---------------------------------------------------------------------------
 // tcgen05: tensor memory management
