@@ -837,8 +837,8 @@ inline int attn_fwd_impl_lse_stride(const void* q, const void* k, const void* v,
   constexpr int NQ = 1;
 #endif
   if (!one_tile_per_cta && B200_BN128 == 64 && B200_SB128 == 2) {
-    CUtensorMap to;   // a warp stores 32 rows
-    if ((rc = make_bshd_tensor_map(&to, out, batch, q_len, heads, head_dim, 32, bf16)) != B200_OK) return rc;
+    CUtensorMap to = tq;   // a warp stores 32 rows (unused with a soft-cap)
+    if (!cap && (rc = make_bshd_tensor_map(&to, out, batch, q_len, heads, head_dim, 32, bf16)) != B200_OK) return rc;
     return bf16 ? (cap ? launch_attn_fwd_persist<true, true>(tq, tk, tv, to, p, stream)
                        : launch_attn_fwd_persist<true, false>(tq, tk, tv, to, p, stream))
                 : (cap ? launch_attn_fwd_persist<false, true>(tq, tk, tv, to, p, stream)

@@ -83,10 +83,11 @@ __device__ __forceinline__ void xor_permute4(uint32_t (&x)[4], uint32_t c) {
 struct SweepParams {
   const float* lse;     // [B*H][lse_stride]  row normalisers (COLSUM: L, KF_COLSUM: Lz)
   float* lse_out;       // [B*H][lse_stride]  KF_ROWLSE output
-  float* partial;       // [B*H][n_chunks][kv_pad]
-  float* partial_sq;    // same shape, RoCo only
+  float* partial;       // [B*H][n_chunks][row_stride], the first row_len of a row are written
+  float* partial_sq;    // same shape, RoCo and Corm only
+  int row_stride, row_len;
   int batch, heads, q_len, kv_len, delta, causal, window;
-  int lse_stride, kv_pad, n_chunks, chunk_blocks;
+  int lse_stride, n_chunks, chunk_blocks;
   int kv_group;         // query heads per K/V head (the key operand of head h is K head h / kv_group)
   // stationary operand as plain memory (configurations that keep it in TMEM load it with ordinary loads):
   const uint16_t* a_base;   // K (column-sum sweeps) or Q (row-LSE sweep), [batch, rows, a_heads, 128]
@@ -459,7 +460,8 @@ __device__ __forceinline__ void sweep_compute_colsum(const SweepCtx<Cfg>& c, con
     acc += c.sCombine[r];
     aux = AUX == AUX_CORM ? fmaxf(aux, c.sCombine[128 + r]) : aux + c.sCombine[128 + r];
   }
-  const int64_t off = ((int64_t)c.bh * p.n_chunks + chunk) * p.kv_pad + key;
+  if (key >= p.row_len) return;
+  const int64_t off = ((int64_t)c.bh * p.n_chunks + chunk) * p.row_stride + key;
   p.partial[off] = acc;
   if constexpr (AUX != AUX_NONE) p.partial_sq[off] = aux;
 }
@@ -548,7 +550,8 @@ __device__ __forceinline__ void sweep_compute_colsum_grouped(const SweepCtx<Cfg>
       ++hh;
     }
   }
-  const int64_t off = ((int64_t)c.bh * p.n_chunks + chunk) * p.kv_pad + key;
+  if (key >= p.row_len) return;
+  const int64_t off = ((int64_t)c.bh * p.n_chunks + chunk) * p.row_stride + key;
   p.partial[off] = acc;
   if constexpr (AUX != AUX_NONE) p.partial_sq[off] = aux;
 }
@@ -725,8 +728,8 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   if (c.blk_hi == c.blk_lo) {
     // nothing visible in this chunk: its partial vector is all zeros
     if constexpr (MODE != SWEEP_KF_ROWLSE) {
-      if (threadIdx.x < 128) {
-        const int64_t off = ((int64_t)c.bh * p.n_chunks + chunk) * p.kv_pad + c.a0 + threadIdx.x;
+      if (threadIdx.x < 128 && c.a0 + (int)threadIdx.x < p.row_len) {
+        const int64_t off = ((int64_t)c.bh * p.n_chunks + chunk) * p.row_stride + c.a0 + threadIdx.x;
         p.partial[off] = 0.f;
         if constexpr (AUX != AUX_NONE) p.partial_sq[off] = 0.f;
       }
@@ -937,6 +940,19 @@ inline int64_t score_workspace_bytes(int batch, int q_len, int kv_len, int heads
   return score_workspace_layout(batch, q_len, kv_len, heads).total;
 }
 
+// Where the sweep writes its sums: to the result itself where a key has one partial sum -- one chunk, one query head per K/V head (or the
+// sweep over the group's mean) --, else to scratch, for the ordered reduce.  A third launch that only copies cost, us per call, bf16,
+// H2O / RoCo, with -> without it: 12 heads, 128 tokens 11.61 / 11.93 -> 10.32 / 10.35; 32 heads, 512 tokens 19.95 / 20.49 -> 18.49 / 18.53,
+// 1501 tokens 47.7 / 48.5 -> 46.1 / 46.6; KeyFormer, 32 heads, 512 tokens 35.3 -> 33.9.  Returns true if there is nothing left to reduce.
+inline bool sums_to_result(SweepParams* p, const ScoreWorkspace& w, uint8_t* ws, int partial_sums, float* score, float* score_sq, int kv_len) {
+  const bool direct = partial_sums == 1;
+  p->partial = direct ? score : reinterpret_cast<float*>(ws + w.partial_off);
+  p->partial_sq = direct ? score_sq : reinterpret_cast<float*>(ws + w.partial_sq_off);
+  p->row_stride = direct ? kv_len : w.kv_pad;
+  p->row_len = direct ? kv_len : w.kv_pad;
+  return direct;
+}
+
 // n_chunks chunks of streamed blocks x n_tiles stationary tiles x (batch x heads) units -- (batch x K/V heads) when GROUPED
 template <int MODE, int BX, int STAGES, bool BF16, bool SOFTCAP, int AUX, bool GROUPED = false, int CWG = 1,
           bool GEN = false>
@@ -1036,8 +1052,6 @@ inline int attn_score_impl(const void* q, const void* k, const void* v, void* ou
   SweepParams p;
   std::memset(&p, 0, sizeof(p));
   p.lse = lse;
-  p.partial = reinterpret_cast<float*>(ws + w.partial_off);
-  p.partial_sq = reinterpret_cast<float*>(ws + w.partial_sq_off);
   p.batch = batch;
   p.heads = heads;
   p.q_len = q_len;
@@ -1046,8 +1060,9 @@ inline int attn_score_impl(const void* q, const void* k, const void* v, void* ou
   p.causal = causal ? 1 : 0;
   p.window = window > 0 ? window : 0;
   p.lse_stride = w.lse_stride;
-  p.kv_pad = w.kv_pad;
   p.n_chunks = w.n_chunks_colsum;
+  // (Corm's flags are reduced from the scratch)
+  const bool reduced = sums_to_result(&p, w, ws, corm_flags != nullptr ? 0 : p.n_chunks * (grouped ? 1 : group), score, score_sq, kv_len);
   p.chunk_blocks = kSweepChunkBlocks * (128 / (grouped ? 64 : B200_COLSUM_BX));
   p.a_base = static_cast<const uint16_t*>(k);
   p.a_rows = kv_len;
@@ -1073,7 +1088,7 @@ inline int attn_score_impl(const void* q, const void* k, const void* v, void* ou
     else
       rc = cap ? B200_SWEEPG(false, true, AUX_SQUARES) : B200_SWEEPG(false, false, AUX_SQUARES);
 #undef B200_SWEEPG
-    if (rc != B200_OK) return rc;
+    if (rc != B200_OK || reduced) return rc;
     dim3 ggrid((kv_len + 255) / 256, batch * kv_heads);
     B200_CUDA_TRY(launch_kernel(score_reduce_kernel, ggrid, 256, 0, stream, 1, score, score_sq, p.partial, p.partial_sq,
                                 kv_len, w.kv_pad, p.n_chunks, 1.0f));
@@ -1096,7 +1111,7 @@ inline int attn_score_impl(const void* q, const void* k, const void* v, void* ou
     rc = cap ? (sq ? B200_SWEEP0(false, true, AUX_SQUARES) : B200_SWEEP0(false, true, AUX_NONE))
              : (sq ? B200_SWEEP0(false, false, AUX_SQUARES) : B200_SWEEP0(false, false, AUX_NONE));
 #undef B200_SWEEP0
-  if (rc != B200_OK) return rc;
+  if (rc != B200_OK || reduced) return rc;
 
   dim3 rgrid((kv_len + 255) / 256, batch * kv_heads);
   B200_CUDA_TRY(launch_kernel(score_reduce_kernel, rgrid, 256, 0, stream, 1, score, score_sq, p.partial, p.partial_sq,
@@ -1153,8 +1168,6 @@ inline int attn_kf_impl(const void* q, const void* k, const void* v, const float
   std::memset(&p, 0, sizeof(p));
   p.lse = lse2;
   p.lse_out = lse2;
-  p.partial = reinterpret_cast<float*>(ws + w.partial_off);
-  p.partial_sq = nullptr;
   p.batch = batch;
   p.heads = heads;
   p.q_len = q_len;
@@ -1163,8 +1176,8 @@ inline int attn_kf_impl(const void* q, const void* k, const void* v, const float
   p.causal = causal ? 1 : 0;
   p.window = 0;
   p.lse_stride = w.lse_stride;
-  p.kv_pad = w.kv_pad;
   p.n_chunks = w.n_chunks_kf;
+  const bool reduced = sums_to_result(&p, w, ws, p.n_chunks * group, kf_score, nullptr, kv_len);
   p.chunk_blocks = kSweepChunkBlocks;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.inv_tau = 1.0f / tau;
@@ -1199,7 +1212,7 @@ inline int attn_kf_impl(const void* q, const void* k, const void* v, const float
     rc = bf16 ? B200_KF_SWEEP(SWEEP_KF_COLSUM, true, false, tk128, tq64, tn_rows64, p.n_chunks, gy)
               : B200_KF_SWEEP(SWEEP_KF_COLSUM, false, false, tk128, tq64, tn_rows64, p.n_chunks, gy);
 #undef B200_KF_SWEEP
-  if (rc != B200_OK) return rc;
+  if (rc != B200_OK || reduced) return rc;
 
   dim3 rgrid((kv_len + 255) / 256, batch * kv_heads);
   B200_CUDA_TRY(launch_kernel(score_reduce_kernel, rgrid, 256, 0, stream, 1, kf_score, (float*)nullptr, p.partial,

@@ -38,7 +38,7 @@ static ReplaceAddressFn get_replace_address() {
   return fn;
 }
 
-// One tensor map.  A call on a short problem is bound by the host, and an attention call needs three to nine maps.  Each thread
+// One tensor map.  A call on a short problem is bound by the host, and an attention call needs three to ten maps.  Each thread
 // keeps the layouts that it encoded last -- sizes, strides and box, a direct-mapped table of 64, 16 KB -- and every call puts
 // its own address into a copy: a call on new buffers costs what a repeated one does.  Measured from Python on a
 // tiny problem: attention with scores 12.2 us a call on one set of buffers and 12.3 on 400 in turn.

@@ -40,3 +40,28 @@ def test_keyformer_ring_depths(cuda_device, seq):
   _, score = att.attn_kf_fwd(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), noise.to(cuda_device), tau=1.5)
   # sums of at most 388 fp32 probabilities, exponents good to 2^-20
   torch.testing.assert_close(score.cpu(), ref, rtol=1e-3, atol=1e-5)
+
+
+@pytest.mark.parametrize("q_len,kv_len,heads,kv_heads", [(1, 200, 2, 2), (127, 129, 2, 2), (4096, 4100, 1, 1), (4097, 4100, 1, 1),
+                                                         (300, 300, 4, 2), (4100, 4100, 2, 1)])
+def test_sums_written_to_the_result_or_reduced(cuda_device, q_len, kv_len, heads, kv_heads):
+  # one partial sum per key (up to 4096 queries, one query head per K/V head or the sweep over the group's mean), or several
+  q = _rand(1, q_len, heads, 128, seed=q_len, dtype=torch.bfloat16).to(cuda_device)
+  k, v = (_rand(1, kv_len, kv_heads, 128, seed=kv_len + i, dtype=torch.bfloat16).to(cuda_device) for i in range(2))
+  ref = rm.attention_ref(q, k, v, want=("out", "colsum", "colsum_sq"))
+  _, score, score_sq = att.attn_score_fwd(q, k, v, want_sq=True)
+  _, alone = att.attn_score_fwd(q, k, v)
+  # fp32 sums of at most 4100 probabilities, exponents good to 2^-20
+  torch.testing.assert_close(score, ref["colsum"], rtol=1e-3, atol=1e-5)
+  torch.testing.assert_close(score_sq, ref["colsum_sq"], rtol=1e-3, atol=1e-5)
+  torch.testing.assert_close(alone, ref["colsum"], rtol=1e-3, atol=1e-5)
+
+
+@pytest.mark.parametrize("q_len,kv_len", [(2048, 2048), (2049, 2052)])
+def test_keyformer_sums_of_one_and_two_chunks(cuda_device, q_len, kv_len):
+  q = _rand(1, q_len, 1, 128, seed=1, dtype=torch.float16).to(cuda_device)
+  k, v = (_rand(1, kv_len, 1, 128, seed=2 + i, dtype=torch.float16).to(cuda_device) for i in range(2))
+  noise = -torch.rand(1, 1, q_len, kv_len, generator=torch.Generator().manual_seed(5)).clamp_min(1e-10).log().to(cuda_device)
+  ref = rm.attention_ref(q, k, v, exp_rand=noise, tau=1.0, want=("kf",))["kf"]
+  _, score = att.attn_kf_fwd(q, k, v, noise, tau=1.0)
+  torch.testing.assert_close(score, ref, rtol=1e-3, atol=1e-5)
