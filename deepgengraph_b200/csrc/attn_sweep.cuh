@@ -12,7 +12,7 @@
 //                    thread j accumulates sum_i p_ij (and sum_i p_ij^2): no cross-thread
 //                    reduction at all.  Query blocks are split into chunks over CTAs; each CTA
 //                    writes one partial vector and a small pass adds the partials in a fixed
-//                    order (no atomics, bit-reproducible).
+//                    order (no atomics, bit-reproducible); a single partial is the result.
 //                    -- H2O.forward kernels/h2o.py:35-38, RoCo.forward kernels/roco.py:42-48
 //   SWEEP_KF_COLSUM  same, with p2_ij = exp2((x_ij - log2 e_ij) / tau - Lz_i), e = exp_rand
 //                    -- KeyFormer.forward kernels/kf.py:36-42
