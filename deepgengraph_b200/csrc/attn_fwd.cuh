@@ -105,6 +105,7 @@ template <class Cfg, bool BF16>
 __device__ __forceinline__ void fwd_producer(const FwdCtx<Cfg, BF16>& c, const CUtensorMap* tm_q,
                                              const CUtensorMap* tm_k, const CUtensorMap* tm_v) {
   constexpr int SL = Cfg::SLOTS;
+  fence_proxy_async_global();
 #pragma unroll
   for (int t = 0; t < Cfg::NQ; ++t) {
     if (c.rng[t].hi > c.rng[t].lo) {

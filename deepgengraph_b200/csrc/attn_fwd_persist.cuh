@@ -214,6 +214,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const uint32_t o_addr = lane_addr + Cfg::O_BASE;
     uint64_t* o_full = &c.bars[Cfg::BAR_O_FULL];
     const float cmul = SOFTCAP ? p.cap_out : p.scale_log2;
+    if (Cfg::STAGED && lane == 0) fence_proxy_async_global();   // before the first bulk store: `out` may have been in use until now
     int g = 0;   // blocks processed by this CTA so far (S / P buffer = g % SB, barrier phases follow g)
     for (int k = 0;; ++k) {
       if (!mbar_wait_warp(&c.bars[Cfg::BAR_SCHED + (k & 1)], (k >> 1) & 1, c.abort_flag, WAIT_SCHED)) break;
@@ -270,6 +271,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   } else if (warp == PRODUCER_WARP) {
     // --------------------------- TMA producer + tile scheduler ---------------------------
     if (lane == 0) {
+      if (!Cfg::STAGED) fence_proxy_async_global();   // (otherwise before the first loads, above)
       int ring_i = Cfg::STAGED ? 1 : 0;   // K/V ring items issued so far (continuous across tiles)
       bool ok = true;
       for (int k = 0; ok; ++k) {

@@ -178,6 +178,7 @@ __device__ __forceinline__ void sweep_producer(const SweepCtx<Cfg>& c, const Swe
                                                const CUtensorMap* tm_x, const CUtensorMap* tm_n) {
   constexpr int XST = Cfg::XST, NST = Cfg::NST, BX = Cfg::BX;
   static_assert(!GROUPED || (Cfg::A_TMEM && !Cfg::NOISE), "grouped sweep: stationary tile in TMEM, no noise");
+  fence_proxy_async_global();   // (the row normalisers: ordinary stores of the launch before)
   if constexpr (!Cfg::A_TMEM) {
     mbar_expect_tx(&c.bars[Cfg::BAR_A_FULL], Cfg::A_BYTES);
 #pragma unroll
@@ -760,7 +761,6 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         tma_prefetch_desc(&tm_a);
         tma_prefetch_desc(&tm_x);
         init_barriers();
-        fence_proxy_async_global();
       }
       __syncwarp();
       asm volatile("barrier.cta.arrive 1, %0;" ::"n"(Cfg::THREADS) : "memory");

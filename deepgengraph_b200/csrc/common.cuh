@@ -209,7 +209,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 
 // programmatic dependent launch (see launch_kernel below)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// for the thread that issues bulk copies right behind pdl_wait: what the predecessor wrote with ordinary stores comes before them
+// For every thread that issues bulk copies to or from global memory, behind pdl_wait and before the first of them: what earlier kernels read
+// and wrote with ordinary loads and stores comes before copies that go through the async proxy.
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------

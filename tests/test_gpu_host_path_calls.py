@@ -110,6 +110,11 @@ def test_keyformer_with_a_noise_tensor_matches_the_python_path(cuda_device, kv_h
   assert all(torch.equal(a, b) for a, b in zip(got, att._attn_kf_impl(q, k, v, noise, 1.5, True, None)))
 
 
+def _same(got, want, what):
+  bad = (got != want).flatten().nonzero().flatten()
+  assert bad.numel() == 0, f"{what}: {bad.numel()} of {want.numel()} elements differ, flat indices {bad[0].item()} to {bad[-1].item()}"
+
+
 def test_library_launches_with_other_kernels_between_them(cuda_device):
   # every launch may start while its predecessor drains: neither side of a foreign kernel may be overtaken
   T, H, D = 700, 8, 128
@@ -138,3 +143,39 @@ def test_library_launches_with_other_kernels_between_them(cuda_device):
   for _ in range(20):
     got = chain(lambda: None)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("kind", ["scores", "capped_scores", "keyformer"])
+def test_launches_behind_ordinary_kernels_on_the_same_buffers(cuda_device, kind):
+  # q, k, v and the noise are rewritten, and the output buffer is read and overwritten, by ordinary kernels right before the call
+  B, S, H, D = 2, 700, 4, 128
+  lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+  sets = [[_rand(B, S, H, D, seed=10 * i + j) for j in range(3)] + [_rand(B, H, S, S, dtype=torch.float32, seed=10 * i + 3).abs() + 1e-3]
+          for i in range(2)]
+  ins = [torch.empty_like(t) for t in sets[0]]
+  ws = torch.empty(lib.b200_attn_score_workspace_bytes(B, S, S, H), dtype=torch.uint8, device="cuda")
+  out, score, seen = torch.empty_like(ins[0]), torch.empty(B, H, S, device="cuda"), torch.zeros_like(ins[0])
+
+  def call(src, between):
+    for a, b in zip(ins, src):
+      a.copy_(b)
+    seen.add_(out)
+    out.fill_(7.0)
+    score.fill_(7.0)
+    between()
+    args = [t.data_ptr() for t in ins]
+    if kind == "keyformer":
+      st = lib.b200_attn_kf_score(*args, out.data_ptr(), score.data_ptr(), ws.data_ptr(), ws.numel(), B, S, S, H, D, _lib.BF16, 1, 1.5,
+                                  D ** -0.5, stream)
+    else:
+      st = lib.b200_attn_score(*args[:3], out.data_ptr(), score.data_ptr(), None, ws.data_ptr(), ws.numel(), B, S, S, H, D, _lib.BF16, 1, 0,
+                               50.0 if kind == "capped_scores" else 0.0, D ** -0.5, stream)
+    assert st == 0
+    between()
+    return out.clone(), score.clone()
+
+  want = [call(src, torch.cuda.synchronize) for src in sets]
+  got = [call(sets[n % 2], lambda: None) for n in range(40)]
+  for n, pair in enumerate(got):
+    for what, a, b in zip(("out", "score"), pair, want[n % 2]):
+      _same(a, b, f"pass {n}: {what}")

@@ -56,3 +56,42 @@ def test_only_the_plain_launches_are_plain():
   for path in glob.glob(os.path.join(CSRC, "*.cu*")):
     launched |= set(re.findall(r"(\w+)(?:<[^<>;]*>)?<<<", open(path).read()))
   assert launched == PLAIN_LAUNCHES
+
+
+BULK_COPY = re.compile(r"\btma_(?:load|store)_\dd\(|cp\.async\.bulk\.(?!commit|wait)")
+FENCE = "fence_proxy_async_global();"
+
+
+def _functions_with_bulk_copies():
+  for path in sorted(glob.glob(os.path.join(CSRC, "attn_*.cuh"))):
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    for m in re.finditer(r"__device__ __forceinline__ void (\w+)\([^;{]*\{", text):
+      depth, end = 1, m.end()
+      while depth:
+        depth += {"{": 1, "}": -1}.get(text[end], 0)
+        end += 1
+      if BULK_COPY.search(text, m.end(), end):
+        yield m.group(1), text[m.end():end]
+  yield from ((name, body) for name, body in KERNELS.items() if BULK_COPY.search(body))
+
+
+def test_bulk_copies_follow_a_proxy_fence():
+  # Earlier kernels read and wrote with ordinary loads and stores; a copy through the async proxy is ordered behind them by a fence of
+  # the thread that issues it, after its pdl_wait.
+  found = dict(_functions_with_bulk_copies())
+  helpers = {"split_load_q", "split_load_k", "row_store_bulk"}   # called by the roles below
+  assert set(found) == helpers | {"fwd_producer", "sweep_producer", "split_producer", "attn_fwd_persist_kernel"}
+  for name in ("fwd_producer", "sweep_producer"):                # roles that begin behind the wait, one thread each
+    assert found[name].index(FENCE) < BULK_COPY.search(found[name]).start(), name
+    assert found[name][:found[name].index(FENCE)].count("{") == found[name][:found[name].index(FENCE)].count("}"), name
+  # head_dim 256: the producer thread's first loads come before its role
+  assert re.search(r"pdl_wait\(\);\s*if \(producer\) \{\s*fence_proxy_async_global\(\);\s*split_first_loads\(", KERNELS["attn_fwd_split_kernel"])
+  # head_dim 128: the producer, with and without loads before its role, and the threads that store
+  body = KERNELS["attn_fwd_persist_kernel"]
+  wait = body.index("pdl_wait();")
+  assert BULK_COPY.search(body).start() > wait
+  early, = re.findall(r"if \((Cfg::STAGED && warp == PRODUCER_WARP && lane == 0)\) \{\s*fence_proxy_async_global\(\);\s*load_q\(first_tile\);", body)
+  softmax, rest = body[wait:].split("if (warp < PRODUCER_WARP) {")[1].split("} else if (warp == PRODUCER_WARP) {")
+  assert "if (Cfg::STAGED && lane == 0) " + FENCE in softmax[:softmax.index("for (int k = 0;;")]
+  producer = rest[:rest.index("for (int k = 0; ok;")]
+  assert re.search(r"if \(lane == 0\) \{\s*if \(!Cfg::STAGED\) fence_proxy_async_global\(\);", producer)
