@@ -175,13 +175,17 @@ __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&w)[8]) 
 // roles fall through to the common tear-down (TMEM is always released).
 // Limit: 2 s of wall time -- three orders of magnitude above any legitimate wait.
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
+// A try that fails takes 60 to 90 ns.  The flag is looked at after every 16th: a CTA of a launch that drains leaves only when the role that
+// waits longest has seen it, and a launch has many waves of CTAs (plain column sums, 16 x 64 heads, 512 tokens, 14 waves, drained: 235 us
+// with a look after every 256th try, 65 now; launches that run take the same time).
+constexpr uint32_t kTriesPerLook = 16;
 
 __device__ __forceinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                             int code, uint64_t limit_ns = kWaitLimitNs) {
   const uint64_t t0 = global_timer_ns();
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity)) {
-    if ((++spins & 0xff) == 0) {
+    if (++spins % kTriesPerLook == 0) {
       if (*abort_flag != 0) return false;
       if (global_timer_ns() - t0 > limit_ns) {
         *abort_flag = code;
