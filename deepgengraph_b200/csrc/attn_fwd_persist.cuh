@@ -119,8 +119,9 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   using Cfg = PersistCfg<SOFTCAP>;
   constexpr int SL = Cfg::SLOTS, D = Cfg::D, BN = Cfg::BN, BM = Cfg::BM, SB = Cfg::SB;
   constexpr int PRODUCER_WARP = Cfg::SOFTMAX_WARPS;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = Cfg::STAGED ? smem_raw : reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  // (a name of its own: declarations of one name share one alignment, and swizzled tiles need 1024 bytes)
+  extern __shared__ __align__(1024) uint8_t persist_smem[];
+  uint8_t* smem = Cfg::STAGED ? persist_smem : reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(persist_smem) + 1023) & ~(uintptr_t)1023);
 
   if (threadIdx.x == 32) prefetch_l2(&g_device_status);   // read after the wait below
 

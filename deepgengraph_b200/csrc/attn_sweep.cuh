@@ -681,7 +681,9 @@ attn_sweep_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                   const __grid_constant__ CUtensorMap tm_n, const SweepParams p) {
   using Cfg = SweepCfg<MODE, BX, STAGES, CWG, GEN>;
   constexpr int CW = Cfg::COMPUTE_WARPS;
-  extern __shared__ __align__(1024) uint8_t smem[];   // (no static shared memory: it starts at a multiple of 1024)
+  // (a name of its own: declarations of one name share one alignment, and swizzled tiles need 1024 bytes)
+  extern __shared__ __align__(1024) uint8_t sweep_smem[];
+  uint8_t* smem = sweep_smem;
   // The wait comes before the TMEM allocation and the status word: a predecessor that let this launch start early may still have
   // to allocate columns of its own, and what it wrote is visible only now.  It comes first of all, because a launch has several
   // waves of CTAs: those of the later ones load the word while they set up.

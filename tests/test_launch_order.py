@@ -95,3 +95,13 @@ def test_bulk_copies_follow_a_proxy_fence():
   assert "if (Cfg::STAGED && lane == 0) " + FENCE in softmax[:softmax.index("for (int k = 0;;")]
   producer = rest[:rest.index("for (int k = 0; ok;")]
   assert re.search(r"if \(lane == 0\) \{\s*if \(!Cfg::STAGED\) fence_proxy_async_global\(\);", producer)
+
+
+def test_dynamic_shared_memory_has_one_alignment_per_name():
+  # the compiler gives all declarations of a name the alignment of one of them; kernels that do not round up rely on their own
+  found = {}
+  for path in glob.glob(os.path.join(CSRC, "*.cuh")):
+    for align, name in re.findall(r"extern __shared__ (?:__align__\((\d+)\) )?\w+ (\w+)\[\]", open(path).read()):
+      found.setdefault(name, set()).add(align)
+  assert found["sweep_smem"] == found["persist_smem"] == {"1024"}
+  assert all(len(aligns) == 1 for aligns in found.values()), found
