@@ -68,8 +68,8 @@ struct PersistCfg : FwdCfg<64, 1, 2> {
   // are issued before the set-up is over.  32 query heads, bf16, us per call, before -> with the bulk stores -> with both: 4 x 256
   // tokens, 8 K/V heads 9.89 -> 9.46 -> 9.13; 4 x 1024 tokens, 8 K/V heads 44.5 -> 43.1 -> 42.5; 128 tokens 6.66 -> 6.65 -> 6.47;
   // 512 tokens 10.94 -> 10.96 -> 10.71; 2048 tokens 37.1 -> 36.7 -> 35.5; 4 x 4096 tokens 499 -> 499 -> 486 (idle GPU).
-  // With a soft-cap the compiler schedules the longer softmax worse around either (2 x 4096 tokens 327 -> 338, 2048 tokens 52.2 -> 54.5,
-  // 159 -> 160 registers), so that kernel stores its rows directly and loads after the set-up.
+  // With a soft-cap the compiler schedules the longer softmax worse around either (2 x 4096 tokens 327 -> 338, 2048 tokens 52.2 -> 54.5),
+  // so that kernel stores its rows directly and loads after the set-up.
   static constexpr bool STAGED = !SOFTCAP;
   // Behind Q, the ring and the staging: barriers, a few words.  Without static shared memory, dynamic shared memory starts at a
   // multiple of 1024 bytes.
@@ -135,7 +135,9 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   c.bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BARS);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c.bars + Cfg::NUM_BARS_P);
   c.abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* s_skip = reinterpret_cast<volatile int*>(tmem_slot + 4);
+  // The status word reaches everybody with the barrier.  As a word among the barriers it cost the soft-capped kernel 2 % at some sizes (32 heads:
+  // 2048 tokens 53.6 against 52.3 us; 4 x 1024 tokens, 8 K/V heads 62.2 against 61.3).
+  int skip = 0;
   volatile int* sched = reinterpret_cast<volatile int*>(tmem_slot + 2);   // [2] item index or -1
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -186,18 +188,18 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     load_q(first_tile);
     load_kv(first_tile, false, 0, 0);
   }
-  if (threadIdx.x == 32) *s_skip = *reinterpret_cast<volatile int*>(&g_device_status);
+  if (threadIdx.x == 32) skip = *reinterpret_cast<volatile int*>(&g_device_status);
   if (warp == 0) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  skip = __syncthreads_or(skip);
   tc_fence_after();
   c.tmem_base = *tmem_slot;
   // A launch that follows an expired wait on this device drains immediately (the status word stays set until the host reads it; the tile
   // counter is untouched: the host zeroes it when it clears the word).
-  if (*s_skip != 0) {
+  if (skip != 0) {
     if (Cfg::STAGED && warp == PRODUCER_WARP && lane == 0) {
       const uint64_t t0 = global_timer_ns();   // the two loads above land before the CTA exits (bounded, 20 ms)
       for (int bar : {Cfg::BAR_Q_FULL, Cfg::BAR_FULL})
