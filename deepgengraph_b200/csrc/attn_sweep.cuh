@@ -133,7 +133,11 @@ struct SweepCfg {
   static constexpr int TMEM_COLS = A_TMEM ? 256 : 2 * BX;               // two product tiles (+ the stationary tile)
   static constexpr int COMPUTE_WARPS = 4 * CWG;
   static constexpr int THREADS = (COMPUTE_WARPS + 2) * 32;   // + TMA producer warp + MMA issuer warp
-  // launch bound (registers): two CTAs share an SM -- the 320-thread column-sum CTAs and the KeyFormer CTAs
+  // launch bound (registers): two CTAs share an SM -- the 320-thread column-sum CTAs and the KeyFormer CTAs.  The grouped sweep's 192-thread
+  // CTAs share one too, without the bound: they take 163 registers (141 with the soft-cap), and a bound of two costs them 2 to 4 % (32/8 heads,
+  // us, RoCo / Corm, 512 tokens 36.4 / 39.6 -> 37.7 / 41.0, 1500 tokens 94.3 / 98.7 -> 98.2 / 102.9).  What it is worth that they fit (more
+  // than 168 registers leave one CTA per SM; 254 -> 163): 512 tokens 40.9 / 42.3 -> 36.4 / 39.6, 2 x 4096 tokens 604 / 613 -> 509 / 524; a
+  // launch of 149 to 296 CTAs gains nothing, since its lighter tiles now run beside the heaviest (4096 tokens 317 / 322 -> 318 / 329).
   static constexpr int CTAS_PER_SM = (CWG == 2 || MODE != SWEEP_COLSUM) ? 2 : 1;
   static_assert(CWG == 1 || CWG == 2, "one or two compute warpgroups");
   static_assert(BX / 32 % CWG == 0, "every compute warpgroup takes whole 32-column chunks");
@@ -151,7 +155,8 @@ struct SweepCfg {
   static constexpr int COMBINE_BYTES = CWG == 2 && !NOISE ? 2 * 128 * 4 : 0;
   static constexpr int SMEM_BYTES = A_BYTES + XST * X_STAGE_BYTES + NST * N_STAGE_STRIDE + LSE_RING_BYTES + COMBINE_BYTES +
                                     NUM_BARS * 8 + 16;
-  static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 233472, "shared memory budget exceeded");   // 1 KB per CTA is reserved
+  static_assert(2 * (SMEM_BYTES + 1024) <= 233472, "shared memory budget of two CTAs per SM exceeded");   // 1 KB per CTA is reserved
+  static_assert(2 * TMEM_COLS <= 512, "TMEM of two CTAs per SM exceeded");
 };
 
 template <class Cfg>
