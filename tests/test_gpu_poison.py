@@ -9,6 +9,7 @@ import torch
 
 from deepgengraph_b200 import _lib
 from deepgengraph_b200 import attention as att
+from oracle import reference_math as rm
 
 pytestmark = pytest.mark.gpu
 GUARD = 4096   # elements
@@ -66,6 +67,60 @@ def test_scores_do_not_depend_on_scratch_contents(cuda_device):
     tail = ws[nbytes // 4:]
     assert (torch.isnan(tail).all() if math.isnan(fill) else (tail == fill).all())   # nothing past the stated size
     results.append((out.clone(), score.clone(), score_sq.clone()))
+  for r in results[1:]:
+    assert all(torch.equal(a, b) for a, b in zip(results[0], r))
+
+
+# Scores with one partial sum per key (up to 4096 queries, KeyFormer 2048, one query head per K/V head or the sweep over the group's mean) are
+# written by the sweep itself; others are reduced from the scratch.  Odd key lengths: a row that ran over would end in the next head's.
+# The windowed cases have key tiles that no query sees.
+@pytest.mark.parametrize("kind,B,Sq,Skv,H,Hk,window", [
+    ("sums", 1, 301, 433, 3, 3, 0), ("squares", 2, 301, 433, 3, 3, 0), ("squares", 1, 4100, 4101, 2, 2, 0), ("sums", 2, 300, 301, 4, 2, 0),
+    ("squares", 2, 300, 301, 4, 2, 0), ("squares", 1, 4100, 4101, 2, 1, 0), ("corm", 1, 300, 301, 2, 2, 0), ("corm", 1, 300, 301, 4, 2, 0),
+    ("seeded", 2, 301, 303, 3, 3, 0), ("seeded", 1, 2050, 2051, 2, 2, 0), ("seeded", 1, 300, 301, 4, 2, 0), ("keyformer", 1, 300, 300, 3, 3, 0),
+    ("keyformer", 1, 2050, 2052, 2, 2, 0), ("squares", 1, 200, 1001, 3, 3, 150), ("squares", 1, 200, 1001, 4, 2, 150),
+    ("sums", 1, 200, 1001, 4, 2, 150), ("capped", 1, 200, 1001, 3, 3, 150), ("sums", 1, 4100, 4500, 2, 2, 100)])
+def test_scores_on_every_route_write_their_rows_and_nothing_else(cuda_device, kind, B, Sq, Skv, H, Hk, window):
+  g = torch.Generator().manual_seed(Sq + Skv)
+  q, k, v = (torch.randn(B, s, h, 128, generator=g).to(torch.bfloat16).to(cuda_device) for s, h in ((Sq, H), (Skv, Hk), (Skv, Hk)))
+  lib, scale, tau = _lib.load(), 128 ** -0.5, 1.5
+  nbytes = lib.b200_attn_score_workspace_bytes(B, Sq, Skv, H)
+  noise = torch.empty(B, H, Sq, Skv, device=cuda_device) if kind in ("keyformer", "seeded") else None
+  if noise is not None:
+    assert lib.b200_kf_noise_fill(noise.data_ptr(), 11, B, H, Sq, Skv, _stream(cuda_device)) == 0
+  want = {"sums": ("colsum",), "squares": ("colsum", "colsum_sq"), "capped": ("colsum", "colsum_sq"), "corm": ("colsum",)}.get(kind, ("kf",))
+  ref = rm.attention_ref(q, k, v, window=window, softcap=5.0 if kind == "capped" else 0.0, exp_rand=noise, tau=tau, want=want + ("out",))
+  results = []
+  for fill in (float("nan"), 0.0, 1e30):
+    ws = torch.full((nbytes // 4 + 64,), fill, dtype=torch.float32, device=cuda_device)
+    out_flat, out = _guarded((B, Sq, H, 128), torch.bfloat16, cuda_device)
+    flats, scores = zip(*(_guarded((B, Hk, Skv), torch.float32, cuda_device) for _ in range(2)))
+    flags = torch.full((B * Hk * Skv + GUARD,), 7, dtype=torch.uint8, device=cuda_device)
+    inputs, sizes = (q.data_ptr(), k.data_ptr(), v.data_ptr()), (ws.data_ptr(), nbytes, B, Sq, Skv, H, Hk, 128, _lib.BF16, 1)
+    score, score_sq = (s.data_ptr() for s in scores)
+    if kind == "keyformer":
+      st = lib.b200_attn_kf_score_gqa(*inputs, noise.data_ptr(), out.data_ptr(), score, *sizes, tau, scale, _stream(cuda_device))
+    elif kind == "seeded":
+      st = lib.b200_attn_kf_score_seeded(*inputs, 11, out.data_ptr(), score, *sizes, tau, scale, _stream(cuda_device))
+    else:
+      st = lib.b200_attn_score_gqa(*inputs, out.data_ptr(), score, score_sq if kind in ("squares", "capped") else None,
+                                   flags.data_ptr() if kind == "corm" else None, *sizes, window, 5.0 if kind == "capped" else 0.0, scale,
+                                   _stream(cuda_device))
+    assert st == 0, _lib.STATUS_NAMES.get(st, st)
+    torch.cuda.synchronize()
+    for flat, t in ((out_flat, out),) + tuple(zip(flats, scores)):
+      assert torch.isnan(flat[t.numel():].float()).all()
+    tail = ws[nbytes // 4:]
+    assert (torch.isnan(tail).all() if math.isnan(fill) else (tail == fill).all())   # nothing past the stated size
+    assert (flags[B * Hk * Skv:] == 7).all() and bool((flags[:B * Hk * Skv] <= 1).all()) == (kind == "corm")
+    results.append([out, flags] + list(scores[:len(want)]))
+    # fp32 sums of at most 4100 probabilities, exponents good to 2^-20; with a soft-cap tanh.approx (2^-11) above the cap
+    tol = dict(rtol=5e-3, atol=1e-5) if kind == "capped" else dict(rtol=1e-3, atol=1e-5)
+    for name, t in zip(want, scores):
+      torch.testing.assert_close(t, ref[name], **tol)
+    torch.testing.assert_close(out.float(), ref["out"], rtol=2e-2, atol=2e-2)
+    if window:
+      assert (scores[0][..., :(Skv - Sq - window + 1) // 128 * 128] == 0).all()
   for r in results[1:]:
     assert all(torch.equal(a, b) for a, b in zip(results[0], r))
 
