@@ -65,14 +65,15 @@ struct PersistCfg : FwdCfg<64, 1, 2> {
   static constexpr int BAR_SCHED_FREE = BAR_Q_FREE + 1;   // [2] descriptor slot read by all its consumers
   static constexpr int NUM_BARS_P = BAR_SCHED_FREE + 2;
   // Without a soft-cap the output goes through 4 KB of staging per softmax warp (32 rows x 64 columns) to bulk stores, and the first loads
-  // are issued before the set-up is over.  32 query heads, bf16, us per call, before -> with the bulk stores -> with both: 4 x 256
-  // tokens, 8 K/V heads 9.89 -> 9.46 -> 9.13; 4 x 1024 tokens, 8 K/V heads 44.5 -> 43.1 -> 42.5; 128 tokens 6.66 -> 6.65 -> 6.47;
-  // 512 tokens 10.94 -> 10.96 -> 10.71; 2048 tokens 37.1 -> 36.7 -> 35.5; 4 x 4096 tokens 499 -> 499 -> 486 (idle GPU).
+  // are issued before the set-up is over.  32 query heads, bf16, us per call, before -> with the bulk stores and one loop over K and V in the
+  // producer -> with the early loads, too: 4 x 256 tokens, 8 K/V heads 9.91 -> 9.37 -> 9.23; 4 x 1024 tokens, 8 K/V heads 44.0 -> 42.1 ->
+  // 41.9; 128 tokens 6.64 -> 6.62 -> 6.47; 512 tokens 10.89 -> 10.77 -> 10.73; 1024 tokens 17.43 -> 17.41 -> 17.38; 4 x 4096 tokens 496, 494,
+  // 490, where two runs of one build differ by 3 %.  The early loads are worth what they save once per CTA, up to 0.15 us.
   // With a soft-cap the compiler schedules the longer softmax worse around either (2 x 4096 tokens 327 -> 338, 2048 tokens 52.2 -> 54.5),
   // so that kernel stores its rows directly and loads after the set-up.
   static constexpr bool STAGED = !SOFTCAP;
-  // Behind Q, the ring and the staging: barriers, a few words.  Without static shared memory, dynamic shared memory starts at a
-  // multiple of 1024 bytes.
+  // Behind Q, the ring and the staging: barriers, a few words.  (The staged kernel has no room to round its memory up to 1024 bytes; it is
+  // declared with that alignment.)
   static constexpr int STAGE_OUT_BYTES = 32 * 128;
   static constexpr int OFF_BARS = Base::SMEM_TILES + (STAGED ? SOFTMAX_WARPS * STAGE_OUT_BYTES : 0);
   static constexpr int SMEM_BYTES_P = OFF_BARS + NUM_BARS_P * 8 + 64 + (STAGED ? 0 : 1024);
@@ -317,7 +318,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
           load_kv(t, is_v, n, slot);
           ++ring_i;
         };
-        if constexpr (Cfg::STAGED) {   // (one loop for both: 1024 tokens 17.6 us, with the two loops below 17.8)
+        if constexpr (Cfg::STAGED) {   // (one loop for both: 4 x 1024 tokens, 32/8 heads 41.9 us, with the two loops below 42.7; 1024 tokens 17.38, 17.55)
           int next_k = k == 0 ? 1 : 0, next_v = 0;
           while (ok && next_v < nb) {
             const bool is_v = next_k == nb || next_k - next_v == SB;

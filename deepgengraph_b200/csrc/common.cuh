@@ -47,7 +47,9 @@ __device__ long long* g_timeline = nullptr;
 __device__ int g_timeline_block = 0;
 __device__ long long* g_cta_times = nullptr;   // [num CTAs][8]: start ns, end ns, SM id, key blocks, SM clocks
 constexpr int kTimelineSlots = 2048;
-__shared__ unsigned int s_timeline[kTimelineSlots];   // stamps stay in shared memory until the CTA ends
+// Stamps stay in shared memory until the CTA ends.  (8 KB that the head_dim 128 forward without a soft-cap has not got beside its output staging:
+// such a build runs it with one CTA per SM, unless the slots are cut down to the few that are looked at.)
+__shared__ unsigned int s_timeline[kTimelineSlots];
 __device__ __forceinline__ unsigned int clock32() {
   unsigned int c;
   asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
