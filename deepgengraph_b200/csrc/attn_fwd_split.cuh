@@ -6,7 +6,8 @@
 //
 // What bounds it and why this shape.  Per block of 128 keys the tensor pipe needs 16 x 64 clk for S and 8 x 128 for P V, 2048 in all,
 // the special-function unit 1024; a block takes 3100 clk with the soft-cap and 2830 without (a launch of 85.6 blocks per SM, everything
-// included; with two S buffers, below, 3130 and 2900): no pipe is full, the chain S -> softmax -> P -> P V of one tile is what is left, and in long launches the power limit.
+// included; with two S buffers, below, 3130 and 2900): no pipe is full, the chain S -> softmax -> P -> P V of one tile is what is left, and
+// in long launches the power limit.
 // S is free as soon as the softmax warps have it in registers, so that S(n+1) is computed under the softmax of block n and before
 // P V(n).  With two S buffers, in which P took S's place, S(n+2) had to wait for P V(n) (us, before -> now, bf16, no soft-cap): 16/8 heads,
 // causal, 1024 tokens 18.23 -> 18.02, 4096 tokens 110.5 -> 106.5, 8192 tokens 405.2 -> 398.7; 500 queries on 4000 keys, 32/8 heads 50.9 ->
